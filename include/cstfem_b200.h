@@ -96,8 +96,10 @@ typedef struct {
                                    cstg_pcg_setup                                                */
 
 /* launch_mode of cstg_pcg_solve */
-#define CSTG_LAUNCH_AUTO 0        /* persistent kernel for mesh-pattern matrices, else graph  */
-#define CSTG_LAUNCH_PERSISTENT 1  /* one cooperative kernel runs all iterations (mesh pattern) */
+#define CSTG_LAUNCH_AUTO 0        /* one persistent kernel runs all iterations (mesh pattern, or CSR
+                                     with short rows of like length) where the blocks' shares of the
+                                     matrix fit, else graph */
+#define CSTG_LAUNCH_PERSISTENT 1  /* the same without the one-cluster variant for small systems  */
 #define CSTG_LAUNCH_GRAPH 2       /* 3-4 kernels per iteration, chunks replayed as CUDA graphs */
 #define CSTG_LAUNCH_INSTRUMENTED 3 /* FP64 Jacobi-PCG with its kernels launched one by one and CUDA
                                       events between the phases (cstg_solve_breakdown); slower  */
@@ -173,8 +175,8 @@ int cstg_version(void);
 int cstg_binary_version(int device, int* version);
 /* Bounded device waits (no reference counterpart). Every device-side wait of the library gives
  * up after a number of polls and reports CSTG_ERR_TIMEOUT (stats->status CSTG_SOLVE_TIMEOUT where
- * a solve was running) with the context still usable: the persistent solve's grid barriers
- * (default 50,000,000 polls, about 2 s) and the learned network's tensor-core waits (default
+ * a solve was running) with the context still usable: the persistent solve's waits
+ * between blocks (default 50,000,000 polls, about 2 s) and the learned network's tensor-core waits (default
  * 4,194,304 polls). 0 makes a wait give up at once (failure-detection tests); -1 restores the
  * default. A tensor-core wait that gives up still lets its matrix multiply finish (bounded)
  * before the kernel releases its memory. */

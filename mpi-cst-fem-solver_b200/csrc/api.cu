@@ -84,7 +84,7 @@ void cstg_destroy(cstg_ctx* ctx) {
                    &ctx->ne,      &ctx->scan_tmp, &ctx->deg,    &ctx->node_ptr, &ctx->bnbr,
                    &ctx->slot,    &ctx->row_ptr, &ctx->cols,    &ctx->vals,     &ctx->fixed,
                    &ctx->ubar,    &ctx->dofs,   &ctx->dvals,    &ctx->b_in,     &ctx->x,
-                   &ctx->r,       &ctx->p,      &ctx->Ap,       &ctx->inv_diag, &ctx->partials,
+                   &ctx->pcg_work, &ctx->pcg_slots, &ctx->r,       &ctx->p,      &ctx->Ap,       &ctx->inv_diag, &ctx->partials,
                    &ctx->state,   &ctx->err_word, &ctx->hist,   &ctx->vec_in,   &ctx->vec_out,
                    &ctx->stress,    &ctx->val32,  &ctx->nbr32,    &ctx->S32,      &ctx->mat,
                    &ctx->mat_tab, &ctx->bat_sys, &ctx->bat_order, &ctx->bat_queue, &ctx->bat_b,
@@ -375,6 +375,8 @@ int cstg_set_csr(cstg_ctx* ctx, int n, const int32_t* row_ptr, const int32_t* co
   int sub = 1;
   while (sub < 32 && sub < avg) sub <<= 1;
   ctx->csr_sub = sub;
+  ctx->csr_longest = 0;
+  for (int i = 0; i < n; ++i) ctx->csr_longest = std::max(ctx->csr_longest, row_ptr[i + 1] - row_ptr[i]);
   ctx->kind = 2;
   ctx->n_rows = n;
   ctx->nnz = nnz;
@@ -646,20 +648,31 @@ static int run_solve(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg_s
   }
   const long long per_iter = mixed ? 4 : 3;
 
-  // Mesh-pattern matrices run as one persistent cooperative kernel per solve (unless the
-  // caller asks for the graph path); caller CSR matrices use the graph path.
+  // One persistent kernel runs the solve (unless the caller asks for the graph path) on the first team
+  // of blocks whose shared memory holds it. CSR matrices take it only with short rows of like length:
+  // one or two lanes walk a row there, where the graph path's SpMV has up to 32.
   const bool instrumented = o.launch_mode == CSTG_LAUNCH_INSTRUMENTED;
   if (instrumented && mixed)
     return fail(ctx, CSTG_ERR_UNSUPPORTED, "pcg_solve: the instrumented launch mode runs FP64 Jacobi-PCG only");
-  const bool persist = ctx->kind == 1 && o.launch_mode != CSTG_LAUNCH_GRAPH && !instrumented && !snap;
-  const int chunk = snap ? snap->every : persist ? o.max_iter + 1 : instrumented ? kBdChunk
-                                                                  : (o.check_interval > 0 ? o.check_interval : 50);
-  // (Re)capture the chunk graph when a buffer, the shape or the method changed. The mixed
+  const bool csr = ctx->kind != 1;
+  const bool even_rows = !csr || pcg_persistent_rows(n, ctx->nnz, ctx->csr_longest);
+  const int units = csr ? n : ctx->n_nodes;
+  const long long entries = csr ? ctx->nnz : ctx->nnz / 4;
+  const auto next_team = [&](PcgTeam after) {
+    return pcg_persistent_team(units, entries, mixed, csr, o.launch_mode == CSTG_LAUNCH_AUTO, after);
+  };
+  PcgTeam team = n > 0 && even_rows && o.launch_mode != CSTG_LAUNCH_GRAPH && !instrumented && !snap
+                     ? next_team(PcgTeam::kFirst)
+                     : PcgTeam::kNone;
+  if (team != PcgTeam::kNone) ENSURE(ctx->pcg_work, pcg_persistent_work(n));
+  const int chunk = snap ? snap->every : instrumented ? kBdChunk : (o.check_interval > 0 ? o.check_interval : 50);
+  // (Re)captures the chunk graph when a buffer, the shape or the method changed. The mixed
   // graph reads b (reliable updates), so it is also tied to the right-hand-side pointer.
-  if (!persist && !instrumented && (!ctx->graph || ctx->graph_gen != ctx->generation || ctx->graph_chunk != chunk ||
-      ctx->graph_hist != (hist ? 1 : 0) || ctx->graph_kind != ctx->kind || ctx->graph_n != n ||
-      ctx->graph_prec != o.precision || ctx->graph_refs != o.max_refinements ||
-      (mixed && ctx->graph_b != d_b))) {
+  const auto ensure_graph = [&]() -> int {
+    if (!(!ctx->graph || ctx->graph_gen != ctx->generation || ctx->graph_chunk != chunk ||
+          ctx->graph_hist != (hist ? 1 : 0) || ctx->graph_kind != ctx->kind || ctx->graph_n != n ||
+          ctx->graph_prec != o.precision || ctx->graph_refs != o.max_refinements || (mixed && ctx->graph_b != d_b)))
+      return CSTG_OK;
     if (ctx->graph) {
       cudaGraphExecDestroy(ctx->graph);
       ctx->graph = nullptr;
@@ -685,7 +698,8 @@ static int run_solve(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg_s
     ctx->graph_prec = o.precision;
     ctx->graph_refs = o.max_refinements;
     ctx->graph_b = d_b;
-  }
+    return CSTG_OK;
+  };
 
   // instrumented: events around the phases of every iteration (kBdChunk iterations per batch)
   double bd_spmv = 0.0, bd_vec = 0.0;
@@ -701,7 +715,7 @@ static int run_solve(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg_s
   long long spmv_calls = 0;
   int rc = snapshot(ctx);
   if (rc) return rc;
-  const long long max_chunks = (long long)o.max_iter / chunk + 2 + (long long)o.max_refinements * 4;
+  const long long max_chunks = (long long)o.max_iter / chunk + 8 + (long long)o.max_refinements * 4;
   long long chunks = 0;
   bool true_done = false;
   while (ctx->h_state->done != CSTG_SOLVE_ZERO_RHS + 1) {
@@ -710,8 +724,12 @@ static int run_solve(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg_s
         return fail(ctx, CSTG_ERR_TIMEOUT, "pcg_solve: the device state did not finish after %lld chunks",
                     chunks);
       const int it0 = ctx->h_state->iter;
-      if (persist) {
-        CK(launch_pcg_persistent(w, bm, mixed ? &mm : nullptr, o.max_refinements, ctx->barrier_spin, ctx->stream));
+      if (team != PcgTeam::kNone) {
+        // (rounded up to what a bulk copy reads)
+        if (mixed || team >= PcgTeam::kStream) ENSURE(ctx->pcg_slots, sizeof(unsigned short) * ((size_t)entries + 32));
+        CK(launch_pcg_persistent(team, w, pbm, mixed ? &mm : nullptr, pcm, ctx->pcg_work.p,
+                                 buf_ptr<unsigned short>(ctx->pcg_slots), o.max_refinements, ctx->barrier_spin,
+                                 ctx->stream));
       } else if (instrumented) {
         // SpMV (with its fused p'Ap partials), then the vector phase (x, r, p updates with their
         // fused dots), an event after each; the elapsed times are summed after the batch
@@ -731,6 +749,8 @@ static int run_solve(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg_s
           bd_vec += b_ms * 1e-3;
         }
       } else {
+        rc = ensure_graph();
+        if (rc) return rc;
         CK(cudaGraphLaunch(ctx->graph, ctx->stream));
         count_launches(per_iter * chunk);
         if (snap && snap->count < snap->max && n)
@@ -739,6 +759,10 @@ static int run_solve(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg_s
       }
       rc = snapshot(ctx);
       if (rc) return rc;
+      if (team != PcgTeam::kNone && ctx->h_state->no_halo)
+        team = next_team(team);  // (the blocks' shares did not fit: nothing was done)
+      else if (team != PcgTeam::kNone && ctx->h_state->done == 0)
+        team = PcgTeam::kNone;  // (a streamed mixed solve after its switch to FP64)
       if (ctx->h_state->done == CSTG_SOLVE_TIMEOUT + 1) {
         if (stats) {
           std::memset(stats, 0, sizeof *stats);

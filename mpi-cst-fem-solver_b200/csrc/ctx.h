@@ -66,12 +66,14 @@ struct cstg_ctx {
   int n_rows = 0;
   long long nnz = 0;
   int csr_sub = 8;
+  int csr_longest = 0;  // entries of the longest row (caller CSR)
   bool has_values = false, setup_done = false;
 
   // Dirichlet
   DevBuf fixed, ubar, dofs, dvals;
 
   // solver
+  DevBuf pcg_work, pcg_slots;  // persistent solve: what passes between blocks, rows in their numbering
   DevBuf b_in, x, r, p, Ap, inv_diag, partials, state, err_word, hist, vec_in, vec_out, stress;
   // mixed precision: FP32 difference-form operator and FP32 work vectors
   DevBuf val32, nbr32, S32;

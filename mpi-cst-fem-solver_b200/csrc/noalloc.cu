@@ -6,7 +6,8 @@
 // the solve from a callback where cudaMalloc / cudaFree would synchronise the whole device
 // and stall other work, and real-time loops that must not block in the driver's allocator.
 // For them, cstg_pcg_solve_static keeps every work vector of the solve (inverse diagonal,
-// r, p, A p, the block partial sums and the solver state) in one file-scope static
+// r, then p and A p or what passes between the persistent kernel's blocks, the block partial sums
+// and the solver state) in one file-scope static
 // __device__ array whose size is fixed when the library is loaded; the caller passes only
 // its matrix, right-hand side and solution.
 //
@@ -148,7 +149,7 @@ extern "C" int cstg_pcg_solve_static(int n_rows, const int32_t* d_row_ptr, const
   w.err = err;
 
   const int chunk = o.check_interval > 0 ? o.check_interval : 50;
-  const long long max_chunks = (long long)o.max_iter / chunk + 2 + (long long)o.max_refinements * 4;
+  const long long max_chunks = (long long)o.max_iter / chunk + 8 + (long long)o.max_refinements * 4;
   PcgState h;
   auto snap = [&]() -> cudaError_t {
     cudaError_t e = cudaMemcpyAsync(&h, st, sizeof h, cudaMemcpyDeviceToHost, s);
@@ -158,6 +159,18 @@ extern "C" int cstg_pcg_solve_static(int n_rows, const int32_t* d_row_ptr, const
   const auto t0 = std::chrono::steady_clock::now();
   SCK(launch_pcg_init(w, o.rtol, o.max_iter, false, s));
   SCK(snap());
+  // The context's rule for the persistent kernel, where what passes between its blocks fits in place of
+  // p and Ap, which it does not use.
+  int longest = 0;
+  PcgTeam team = PcgTeam::kNone;
+  if (n_rows && pcg_persistent_work(n_rows) <= 2 * kVecBytes && h.done == 0) {
+    SCK(launch_longest_row(n_rows, d_row_ptr, err + kErrSlots, s));
+    SCK(cudaMemcpyAsync(&longest, err + kErrSlots, sizeof longest, cudaMemcpyDeviceToHost, s));
+    SCK(cudaStreamSynchronize(s));
+    if (pcg_persistent_rows(n_rows, nnz, longest))
+      team = pcg_persistent_team(n_rows, nnz, false, true, o.launch_mode == CSTG_LAUNCH_AUTO, PcgTeam::kFirst);
+    if (o.launch_mode == CSTG_LAUNCH_GRAPH || o.launch_mode == CSTG_LAUNCH_INSTRUMENTED) team = PcgTeam::kNone;
+  }
   long long chunks = 0, spmv_calls = 0;
   bool true_done = false;
   while (h.done != CSTG_SOLVE_ZERO_RHS + 1) {
@@ -165,8 +178,17 @@ extern "C" int cstg_pcg_solve_static(int n_rows, const int32_t* d_row_ptr, const
       if (++chunks > max_chunks)
         return fail_msg(stats, CSTG_ERR_TIMEOUT, "pcg_solve_static: no end after %lld chunks", chunks);
       const int it0 = h.iter;
-      for (int k = 0; k < chunk; ++k) SCK(launch_pcg_iteration(w, nullptr, &A, s));
+      if (team != PcgTeam::kNone)
+        SCK(launch_pcg_persistent(team, w, nullptr, nullptr, &A, p, nullptr, o.max_refinements, kBarrierSpinDefault, s));
+      else
+        for (int k = 0; k < chunk; ++k) SCK(launch_pcg_iteration(w, nullptr, &A, s));
       SCK(snap());
+      if (h.done == CSTG_SOLVE_TIMEOUT + 1)
+        return fail_msg(stats, CSTG_ERR_TIMEOUT, "pcg_solve_static: a barrier of the persistent solve timed out");
+      if (team != PcgTeam::kNone && h.no_halo) {  // (nothing was done, but p was overwritten)
+        team = pcg_persistent_team(n_rows, nnz, false, true, o.launch_mode == CSTG_LAUNCH_AUTO, team);
+        if (team == PcgTeam::kNone) SCK(launch_pcg_init(w, o.rtol, o.max_iter, false, s));
+      }
       spmv_calls += h.iter - it0 + (h.done == CSTG_SOLVE_BREAKDOWN + 1);
     }
     SCK(launch_spmv(nullptr, &A, w.x, w.Ap, s));

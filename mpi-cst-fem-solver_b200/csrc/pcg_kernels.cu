@@ -361,6 +361,14 @@ __global__ void __launch_bounds__(kThreads) k_true_residual(int n, const double*
   }
 }
 
+__global__ void __launch_bounds__(kThreads) k_longest_row(int n, const int* __restrict__ row_ptr, int* longest) {
+  int m = 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    m = max(m, row_ptr[i + 1] - row_ptr[i]);
+  m = __reduce_max_sync(kFull, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(longest, m);
+}
+
 // ---- launchers --------------------------------------------------------------------------------
 
 // One full wave of `kernel` on the current device: SMs x resident blocks per SM at kThreads
@@ -414,6 +422,14 @@ cudaError_t launch_pcg_iteration(const PcgBuffers& w, const BlockMatrix* bm,
                                               w.st, w.history);
   k_pupdate<<<wave_grid<k_pupdate>(), kThreads, 0, s>>>(w.n, w.r, w.inv_diag, w.p, w.st);
   count_launches(2);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_longest_row(int n, const int* row_ptr, int* longest, cudaStream_t s) {
+  const cudaError_t e = cudaMemsetAsync(longest, 0, sizeof(int), s);
+  if (e != cudaSuccess) return e;
+  k_longest_row<<<std::min((n + kThreads - 1) / kThreads, kSMs), kThreads, 0, s>>>(n, row_ptr, longest);
+  count_launches(1);
   return cudaGetLastError();
 }
 
