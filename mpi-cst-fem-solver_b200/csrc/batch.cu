@@ -19,13 +19,26 @@
 // operator stops improving the true residual (or fails more checks than max_refinements)
 // switches to the FP64 operator with one restart.
 //
-// Vectors are interleaved per node: [node][load case][2] doubles, so one neighbour gather
-// serves all load cases and every matrix block is read once per iteration for all of them.
+// Vectors are interleaved per node: [node][load case][2] doubles, so every matrix block is read once
+// per iteration for all load cases.
+//
+// Two kernels. k_batch_halo keeps p of a block's own nodes and of its halo (the neighbours' nodes that
+// its rows read) in shared memory for all load cases, forms p = z + beta p there itself, and so needs
+// two reductions an iteration and passes only z between blocks; r, Ap and x follow as far as they fit.
+// It is bound by the L2 traffic of what does not (x, the matrix) and the shared-memory gathers of p:
+// 38 us an iteration for 20,301 nodes x 4 cases on 8 SMs, against about 100 us for k_batch_pcg, which
+// gathers p through L2 and runs three phases (64 plates of n_r 20 .. 100: 177 against 382 ms). Larger
+// plates, whose p does not fit, run faster with all cases on k_batch_pcg than with a case or two
+// at a time here (n_r 20 .. 200: 2.1 against 3.6 s), so a batch that holds one goes there as a whole; a
+// single plate whose numbering makes its halo too large is put on a list for it.
 #include <cooperative_groups.h>
 
 #include "../../include/cstfem_b200.h"
 #include "common.cuh"
 #include "kernels.h"
+
+#include <algorithm>
+#include <cmath>
 
 namespace cg = cooperative_groups;
 
@@ -97,8 +110,8 @@ __global__ void __launch_bounds__(T, (T >= 512 ? 1 : 512 / T)) k_batch_pcg(const
 
   for (;;) {
     if (crank == 0 && threadIdx.x == 0) {
-      const int q = atomicAdd(a.queue, 1);
-      s_plate = q < a.n_sys ? a.order[q] : -1;
+      const int q = atomicAdd(a.queue + 1, 1);
+      s_plate = q < (a.n_rest ? *a.n_rest : a.n_sys) ? (a.n_rest ? a.rest[q] : a.order[q]) : -1;
     }
     cl.sync();
     const int plate = *cl.map_shared_rank(&s_plate, 0);
@@ -401,6 +414,575 @@ __global__ void __launch_bounds__(T, (T >= 512 ? 1 : 512 / T)) k_batch_pcg(const
   cl.sync();  // no CTA leaves while another may still read its shared memory
 }
 
+// ---- plates whose p fits in shared memory ----------------------------------------------------------
+
+constexpr int kHaloHash = 8192;  // slots of the halo's hash set; a halo holds at most half as many
+
+template <int R, int T>
+struct HaloShared {
+  double wsum[T / 32][2 * R];
+  double inbox[2][16][2 * R];  // every block's sums, double-buffered
+  double alpha[R], beta[R], xalpha[R];  // xalpha: step of x not yet taken
+  // per load case, kept by lane q of warp 0 (the same values in every block)
+  double rz[R], bn2[R], rel[R], true_rel[R], prev_true[R], rmax[R];
+  int it[R], nref[R], nfail[R], last_rep[R], status[R];
+  unsigned active, repl;
+  int fp64, plate, halo;
+  int scan[T / 32];
+};
+
+// Cluster-wide sums of V values per thread: lane i < V of warp 0 gets sum i (the others nothing). The
+// values are halved over the lanes on the way down, so a warp adds 7 + 2 numbers instead of 8 x 5.
+template <int V, int R, int T>
+__device__ __forceinline__ double cluster_totals(const cg::cluster_group& cl, HaloShared<R, T>& sh, unsigned& seq,
+                                                 const double (&v)[V]) {
+  constexpr int P = V <= 2 ? 2 : V <= 4 ? 4 : 8, kPart = 32 / P;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int idx = lane / kPart, part = lane % kPart;
+  double a[P];
+#pragma unroll
+  for (int j = 0; j < P; ++j) a[j] = j < V ? v[j] : 0.0;
+  int o = 16;
+#pragma unroll
+  for (int h = P / 2; h > 0; h >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int j = 0; j < h; ++j) {
+      const double give = up ? a[j] : a[j + h];
+      a[j] = (up ? a[j + h] : a[j]) + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+#pragma unroll
+  for (int k = kPart / 2; k > 0; k >>= 1) a[0] += __shfl_xor_sync(0xffffffffu, a[0], k);
+  if (part == 0 && idx < V) sh.wsum[w][idx] = a[0];
+  ++seq;
+  __syncthreads();
+  const int C = (int)cl.num_blocks();
+  double(*box)[2 * R] = sh.inbox[seq & 1u];
+  if (w == 0) {
+    double s = 0.0;
+    if (idx < V)
+      for (int k = part; k < T / 32; k += kPart) s += sh.wsum[k][idx];
+#pragma unroll
+    for (int k = kPart / 2; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+    if (idx < V)
+      for (int c = part; c < C; c += kPart) *cl.map_shared_rank(&box[cl.block_rank()][idx], c) = s;
+  }
+  cl.sync();  // release / acquire at cluster scope: sums and vectors
+  double s = 0.0;
+  if (w == 0) {
+    if (idx < V)
+      for (int c = part; c < C; c += kPart) s += box[c][idx];
+#pragma unroll
+    for (int k = kPart / 2; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+    s = __shfl_sync(0xffffffffu, s, (lane * kPart) & 31);
+  }
+  return s;
+}
+
+// A block's own vector of G load cases: [node][case] (IT) or [case][node], the first `lim` nodes in
+// shared memory, the others in the interleaved global array.
+template <int G, bool IT>
+struct OwnCases {
+  double2* s;
+  double2* g;      // at the block's first node
+  int lim, pitch;  // (pitch of a case in shared memory)
+  __device__ __forceinline__ double2& at(int i, int q) const {
+    return i < lim ? s[IT ? i * G + q : q * pitch + i] : g[(size_t)i * G + q];
+  }
+};
+
+// Slots of a case's array: a multiple of 8 plus 8 / G, so that the 8 lanes of a shared-memory phase
+// that hold consecutive (node, case) items hit different banks.
+template <int G>
+__device__ __forceinline__ int case_pitch(int n) {
+  return (n + 7) / 8 * 8 + (G == 1 ? 0 : 8 / G);
+}
+
+// All load cases of a plate; dyn: shared memory from the end of the halo's list on.
+template <int R, int T>
+__device__ __forceinline__ void solve_cases(const BatchArgs& a, const cg::cluster_group& cl, HaloShared<R, T>& sh,
+                                            unsigned& seq, unsigned char* dyn, unsigned smem, int n0,
+                                            int cnt, int nh, const int* hid, const unsigned* want, int plate) {
+  constexpr int G = R, V = 2 * G;
+  constexpr int kItems = T / G * G;  // threads of the item loops: a thread keeps its load case
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int tq = tid % G, tn = tid < kItems ? tid / G : 1 << 30;
+  constexpr int kStep = T / G;
+  const double2* __restrict__ invd2 = reinterpret_cast<const double2*>(a.inv_diag) + n0;
+  const double2* __restrict__ v64 = reinterpret_cast<const double2*>(a.A64.vals);
+  const double rtol2 = a.rtol * a.rtol;
+  const size_t base = (size_t)n0 * R;
+  double2* zg = reinterpret_cast<double2*>(a.p);  // z of wanted nodes, in p's array
+  const double2* bg = reinterpret_cast<const double2*>(a.b) + base;
+
+  unsigned used = 0;
+  const int pitch = case_pitch<G>(cnt + nh);
+  double2* p = reinterpret_cast<double2*>(dyn);
+  used += (unsigned)pitch * G * 16u;
+  auto room = [&]() { return smem > used ? (int)min((smem - used) / (16u * G), (unsigned)cnt) : 0; };
+  OwnCases<G, true> r, x;
+  OwnCases<G, false> Ap;
+  r.g = reinterpret_cast<double2*>(a.r) + base;
+  x.g = reinterpret_cast<double2*>(a.x) + base;
+  Ap.g = reinterpret_cast<double2*>(a.Ap) + base;
+  r.pitch = x.pitch = 0;
+  r.lim = room();
+  r.s = reinterpret_cast<double2*>(dyn + used);
+  used += (unsigned)r.lim * G * 16u;
+  Ap.lim = max(0, room() - 16);
+  Ap.pitch = case_pitch<G>(Ap.lim);
+  Ap.s = reinterpret_cast<double2*>(dyn + used);
+  if (Ap.lim > 0) used += (unsigned)Ap.pitch * G * 16u;
+  x.lim = room();
+  x.s = reinterpret_cast<double2*>(dyn + used);
+
+  // x = 0, r = b, p = D^-1 b; r'z and b'b per load case (solver.cpp:42-58)
+  double v[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) v[i] = 0.0;
+  double s0 = 0.0, s1 = 0.0;
+  for (int i = tn; i < cnt; i += kStep) {
+    const double2 d = invd2[i], bk = bg[(size_t)i * R + tq];
+    const double2 z = make_double2(d.x * bk.x, d.y * bk.y);
+    x.at(i, tq) = make_double2(0.0, 0.0);
+    r.at(i, tq) = bk;
+    p[tq * pitch + i] = z;
+    s0 = dot2(bk, z, s0);
+    s1 = dot2(bk, bk, s1);
+  }
+  for (int j = tn; j < nh; j += kStep) {
+    const int m = hid[j];
+    const double2 d = reinterpret_cast<const double2*>(a.inv_diag)[m];
+    const double2 bk = reinterpret_cast<const double2*>(a.b)[(size_t)m * R + tq];
+    p[tq * pitch + cnt + j] = make_double2(d.x * bk.x, d.y * bk.y);
+  }
+#pragma unroll
+  for (int q = 0; q < G; ++q) {
+    v[q] = q == tq ? s0 : 0.0;
+    v[G + q] = q == tq ? s1 : 0.0;
+  }
+  {
+    const double t = cluster_totals<V>(cl, sh, seq, v);
+    const double t2 = __shfl_sync(0xffffffffu, t, (lane + G) & 31);
+    if (tid < 32) {
+      const bool mine = lane < G;
+      if (mine) {
+        sh.rz[lane] = t;
+        sh.bn2[lane] = sh.rmax[lane] = t2;
+        sh.alpha[lane] = sh.beta[lane] = sh.xalpha[lane] = 0.0;
+        sh.it[lane] = sh.nref[lane] = sh.nfail[lane] = sh.last_rep[lane] = 0;
+        sh.prev_true[lane] = INFINITY;
+        sh.true_rel[lane] = 0.0;
+        sh.rel[lane] = t2 > 0.0 ? 1.0 : 0.0;
+        sh.status[lane] = t2 > 0.0 ? CSTG_SOLVE_CONVERGED : CSTG_SOLVE_ZERO_RHS;  // x = 0 is exact
+      }
+      const unsigned act = __ballot_sync(0xffffffffu, mine && t2 > 0.0);
+      if (lane == 0) {
+        sh.active = act;
+        sh.fp64 = a.start_fp64 != 0;
+      }
+    }
+    __syncthreads();
+  }
+
+  for (bool begun = false; sh.active; begun = true) {
+    // ---- Phase 1: the step of x of the iteration before, p = z + beta p at own nodes and halo
+    if (begun) {
+      const double beta = sh.beta[tq], xa = sh.xalpha[tq];
+      if ((sh.active >> tq) & 1u) {
+        constexpr int kU = 4;
+        for (int j0 = tn; j0 < nh; j0 += kU * kStep) {
+          double2 z[kU];
+#pragma unroll
+          for (int u = 0; u < kU; ++u)
+            z[u] = __ldcg(&zg[(size_t)hid[min(j0 + u * kStep, nh - 1)] * R + tq]);
+#pragma unroll
+          for (int u = 0; u < kU; ++u) {
+            const int j = j0 + u * kStep;
+            if (j >= nh) break;
+            double2& pj = p[tq * pitch + cnt + j];
+            pj = make_double2(fma(beta, pj.x, z[u].x), fma(beta, pj.y, z[u].y));
+          }
+        }
+        for (int i0 = tn; i0 < cnt; i0 += kU * kStep) {
+          double2 xi[kU], ri[kU], di[kU];
+#pragma unroll
+          for (int u = 0; u < kU; ++u) {
+            const int i = min(i0 + u * kStep, cnt - 1);
+            xi[u] = x.at(i, tq);
+            ri[u] = r.at(i, tq);
+            di[u] = __ldg(&invd2[i]);
+          }
+#pragma unroll
+          for (int u = 0; u < kU; ++u) {
+            const int i = i0 + u * kStep;
+            if (i >= cnt) break;
+            double2& pi = p[tq * pitch + i];
+            x.at(i, tq) = make_double2(fma(xa, pi.x, xi[u].x), fma(xa, pi.y, xi[u].y));
+            pi = make_double2(fma(beta, pi.x, di[u].x * ri[u].x), fma(beta, pi.y, di[u].y * ri[u].y));
+          }
+        }
+      }
+      __syncthreads();
+    }
+    // Ap = A p and p'Ap: a thread per node, all load cases (the matrix row is read once)
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] = 0.0;
+    double pap[G];
+#pragma unroll
+    for (int q = 0; q < G; ++q) pap[q] = 0.0;
+    const bool fp64 = sh.fp64 != 0;
+    for (int i = tid; i < cnt; i += T) {
+      const int n = n0 + i;
+      const int b0 = __ldg(&a.A64.node_ptr[n]), deg = __ldg(&a.A64.node_ptr[n + 1]) - b0;
+      const unsigned short* sl = a.slots + (b0 - n);
+      double2 y[G], pn[G];
+#pragma unroll
+      for (int q = 0; q < G; ++q) {
+        y[q] = make_double2(0.0, 0.0);
+        pn[q] = p[q * pitch + i];
+      }
+      if (fp64) {
+        const double2 *ra = v64 + 2L * b0, *rb = ra + deg;
+        int off = 0;  // slots are of the off-diagonal blocks only
+        for (int k = 0; k < deg; ++k) {
+          const int slot = __ldg(&a.A64.bnbr[b0 + k]) == n ? i : (int)sl[off++];
+          const double2 ka = __ldg(ra + k), kb = __ldg(rb + k);
+#pragma unroll
+          for (int q = 0; q < G; ++q) {
+            const double2 pm = p[q * pitch + slot];
+            y[q].x = dot2(ka, pm, y[q].x);
+            y[q].y = dot2(kb, pm, y[q].y);
+          }
+        }
+      } else {
+        const int c = deg - 1;
+        const float4* f4 = a.A32.val32 + (b0 - n);
+        constexpr int kN = 3;  // neighbours whose matrix loads are in flight together
+        for (int k0 = 0; k0 < c; k0 += kN) {
+          int slot[kN];
+          float4 f[kN];
+#pragma unroll
+          for (int u = 0; u < kN; ++u) {
+            const int k = min(k0 + u, c - 1);
+            slot[u] = k0 + u < c ? (int)sl[k] : i;  // (the node itself: a zero difference)
+            f[u] = __ldg(f4 + k);
+          }
+#pragma unroll
+          for (int u = 0; u < kN; ++u) {
+#pragma unroll
+            for (int q = 0; q < G; ++q) {
+              const double2 pm = p[q * pitch + slot[u]];
+              const double dx = pm.x - pn[q].x, dy = pm.y - pn[q].y;
+              y[q].x = fma((double)f[u].x, dx, fma((double)f[u].y, dy, y[q].x));
+              y[q].y = fma((double)f[u].z, dx, fma((double)f[u].w, dy, y[q].y));
+            }
+          }
+        }
+        const double2 sa = __ldg(&a.A32.S64[2 * n]), sb = __ldg(&a.A32.S64[2 * n + 1]);
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+          y[q].x = dot2(sa, pn[q], y[q].x);
+          y[q].y = dot2(sb, pn[q], y[q].y);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < G; ++q) {
+        Ap.at(i, q) = y[q];
+        pap[q] = dot2(pn[q], y[q], pap[q]);
+      }
+    }
+    {
+      const double t = cluster_totals<G>(cl, sh, seq, pap);
+      if (tid < 32) {
+        bool on = false;
+        if (lane < G) {
+          on = (sh.active >> lane) & 1u;
+          if (on && !(t > 0.0)) {  // solver.cpp:64-68
+            sh.status[lane] = CSTG_SOLVE_BREAKDOWN;
+            on = false;
+          }
+          sh.alpha[lane] = sh.xalpha[lane] = on ? sh.rz[lane] / t : 0.0;
+        }
+        const unsigned act = __ballot_sync(0xffffffffu, on);
+        if (lane == 0) sh.active = act;
+      }
+      __syncthreads();
+    }
+    if (!sh.active) break;
+
+    // ---- Phase 2: r -= alpha Ap, z = D^-1 r; r'z and r'r
+    {
+      const double alpha = sh.alpha[tq];
+      s0 = s1 = 0.0;
+      constexpr int kU = 4;
+      if ((sh.active >> tq) & 1u)
+        for (int i0 = tn; i0 < cnt; i0 += kU * kStep) {
+          double2 ri[kU], di[kU];
+#pragma unroll
+          for (int u = 0; u < kU; ++u) {
+            const int i = min(i0 + u * kStep, cnt - 1);
+            const double2 ai = Ap.at(i, tq);
+            ri[u] = r.at(i, tq);
+            ri[u] = make_double2(fma(-alpha, ai.x, ri[u].x), fma(-alpha, ai.y, ri[u].y));
+            di[u] = __ldg(&invd2[i]);
+          }
+#pragma unroll
+          for (int u = 0; u < kU; ++u) {
+            const int i = i0 + u * kStep;
+            if (i >= cnt) break;
+            const double2 z = make_double2(di[u].x * ri[u].x, di[u].y * ri[u].y);
+            r.at(i, tq) = ri[u];
+            if ((want[i >> 5] >> (i & 31)) & 1u) __stcg(&zg[(size_t)(n0 + i) * R + tq], z);
+            s0 = dot2(ri[u], z, s0);
+            s1 = dot2(ri[u], ri[u], s1);
+          }
+        }
+#pragma unroll
+      for (int q = 0; q < G; ++q) {
+        v[q] = q == tq ? s0 : 0.0;
+        v[G + q] = q == tq ? s1 : 0.0;
+      }
+      const double t = cluster_totals<V>(cl, sh, seq, v);
+      const double rr = __shfl_sync(0xffffffffu, t, (lane + G) & 31);
+      if (tid < 32) {
+        // Which load cases need the FP64 true residual now (see k_batch_pcg): a convergence check or
+        // a reliable update; the others go on with beta.
+        bool chk = false, rep = false;
+        if (lane < G && ((sh.active >> lane) & 1u)) {
+          const int it = ++sh.it[lane];
+          sh.rel[lane] = sqrt(rr / sh.bn2[lane]);
+          const double rm = fmax(sh.rmax[lane], rr);
+          sh.rmax[lane] = rm;
+          if (rr <= rtol2 * sh.bn2[lane] || it >= a.max_iter) {
+            chk = true;
+          } else if (rr <= kBatchDelta2 * rm || it - sh.last_rep[lane] >= kBatchCycle) {
+            rep = true;
+          } else {
+            sh.beta[lane] = t / sh.rz[lane];
+            sh.rz[lane] = t;
+          }
+        }
+        const unsigned c = __ballot_sync(0xffffffffu, chk), m = __ballot_sync(0xffffffffu, rep);
+        if (lane == 0) sh.repl = (c | m) | c << 16;
+      }
+      __syncthreads();
+    }
+    const unsigned repl = sh.repl & 0xffffu, check = sh.repl >> 16;
+    if (repl) {
+      // ---- Phase R: FP64 true residual r = b - A x for the replaced load cases
+      if ((repl >> tq) & 1u) {
+        const double xa = sh.xalpha[tq];
+        for (int i = tn; i < cnt; i += kStep) {
+          const double2 pi = p[tq * pitch + i];
+          double2 xi = x.at(i, tq);
+          xi = make_double2(fma(xa, pi.x, xi.x), fma(xa, pi.y, xi.y));
+          x.at(i, tq) = xi;
+          __stcg(&x.g[(size_t)i * R + tq], xi);
+        }
+      }
+      cl.sync();  // x visible to the other blocks
+      if (tid < G && ((repl >> tid) & 1u)) sh.xalpha[tid] = 0.0;
+#pragma unroll
+      for (int i = 0; i < V; ++i) v[i] = 0.0;
+      for (int i = tid; i < cnt; i += T) {
+        const int n = n0 + i;
+        const double2 d = invd2[i];
+        const int b0 = __ldg(&a.A64.node_ptr[n]), deg = __ldg(&a.A64.node_ptr[n + 1]) - b0;
+        const double2 *ra = v64 + 2L * b0, *rb = ra + deg;
+        double2 t[G];
+#pragma unroll
+        for (int q = 0; q < G; ++q) t[q] = make_double2(0.0, 0.0);
+        for (int k = 0; k < deg; ++k) {
+          const int m = __ldg(&a.A64.bnbr[b0 + k]);
+          const double2 ka = __ldg(ra + k), kb = __ldg(rb + k);
+#pragma unroll
+          for (int q = 0; q < G; ++q) {
+            if (!((repl >> q) & 1u)) continue;
+            const double2 xm = __ldcg(reinterpret_cast<const double2*>(a.x) + (size_t)m * R + q);
+            t[q].x = dot2(ka, xm, t[q].x);
+            t[q].y = dot2(kb, xm, t[q].y);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+          if (!((repl >> q) & 1u)) continue;
+          const double2 bk = bg[(size_t)i * R + q];
+          const double2 rk = make_double2(bk.x - t[q].x, bk.y - t[q].y);
+          const double2 z = make_double2(d.x * rk.x, d.y * rk.y);
+          r.at(i, q) = rk;
+          if ((want[i >> 5] >> (i & 31)) & 1u) __stcg(&zg[(size_t)n * R + q], z);
+          v[q] = dot2(rk, rk, v[q]);
+          v[G + q] = dot2(rk, z, v[G + q]);
+        }
+      }
+      const double rr = cluster_totals<V>(cl, sh, seq, v);
+      const double rzn = __shfl_sync(0xffffffffu, rr, (lane + G) & 31);
+      if (tid < 32) {
+        bool off = false, restart = false;
+        if (lane < G && ((repl >> lane) & 1u)) {
+          const bool is_check = (check >> lane) & 1u;
+          const double tr = sqrt(rr / sh.bn2[lane]);
+          sh.true_rel[lane] = tr;
+          if (is_check && rr <= rtol2 * sh.bn2[lane]) {
+            sh.status[lane] = CSTG_SOLVE_CONVERGED;
+            off = true;
+          } else if (sh.it[lane] >= a.max_iter) {
+            sh.status[lane] = CSTG_SOLVE_MAX_ITER;
+            off = true;
+          } else {
+            ++sh.nref[lane];
+            sh.last_rep[lane] = sh.it[lane];
+            sh.rmax[lane] = rr;
+            sh.rel[lane] = tr;
+            if (is_check) {  // the recursive residual met rtol but the true one did not
+              ++sh.nfail[lane];
+              // the FP32 operator's accuracy floor: FP64 from here, restarted
+              restart = !fp64 && (sh.nfail[lane] > a.max_refine || tr > 0.5 * sh.prev_true[lane]);
+              sh.prev_true[lane] = tr;
+            }
+            sh.beta[lane] = rzn / sh.rz[lane];
+            sh.rz[lane] = rzn;
+          }
+        }
+        const unsigned gone = __ballot_sync(0xffffffffu, off), again = __ballot_sync(0xffffffffu, restart);
+        if (again && lane < G) sh.beta[lane] = 0.0;
+        if (lane == 0) {
+          sh.active &= ~gone;
+          if (again) sh.fp64 = 1;
+        }
+      }
+      __syncthreads();
+    }
+  }
+
+  // x of the load cases that did not end in a check (breakdown: the step before is already in)
+  for (int i = tn; i < cnt; i += kStep)
+    if (i < x.lim) x.g[(size_t)i * R + tq] = x.s[i * G + tq];
+  if (cl.block_rank() == 0 && tid < G) {
+    BatchResultDev o;
+    o.iterations = sh.it[tid];
+    o.status = sh.status[tid];
+    o.refinements = sh.nref[tid];
+    o.fp64 = sh.fp64 != 0;
+    o.rel = sh.rel[tid];
+    o.true_rel = sh.true_rel[tid];
+    a.res[(size_t)plate * a.res_stride + a.res_offset + tid] = o;
+  }
+  __syncthreads();
+}
+
+template <int R, int T>
+__global__ void __launch_bounds__(T, 1) k_batch_halo(const BatchArgs a) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  __shared__ HaloShared<R, T> sh;
+  const cg::cluster_group cl = cg::this_cluster();
+  const int crank = (int)cl.block_rank(), C = (int)cl.num_blocks();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned seq = 0;
+  for (;;) {
+    if (crank == 0 && tid == 0) {
+      const int q = atomicAdd(a.queue, 1);
+      sh.plate = q < a.n_sys ? a.order[q] : -1;
+    }
+    cl.sync();
+    const int plate = *cl.map_shared_rank(&sh.plate, 0);
+    if (plate < 0) break;
+    const int p0 = a.sys_node[plate], np = a.sys_node[plate + 1] - p0;
+    const int n0 = p0 + (int)((long long)np * crank / C), n1 = p0 + (int)((long long)np * (crank + 1) / C);
+    const int cnt = n1 - n0;
+
+    // -- the halo: nodes outside [n0, n1) among the rows' neighbours, in a hash set keyed by their low
+    // bits (so the compacted list keeps runs of consecutive nodes together)
+    int* hid = reinterpret_cast<int*>(dyn);
+    int* keys = reinterpret_cast<int*>(dyn + a.smem) - kHaloHash;
+    unsigned short* slot = reinterpret_cast<unsigned short*>(keys) - kHaloHash;
+    const int e0 = cnt > 0 ? a.A64.node_ptr[n0] : 0, e1 = cnt > 0 ? a.A64.node_ptr[n1] : 0;
+    const int want_words = (cnt + 31) / 32;
+    for (int i = tid; i < kHaloHash; i += T) keys[i] = -1;
+    if (tid == 0) sh.halo = 0;
+    __syncthreads();
+    volatile int* count = &sh.halo;
+    for (int e = e0 + tid; e < e1 && *count <= kHaloHash / 2; e += T) {
+      const int m = a.A64.bnbr[e];
+      if (m >= n0 && m < n1) continue;
+      for (int h = m & (kHaloHash - 1);; h = (h + 1) & (kHaloHash - 1)) {
+        const int k = atomicCAS(&keys[h], -1, m);
+        if (k == -1) atomicAdd(&sh.halo, 1);
+        if (k == -1 || k == m) break;
+      }
+    }
+    __syncthreads();
+    const int nh = sh.halo;
+    // p of all load cases must fit beside the halo's list and the wanted bits, in every block
+    const unsigned head = (((unsigned)nh + (unsigned)want_words) * 4u + 15u) & ~15u;
+    const bool fits = nh <= kHaloHash / 2 && cnt + nh <= 65535 &&
+                      (long long)head + 16LL * R * case_pitch<R>(cnt + nh) <= (long long)a.smem;
+    bool all = true;
+    ++seq;
+    if (tid < C) *cl.map_shared_rank(&sh.inbox[seq & 1u][crank][0], tid) = fits ? 1.0 : 0.0;
+    cl.sync();
+    for (int c = 0; c < C; ++c) all &= sh.inbox[seq & 1u][c][0] != 0.0;
+    if (!all) {
+      if (crank == 0 && tid == 0) a.rest[atomicAdd(a.n_rest, 1)] = plate;
+      continue;
+    }
+    {
+      constexpr int per = kHaloHash / T;
+      int mine = 0;
+      for (int k = 0; k < per; ++k) mine += keys[tid * per + k] >= 0;
+      int s = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += t;
+      }
+      if (lane == 31) sh.scan[warp] = s;
+      __syncthreads();
+      int at = s - mine;
+      for (int k = 0; k < warp; ++k) at += sh.scan[k];
+      for (int k = 0; k < per; ++k) {
+        const int h = tid * per + k, m = keys[h];
+        if (m >= 0) {
+          hid[at] = m;
+          a.wanted[m] = 1;
+          slot[h] = (unsigned short)(cnt + at);
+          ++at;
+        }
+      }
+      __syncthreads();
+      // slots of the off-diagonal blocks, numbered as the FP32 operator's
+      for (int i = tid; i < cnt; i += T) {
+        const int n = n0 + i, b0 = a.A64.node_ptr[n], b1 = a.A64.node_ptr[n + 1];
+        int o = b0 - n;
+        for (int e = b0; e < b1; ++e) {
+          const int m = a.A64.bnbr[e];
+          if (m == n) continue;
+          unsigned short s16;
+          if (m >= n0 && m < n1) {
+            s16 = (unsigned short)(m - n0);
+          } else {
+            int h = m & (kHaloHash - 1);
+            while (keys[h] != m) h = (h + 1) & (kHaloHash - 1);
+            s16 = slot[h];
+          }
+          a.slots[o++] = s16;
+        }
+      }
+    }
+    cl.sync();  // the wanted marks of all blocks
+    unsigned* want = reinterpret_cast<unsigned*>(hid + nh);
+    for (int i0 = warp * 32; i0 < cnt; i0 += T) {
+      const unsigned m = __ballot_sync(0xffffffffu, i0 + lane < cnt && __ldcg(a.wanted + n0 + i0 + lane));
+      if (lane == 0) want[i0 / 32] = m;
+    }
+    __syncthreads();
+    solve_cases<R, T>(a, cl, sh, seq, dyn + head, a.smem - head, n0, cnt, nh, hid, want, plate);
+  }
+  cl.sync();  // no block leaves while another may still read or write its shared memory
+}
+
 // [rhs][2N] (ld doubles apart) <-> [node][R][2] for load cases q0 .. q0 + R - 1
 __global__ void k_batch_pack(int N, int R, int q0, long long ld, const double* __restrict__ src,
                              double2* __restrict__ dst) {
@@ -456,12 +1038,26 @@ int grid_for(long long work) {
 }
 
 template <int R, int T>
-cudaError_t launch_shape(const BatchArgs* a, int cluster, int n_clusters, int* max_clusters,
+cudaError_t launch_shape(const BatchArgs* a, int cluster, const int* n_clusters, int* max_clusters,
                          cudaStream_t s) {
   auto kern = k_batch_pcg<R, T>;
   if (cluster > 8 && max_clusters) {  // the shape query always precedes a launch (never in a capture)
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
+  }
+  auto halo = k_batch_halo<R, T>;
+  unsigned smem = 0;
+  {
+    int dev = 0, most = 0;
+    cudaGetDevice(&dev);
+    cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e != cudaSuccess) return e;
+    smem = (unsigned)(most - (int)sizeof(HaloShared<R, T>)) / 1024u * 1024u;
+    if (max_clusters) {
+      e = cudaFuncSetAttribute(halo, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(halo, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e != cudaSuccess) return e;
+    }
   }
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
@@ -476,15 +1072,37 @@ cudaError_t launch_shape(const BatchArgs* a, int cluster, int n_clusters, int* m
   cfg.numAttrs = 1;
   if (max_clusters) {
     cfg.gridDim = dim3((unsigned)cluster);
+    int n = 0;
     *max_clusters = 0;
-    return cudaOccupancyMaxActiveClusters(max_clusters, (void*)kern, &cfg);
+    cudaError_t e = cudaOccupancyMaxActiveClusters(&n, (void*)kern, &cfg);
+    if (e != cudaSuccess) return e;
+    *max_clusters = n;
+    cfg.dynamicSmemBytes = smem;
+    e = cudaOccupancyMaxActiveClusters(&n, (void*)halo, &cfg);
+    max_clusters[1] = e == cudaSuccess ? n : 0;
+    return e;
   }
-  cfg.gridDim = dim3((unsigned)(n_clusters * cluster));
-  return cudaLaunchKernelEx(&cfg, kern, *a);
+  BatchArgs b = *a;
+  b.smem = smem;
+  // by the largest plate and a halo of a few rows of nodes (a plate that then does not fit is listed)
+  const double own = std::ceil((double)a->largest / cluster), nodes = own + 3.0 * std::sqrt((double)a->largest) + 64.0;
+  if (nodes * (16.0 * R + 4.0) + 4096.0 <= (double)smem) {
+    cfg.dynamicSmemBytes = smem;
+    cfg.gridDim = dim3((unsigned)(std::min(n_clusters[1], a->n_sys) * cluster));
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, halo, b);
+    if (e != cudaSuccess) return e;
+    count_launches(1);
+    cfg.dynamicSmemBytes = 0;
+  } else {
+    b.n_rest = nullptr;
+  }
+  cfg.gridDim = dim3((unsigned)(std::min(n_clusters[0], a->n_sys) * cluster));
+  count_launches(1);
+  return cudaLaunchKernelEx(&cfg, kern, b);
 }
 
 template <int R>
-cudaError_t launch_r(const BatchArgs* a, int cluster, int threads, int n_clusters, int* max_clusters,
+cudaError_t launch_r(const BatchArgs* a, int cluster, int threads, const int* n_clusters, int* max_clusters,
                      cudaStream_t s) {
   switch (threads) {
     case 256: return launch_shape<R, 256>(a, cluster, n_clusters, max_clusters, s);
@@ -493,7 +1111,7 @@ cudaError_t launch_r(const BatchArgs* a, int cluster, int threads, int n_cluster
   }
 }
 
-cudaError_t dispatch(const BatchArgs* a, int R, int cluster, int threads, int n_clusters, int* max_clusters,
+cudaError_t dispatch(const BatchArgs* a, int R, int cluster, int threads, const int* n_clusters, int* max_clusters,
                      cudaStream_t s) {
   if (cluster < 1 || cluster > 16) return cudaErrorInvalidValue;
   switch (R) {
@@ -508,14 +1126,12 @@ cudaError_t dispatch(const BatchArgs* a, int R, int cluster, int threads, int n_
 }  // namespace
 
 cudaError_t batch_max_clusters(int R, int cluster, int threads, int* n) {
-  return dispatch(nullptr, R, cluster, threads, 0, n, nullptr);
+  return dispatch(nullptr, R, cluster, threads, nullptr, n, nullptr);
 }
 
-cudaError_t launch_batch_pcg(const BatchArgs& a, int R, int cluster, int threads, int n_clusters,
+cudaError_t launch_batch_pcg(const BatchArgs& a, int R, int cluster, int threads, const int* n_clusters,
                              cudaStream_t s) {
-  const cudaError_t e = dispatch(&a, R, cluster, threads, n_clusters, nullptr, s);
-  if (e == cudaSuccess) count_launches(1);
-  return e;
+  return dispatch(&a, R, cluster, threads, n_clusters, nullptr, s);
 }
 
 cudaError_t launch_batch_pack(int N, int R, int q0, long long ld, const double* src, double* dst,

@@ -58,7 +58,9 @@ int prepare(cstg_ctx* ctx, int n_sys, const int32_t* offs, int n_rhs, const cstg
   const size_t vec = sizeof(double) * (size_t)ctx->n_rows * group;
   ENSURE(ctx->bat_sys, sizeof(int) * table.size());
   ENSURE(ctx->bat_order, sizeof(int) * (size_t)n_sys);
-  ENSURE(ctx->bat_queue, 256);
+  ENSURE(ctx->bat_queue, sizeof(int) * ((size_t)n_sys + 64));
+  ENSURE(ctx->bat_wanted, (size_t)ctx->n_nodes);
+  ENSURE(ctx->bat_slots, sizeof(unsigned short) * (size_t)(ctx->nnz / 4));
   ENSURE(ctx->bat_b, vec);
   ENSURE(ctx->bat_x, vec);
   ENSURE(ctx->bat_r, vec);
@@ -99,19 +101,25 @@ int prepare(cstg_ctx* ctx, int n_sys, const int32_t* offs, int n_rhs, const cstg
 // Enqueues one batched solve: per group of up to four load cases, pack, the persistent launch,
 // unpack. `launched` receives the number of kernel launches enqueued.
 int enqueue(cstg_ctx* ctx, int n_sys, int n_rhs, const double* d_b, double* d_x, const cstg_solver_options& o,
-            Shape sh, int n_clusters, long long* launched) {
+            Shape sh, const int* n_clusters, long long* launched) {
   const int N = ctx->n_nodes;
   const long long ld = ctx->n_rows;
-  long long k = 0;
+  const long long before = launches_total();
   for (int q0 = 0; q0 < n_rhs; q0 += kMaxGroup) {
     const int R = std::min(kMaxGroup, n_rhs - q0);
-    CK(cudaMemsetAsync(ctx->bat_queue.p, 0, sizeof(int), ctx->stream));
+    CK(cudaMemsetAsync(ctx->bat_queue.p, 0, sizeof(int) * 64, ctx->stream));
+    CK(cudaMemsetAsync(ctx->bat_wanted.p, 0, (size_t)N, ctx->stream));
     CK(launch_batch_pack(N, R, q0, ld, d_b, buf_ptr<double>(ctx->bat_b), ctx->stream));
     BatchArgs a;
     a.n_sys = n_sys;
     a.sys_node = buf_ptr<int>(ctx->bat_sys);
     a.order = buf_ptr<int>(ctx->bat_order);
     a.queue = buf_ptr<int>(ctx->bat_queue);
+    a.n_rest = a.queue + 2;
+    for (int p = 0; p < n_sys; ++p) a.largest = std::max(a.largest, ctx->bat_offsets[p + 1] - ctx->bat_offsets[p]);
+    a.rest = a.queue + 64;
+    a.wanted = buf_ptr<unsigned char>(ctx->bat_wanted);
+    a.slots = buf_ptr<unsigned short>(ctx->bat_slots);
     if (o.precision == CSTG_PRECISION_MIXED) a.A32 = mixed_view(ctx);
     a.A64 = block_view(ctx);
     a.start_fp64 = o.precision == CSTG_PRECISION_FP64;
@@ -129,44 +137,43 @@ int enqueue(cstg_ctx* ctx, int n_sys, int n_rhs, const double* d_b, double* d_x,
     a.res_offset = q0;
     CK(launch_batch_pcg(a, R, sh.cluster, sh.threads, n_clusters, ctx->stream));
     CK(launch_batch_unpack(N, R, q0, ld, buf_ptr<double>(ctx->bat_x), d_x, ctx->stream));
-    k += N > 0 ? 3 : 1;
   }
-  *launched = k;
+  *launched = launches_total() - before;
   return CSTG_OK;
 }
 
-int fit_shape(cstg_ctx* ctx, int n_rhs, Shape sh, int* max_clusters) {
+// Clusters at a time of both kernels for every group of load cases.
+int fit_shape(cstg_ctx* ctx, int n_rhs, Shape sh, int (&max_clusters)[2]) {
   (void)ctx;
-  int worst = INT_MAX;
+  max_clusters[0] = max_clusters[1] = INT_MAX;
   for (int q0 = 0; q0 < n_rhs; q0 += kMaxGroup) {
-    int m = 0;
-    const cudaError_t e = batch_max_clusters(std::min(kMaxGroup, n_rhs - q0), sh.cluster, sh.threads, &m);
+    int m[2] = {0, 0};
+    const cudaError_t e = batch_max_clusters(std::min(kMaxGroup, n_rhs - q0), sh.cluster, sh.threads, m);
     if (e != cudaSuccess) {
       cudaGetLastError();
-      m = 0;
+      m[0] = m[1] = 0;
     }
-    worst = std::min(worst, m);
+    for (int k = 0; k < 2; ++k) max_clusters[k] = std::min(max_clusters[k], m[k]);
   }
-  *max_clusters = worst == INT_MAX ? 0 : worst;
   return CSTG_OK;
 }
 
 // One batched solve with shape `sh` (graph-captured when `graph`), timed with CUDA events.
 int run(cstg_ctx* ctx, int n_sys, int n_rhs, const double* d_b, double* d_x, const cstg_solver_options& o,
         Shape sh, bool graph, double* seconds) {
-  int maxc = 0;
-  fit_shape(ctx, n_rhs, sh, &maxc);
-  if (maxc < 1)
+  int maxc[2] = {0, 0};
+  fit_shape(ctx, n_rhs, sh, maxc);
+  if (maxc[0] < 1 || maxc[1] < 1)
     return fail(ctx, CSTG_ERR_UNSUPPORTED, "batch_solve: launch shape %d CTAs x %d threads does not fit",
                 sh.cluster, sh.threads);
-  const int n_clusters = std::min(maxc, n_sys);
   long long launched = 0;
   if (graph) {
     unsigned long long key = 0x5eedull;
     for (unsigned long long v :
          {(unsigned long long)ctx->generation, (unsigned long long)n_sys, (unsigned long long)n_rhs,
           (unsigned long long)(uintptr_t)d_b, (unsigned long long)(uintptr_t)d_x, (unsigned long long)sh.cluster,
-          (unsigned long long)sh.threads, (unsigned long long)n_clusters, (unsigned long long)o.max_iter,
+          (unsigned long long)sh.threads, (unsigned long long)maxc[0], (unsigned long long)maxc[1],
+          (unsigned long long)o.max_iter,
           (unsigned long long)o.max_refinements, (unsigned long long)o.precision})
       key = mix(key, v);
     unsigned long long rt;
@@ -179,7 +186,7 @@ int run(cstg_ctx* ctx, int n_sys, int n_rhs, const double* d_b, double* d_x, con
       }
       cudaGraph_t g = nullptr;
       CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-      const int rc = enqueue(ctx, n_sys, n_rhs, d_b, d_x, o, sh, n_clusters, &launched);
+      const int rc = enqueue(ctx, n_sys, n_rhs, d_b, d_x, o, sh, maxc, &launched);
       const cudaError_t ee = cudaStreamEndCapture(ctx->stream, &g);
       count_launches(-launched);  // captured, not run: counted per graph launch below
       if (rc) {
@@ -199,7 +206,7 @@ int run(cstg_ctx* ctx, int n_sys, int n_rhs, const double* d_b, double* d_x, con
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
   } else {
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    const int rc = enqueue(ctx, n_sys, n_rhs, d_b, d_x, o, sh, n_clusters, &launched);
+    const int rc = enqueue(ctx, n_sys, n_rhs, d_b, d_x, o, sh, maxc, &launched);
     if (rc) return rc;
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
   }
@@ -290,9 +297,9 @@ int cstg_batch_autotune(cstg_ctx* ctx, int n_systems, const int32_t* node_offset
   Shape win{0, 0};
   double t_win = 0.0;
   for (const Shape& sh : kShapes) {
-    int maxc = 0;
-    fit_shape(ctx, n_rhs, sh, &maxc);
-    if (maxc < 1) continue;
+    int maxc[2] = {0, 0};
+    fit_shape(ctx, n_rhs, sh, maxc);
+    if (maxc[0] < 1 || maxc[1] < 1) continue;
     double t0 = 0.0, t1 = 0.0;
     rc = run(ctx, n_systems, n_rhs, d_b, d_x, o, sh, false, &t0);  // warm-up (first-launch costs)
     if (rc) return rc;

@@ -138,7 +138,13 @@ struct BatchArgs {
   int n_sys = 0;
   const int* sys_node = nullptr;  // [n_sys + 1] first node of each plate
   const int* order = nullptr;     // [n_sys] plates, largest first (the work queue's order)
-  int* queue = nullptr;           // work counter, zero at launch
+  int* queue = nullptr;           // [2] work counters (k_batch_halo, k_batch_pcg), zero at launch
+  int largest = 0;                // nodes of the largest plate
+  int* n_rest = nullptr;          // plates left to k_batch_pcg, zero at launch (null: all, in `order`)
+  int* rest = nullptr;            // [n_sys] those plates
+  unsigned char* wanted = nullptr;  // [N] nodes that other blocks need, zero at launch
+  unsigned short* slots = nullptr;  // neighbours in a block's own numbering, one per off-diagonal block
+  unsigned smem = 0;              // dynamic shared memory of a block
   MixedMatrix A32;                // FP32 difference-form operator (unused when start_fp64)
   BlockMatrix A64;                // FP64 operator (true residuals, FP64 mode)
   int start_fp64 = 0;
@@ -150,8 +156,9 @@ struct BatchArgs {
   BatchResultDev* res = nullptr;
   int res_stride = 0, res_offset = 0;  // result index = plate * res_stride + res_offset + q
 };
+// n[0], n[1]: clusters at a time of k_batch_pcg and k_batch_halo
 cudaError_t batch_max_clusters(int R, int cluster, int threads, int* n);
-cudaError_t launch_batch_pcg(const BatchArgs& a, int R, int cluster, int threads, int n_clusters,
+cudaError_t launch_batch_pcg(const BatchArgs& a, int R, int cluster, int threads, const int* n_clusters,
                              cudaStream_t s);
 cudaError_t launch_batch_pack(int N, int R, int q0, long long ld, const double* src, double* dst,
                               cudaStream_t s);

@@ -96,3 +96,37 @@ def test_csr_with_a_long_row(pkg, gpu_lib):
     cols = np.concatenate([np.arange(n), np.stack([np.zeros(n - 1, int), np.arange(1, n)], axis=1).reshape(-1)])
     vals = np.concatenate([[2.0], np.full(n - 1, 0.01), np.tile([0.01, 1.0], n - 1)])
     _both(pkg, *_csr(pkg, rp, cols, vals))
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("n_cases,config", [(1, (1, 256)), (1, (4, 512)), (2, (1, 512)), (2, (2, 256)), (3, (1, 512)),
+                                            (3, (16, 256)), (4, (1, 512)), (4, (2, 512)), (4, (8, 256))])
+def test_batch_shapes(pkg, gpu_lib, precision, n_cases, config):
+    """Batches whose largest plate's direction vectors fit a block and batches whose do not, against the
+    single solve of every plate and case."""
+    cases = dict(list(pkg.plate.LOAD_CASES.items())[:n_cases])
+    specs = [pkg.plate.PlateSpec(n_r=n, n_theta=2 * n, a=1.0, E=1.0, nu=0.3, plane_strain=False)
+             for n in (3, 24, 40, 61, 84)]
+    batch = pkg.build_batch(specs, cases=cases)
+    solver = pkg.BatchSolver(pkg.SolverOptions(precision=precision, max_iter=200000))
+    solver.setup(batch)
+    sol = solver.solve(config=config)
+    assert sol.converged.all() and (sol.true_rel_residual <= 1e-10).all()
+    solver.close()
+    for s, spec in enumerate(specs):
+        m = pkg.plate.quarter_plate(spec.n_r, spec.n_theta)
+        K = pkg.build_stiffness_pattern(m)
+        for q, parts in enumerate(cases.values()):
+            pkg.assemble_stiffness(m, pkg.constitutive_matrix(1.0, 0.3), 1.0, K)
+            b = np.zeros(m.num_dofs)
+            for group, tx, ty in parts:
+                pkg.add_traction(K, m.boundary_edges[group], 1.0, tx, ty, b)
+            pkg.apply_dirichlet(pkg.plate.symmetry_dirichlet(m), K, b)
+            one = pkg.CgJacobiSolver(pkg.SolverOptions(precision=precision, max_iter=200000, true_residual_stop=True))
+            one.setup(K)
+            x = np.zeros(b.size)
+            st = one.solve(b, x)
+            assert st.converged
+            assert abs(sol.iterations[s, q] - st.iterations) <= max(2, 0.02 * st.iterations)
+            assert np.linalg.norm(sol.x[q, batch.dof_range(s)] - x) <= REL_TOL * np.linalg.norm(x)
+        K.ctx.close()
