@@ -60,7 +60,7 @@ struct cstg_ctx {
   DevBuf xy, tri;
 
   // incidence + pattern
-  DevBuf cnt, cursor, ne_ptr, ne, scan_tmp, deg, node_ptr, bnbr, slot;
+  DevBuf cnt, cursor, ne_ptr, ne, scan_tmp, deg, node_ptr, bnbr, slot, self_pos, diag;
   DevBuf row_ptr, cols, vals;
   int kind = 0;  // 0 none, 1 mesh block pattern, 2 caller CSR
   int n_rows = 0;

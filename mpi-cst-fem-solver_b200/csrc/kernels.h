@@ -434,17 +434,21 @@ cudaError_t launch_incidence(const MeshDev& m, int* cnt, int* cursor, int* ne_pt
 cudaError_t launch_pattern_count(const MeshDev& m, const int* ne_ptr, const int* ne, int* deg,
                                  int* node_ptr, int* scan_tmp, int* err, cudaStream_t s);
 cudaError_t launch_pattern_fill(const MeshDev& m, const int* ne_ptr, const int* ne,
-                                const int* node_ptr, int* bnbr, int* slot, int* row_ptr,
-                                int* cols, cudaStream_t s);
-cudaError_t launch_assemble(const MeshDev& m, const int* ne_ptr, const int* ne, const int* slot,
+                                const int* node_ptr, int* bnbr, unsigned* slot, unsigned char* self,
+                                int* row_ptr, int* cols, cudaStream_t s);
+cudaError_t launch_assemble(const MeshDev& m, const int* ne_ptr, const int* ne, const unsigned* slot,
                             const int* node_ptr, const Mat3& D, double t, const int* mat,
-                            const double* Dtab, const double* ttab, double* vals, cudaStream_t s);
+                            const double* Dtab, const double* ttab, const unsigned char* self, double* vals,
+                            double* diag, cudaStream_t s);
+// node_ptr, bnbr: the mesh pattern's block rows (null: a caller's CSR)
 cudaError_t launch_dirichlet(int n_rows, const int* row_ptr, const int* cols, double* vals,
                              int n_fixed, const int* dofs, const double* values,
                              unsigned char* fixed, double* ubar, double* b, int n_rhs,
-                             int* err, cudaStream_t s, bool apply);
+                             int* err, cudaStream_t s, bool apply, const int* node_ptr = nullptr,
+                             const int* bnbr = nullptr);
 cudaError_t launch_inv_diag(int n_rows, const int* row_ptr, const int* cols, const double* vals,
                             double* inv_diag, int* err, cudaStream_t s);
+cudaError_t launch_inv_diag_nodes(int n_nodes, const double* diag, double* inv_diag, int* err, cudaStream_t s);
 cudaError_t launch_element_stresses(const MeshDev& m, const double* u, const Mat3& D, double nu,
                                     int plane_strain, double* out, cudaStream_t s);
 
