@@ -213,8 +213,9 @@ struct MpnnWork {  // activations (training keeps every layer; inference ping-po
   __nv_bfloat16* X = nullptr;  // [N][8]
   float* Y = nullptr;          // [N][2]
   float* dY = nullptr;         // [2N]
-  float *dH = nullptr, *dH2 = nullptr, *dU = nullptr, *dAs = nullptr;  // [N][64]
-  float* part = nullptr;       // [kMpPartBlocks][kMpPartStride]
+  float *dH = nullptr, *dH2 = nullptr, *dAs = nullptr, *dAs2 = nullptr;  // [N][64]
+  float* dU = nullptr;         // [kMpL + 1][N][64]: the layers', the encoder's
+  float* part = nullptr;       // [kMpL + 1][kMpPartBlocks][kMpPartStride]: the layers'; decoder and encoder
 };
 
 struct MpScratch {  // small device scalars of the network's reductions

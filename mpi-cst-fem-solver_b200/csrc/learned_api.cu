@@ -387,7 +387,7 @@ struct cstg_trainer {
   cudaStream_t stream = nullptr;
   std::string err;
   DevBuf p32, m, v, grad, pb, pf, sc, az, z;
-  DevBuf H[kMpL + 1], G[kMpL], A[kMpL], X, Y, dY, dH, dH2, dU, dAs, part;
+  DevBuf H[kMpL + 1], G[kMpL], A[kMpL], X, Y, dY, dH, dH2, dU, dAs, dAs2, part;
   int step = 0;
   int cap_nodes = 0;
 };
@@ -442,9 +442,10 @@ int trainer_work(cstg_trainer* tr, int N, MpnnWork& w) {
   TENSURE(tr->dY, sizeof(float) * 2 * (size_t)N);
   TENSURE(tr->dH, sizeof(float) * nf);
   TENSURE(tr->dH2, sizeof(float) * nf);
-  TENSURE(tr->dU, sizeof(float) * nf);
+  TENSURE(tr->dU, sizeof(float) * nf * (kMpL + 1));
   TENSURE(tr->dAs, sizeof(float) * nf);
-  TENSURE(tr->part, sizeof(float) * (size_t)kMpPartBlocks * kMpPartStride);
+  TENSURE(tr->dAs2, sizeof(float) * nf);
+  TENSURE(tr->part, sizeof(float) * (size_t)kMpPartBlocks * kMpPartStride * (kMpL + 1));
   TENSURE(tr->az, sizeof(double) * 2 * (size_t)N);
   TENSURE(tr->z, sizeof(double) * 2 * (size_t)N);
   for (int l = 0; l <= kMpL; ++l) w.H[l] = static_cast<__nv_bfloat16*>(tr->H[l].p);
@@ -459,6 +460,7 @@ int trainer_work(cstg_trainer* tr, int N, MpnnWork& w) {
   w.dH2 = static_cast<float*>(tr->dH2.p);
   w.dU = static_cast<float*>(tr->dU.p);
   w.dAs = static_cast<float*>(tr->dAs.p);
+  w.dAs2 = static_cast<float*>(tr->dAs2.p);
   w.part = static_cast<float*>(tr->part.p);
   return CSTG_OK;
 }
@@ -579,7 +581,7 @@ void cstg_trainer_destroy(cstg_trainer* tr) {
   cudaSetDevice(tr->device);
   if (tr->stream) cudaStreamSynchronize(tr->stream);
   DevBuf* all[] = {&tr->p32, &tr->m, &tr->v, &tr->grad, &tr->pb, &tr->pf, &tr->sc, &tr->az, &tr->z,
-                   &tr->X,   &tr->Y, &tr->dY, &tr->dH,  &tr->dH2, &tr->dU, &tr->dAs, &tr->part};
+                   &tr->X,   &tr->Y, &tr->dY, &tr->dH,  &tr->dH2, &tr->dU, &tr->dAs, &tr->dAs2, &tr->part};
   for (DevBuf* b : all) free_buf(*b);
   for (auto& b : tr->H) free_buf(b);
   for (auto& b : tr->G) free_buf(b);

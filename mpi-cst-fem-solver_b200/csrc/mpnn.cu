@@ -1465,7 +1465,9 @@ __global__ void __launch_bounds__(256) k_mp_dy(int n, const double* __restrict__
 // ---- training: backward ------------------------------------------------------------------------
 
 // dH3 = W_out' dY; partial gradients of W_out (2 x 64) and b_out (2) per block
-__global__ void __launch_bounds__(256) k_mp_dec_bwd(int N, const __nv_bfloat16* __restrict__ H3, MpnnParams P,
+constexpr int kDecLanes = 16;  // node lanes of a block
+
+__global__ void __launch_bounds__(64 * kDecLanes) k_mp_dec_bwd(int N, const __nv_bfloat16* __restrict__ H3, MpnnParams P,
                                                     const float* __restrict__ dY, float* __restrict__ dH,
                                                     float* __restrict__ part /* [grid][130] */) {
   __shared__ float w[2 * F];
@@ -1473,22 +1475,36 @@ __global__ void __launch_bounds__(256) k_mp_dec_bwd(int N, const __nv_bfloat16* 
   for (int i = threadIdx.x; i < 2 * F; i += blockDim.x) w[i] = bf(P.pb[kMpOffWout + i]);
   for (int i = threadIdx.x; i < 2 * F + 2; i += blockDim.x) red[i] = 0.f;
   __syncthreads();
-  // thread layout: 64 features x 4 node lanes
+  // thread layout: 64 features x kDecLanes node lanes
   const int k = threadIdx.x & 63, lane4 = threadIdx.x >> 6;
   float gw0 = 0.f, gw1 = 0.f, gb0 = 0.f, gb1 = 0.f;
-  for (int n = blockIdx.x * 4 + lane4; n < N; n += gridDim.x * 4) {
-    const float d0 = dY[2 * n], d1 = dY[2 * n + 1];
-    const float h = bf(H3[(size_t)n * F + k]);
-    dH[(size_t)n * F + k] = d0 * w[k] + d1 * w[F + k];
-    gw0 = fmaf(d0, h, gw0);
-    gw1 = fmaf(d1, h, gw1);
-    if (k == 0) {
-      gb0 += d0;
-      gb1 += d1;
+  constexpr int kU = 8;  // nodes whose loads are in flight together
+  const int step = gridDim.x * kDecLanes;
+  for (int n0 = blockIdx.x * kDecLanes + lane4; n0 < N; n0 += kU * step) {
+    float2 d[kU];
+    float h[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int n = min(n0 + u * step, N - 1);
+      d[u] = reinterpret_cast<const float2*>(dY)[n];
+      h[u] = bf(H3[(size_t)n * F + k]);
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int n = n0 + u * step;
+      if (n >= N) break;
+      const float d0 = d[u].x, d1 = d[u].y;
+      dH[(size_t)n * F + k] = d0 * w[k] + d1 * w[F + k];
+      gw0 = fmaf(d0, h[u], gw0);
+      gw1 = fmaf(d1, h[u], gw1);
+      if (k == 0) {
+        gb0 += d0;
+        gb1 += d1;
+      }
     }
   }
-  // fixed-order block reduction: the four node lanes in order
-  for (int l = 0; l < 4; ++l) {
+  // fixed-order block reduction: the node lanes in order
+  for (int l = 0; l < kDecLanes; ++l) {
     if (lane4 == l) {
       red[k] += gw0;
       red[F + k] += gw1;
@@ -1502,60 +1518,142 @@ __global__ void __launch_bounds__(256) k_mp_dec_bwd(int N, const __nv_bfloat16* 
   for (int i = threadIdx.x; i < 2 * F + 2; i += blockDim.x) part[(size_t)blockIdx.x * (2 * F + 2) + i] = red[i];
 }
 
-// Layer backward, part 1: dU = dH (G > 0); dHprev = dH + W_h' dU; dAs = (W_a' dU) / deg.
-// 64 threads per node (feature k), four nodes per 256-thread block step.
-__global__ void __launch_bounds__(256) k_mp_layer_bwd_a(int N, const int* __restrict__ node_ptr,
-                                                        const int* __restrict__ nbr, MpnnParams P, int layer,
-                                                        const float* __restrict__ dH,
-                                                        const __nv_bfloat16* __restrict__ G,
-                                                        float* __restrict__ dU, float* __restrict__ dHprev,
-                                                        float* __restrict__ dAs) {
-  extern __shared__ float wsm[];  // W_l as float [64][128]
-  __shared__ float du[4][F];
-  const __nv_bfloat16* W = P.pb + kMpOffL0 + layer * kMpLStride;
-  for (int i = threadIdx.x; i < F * 2 * F; i += blockDim.x) wsm[i] = bf(W[i]);
-  const int k = threadIdx.x & 63, g = threadIdx.x >> 6;
-  for (int base = blockIdx.x * 4; base < N; base += gridDim.x * 4) {
-    const int n = base + g;
-    __syncthreads();
-    float dh = 0.f;
-    if (n < N) {
-      dh = dH[(size_t)n * F + k];
-      const float u = bf(G[(size_t)n * F + k]) > 0.f ? dh : 0.f;
-      du[g][k] = u;
-      dU[(size_t)n * F + k] = u;
-    } else {
-      du[g][k] = 0.f;
+// dH of four features c .. c+3 of K nodes below a layer: dHprev + the mean's transpose, the sum over a
+// node's neighbours m (in pattern order) of dAs_m. Rows of up to eight blocks are read at one go, and
+// the K nodes' reads are in flight together.
+template <int K>
+__device__ __forceinline__ void gathered(const float* __restrict__ dHprev, const float* __restrict__ dAs,
+                                         const int* __restrict__ node_ptr, const int* __restrict__ nbr,
+                                         const int (&n)[K], int c, float4 (&d)[K]) {
+  int b[K], e[K];
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    d[i] = *reinterpret_cast<const float4*>(dHprev + (size_t)n[i] * F + c);
+    if (dAs) {
+      b[i] = node_ptr[n[i]];
+      e[i] = node_ptr[n[i] + 1];
     }
-    __syncthreads();
-    if (n < N) {
-      float sh = 0.f, sa = 0.f;
-#pragma unroll 8
-      for (int o = 0; o < F; ++o) {
-        const float u = du[g][o];
-        sh = fmaf(u, wsm[o * 2 * F + k], sh);
-        sa = fmaf(u, wsm[o * 2 * F + F + k], sa);
+  }
+  if (!dAs) return;
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = b[i]; q < e[i]; q += 8) {
+      float4 v[8];
+      bool on[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int m = nbr[min(q + u, e[i] - 1)];
+        on[u] = q + u < e[i] && m != n[i];
+        v[u] = *reinterpret_cast<const float4*>(dAs + (size_t)m * F + c);
       }
-      int deg = 0;
-      for (int q = node_ptr[n]; q < node_ptr[n + 1]; ++q) deg += nbr[q] != n;
-      dHprev[(size_t)n * F + k] = dh + sh;
-      dAs[(size_t)n * F + k] = deg ? sa / (float)deg : 0.f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (on[u]) {
+          s.x += v[u].x;
+          s.y += v[u].y;
+          s.z += v[u].z;
+          s.w += v[u].w;
+        }
     }
+    d[i].x += s.x;
+    d[i].y += s.y;
+    d[i].z += s.z;
+    d[i].w += s.w;
   }
 }
 
-// Layer backward, part 2: dHprev_m += sum over neighbours n of m of dAs_n (the mean's transpose)
-__global__ void __launch_bounds__(256) k_mp_layer_bwd_b(int N, const int* __restrict__ node_ptr,
-                                                        const int* __restrict__ nbr, const float* __restrict__ dAs,
-                                                        float* __restrict__ dHprev) {
-  const int k = threadIdx.x & 63;
-  for (int m = blockIdx.x * 4 + (threadIdx.x >> 6); m < N; m += gridDim.x * 4) {
-    float s = 0.f;
-    for (int q = node_ptr[m]; q < node_ptr[m + 1]; ++q) {
-      const int n = nbr[q];
-      if (n != m) s += dAs[(size_t)n * F + k];
+__device__ __forceinline__ float4 masked(float4 d, const __nv_bfloat16* g) {  // d where g > 0
+  const uint2 w = *reinterpret_cast<const uint2*>(g);
+  const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w.x));
+  const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w.y));
+  return make_float4(lo.x > 0.f ? d.x : 0.f, lo.y > 0.f ? d.y : 0.f, hi.x > 0.f ? d.z : 0.f, hi.y > 0.f ? d.w : 0.f);
+}
+
+// Layer backward: dH = dHin + the mean's transpose of the layer above (dAsIn, null at the top);
+// dU = dH (G > 0); dHout = dH + W_h' dU; dAsOut = (W_a' dU) / deg.
+// FP32 on the CUDA cores, bound by their multiply-adds: a tile of 64 nodes and all 128 columns per block
+// step, 8 nodes x 4 columns per thread, so that three 16-byte shared-memory reads feed 32 multiply-adds
+// (a thread per node and feature, with a read per multiply-add, took 56 us for 33,153 nodes; this takes
+// 31 with the gather of the layer above, which was a 16 us kernel of its own). Sums over o run in
+// the same order as there.
+constexpr int kBwTile = 64;
+constexpr int kBwSmem = (F * 2 * F + 2 * kBwTile * (F + 4)) * (int)sizeof(float);
+
+__global__ void __launch_bounds__(256) k_mp_layer_bwd(int N, const int* __restrict__ node_ptr,
+                                                      const int* __restrict__ nbr, MpnnParams P, int layer,
+                                                      const float* __restrict__ dHin, const float* __restrict__ dAsIn,
+                                                      const __nv_bfloat16* __restrict__ G, float* __restrict__ dU,
+                                                      float* __restrict__ dHout, float* __restrict__ dAsOut) {
+  extern __shared__ __align__(16) float bwsm[];
+  float* wsm = bwsm;                            // W_l as float [64 o][128]
+  float* dut = wsm + F * 2 * F;                 // dU transposed [64 o][64 nodes + 4]
+  float* dhs = dut + F * (kBwTile + 4);         // dH [64 nodes][64 + 4]
+  const __nv_bfloat16* W = P.pb + kMpOffL0 + layer * kMpLStride;
+  for (int i = threadIdx.x; i < F * 2 * F / 2; i += 256)  // (an offset of two weights is 4-byte aligned)
+    *reinterpret_cast<float2*>(wsm + 2 * i) = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(W)[i]);
+  const int col = (threadIdx.x & 31) * 4, row = (threadIdx.x >> 5) * 8;
+  for (int base = blockIdx.x * kBwTile; base < N; base += gridDim.x * kBwTile) {
+    __syncthreads();
+    constexpr int K = 2;
+    for (int i0 = threadIdx.x; i0 < kBwTile * F / 4; i0 += K * 256) {
+      int nd[K];
+      float4 dv[K];
+      const int c = i0 % (F / 4) * 4;  // (256 is a multiple of F / 4: the same features for every i)
+#pragma unroll
+      for (int h = 0; h < K; ++h) nd[h] = min(base + (i0 + h * 256) / (F / 4), N - 1);
+      gathered<K>(dHin, dAsIn, node_ptr, nbr, nd, c, dv);
+#pragma unroll
+      for (int h = 0; h < K; ++h) {
+        const int j = (i0 + h * 256) / (F / 4), n = base + j;
+        float4 d = dv[h], u = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (n < N) {
+          u = masked(d, G + (size_t)n * F + c);
+          *reinterpret_cast<float4*>(dU + (size_t)n * F + c) = u;
+        }
+        *reinterpret_cast<float4*>(dhs + j * (F + 4) + c) = d;
+        dut[(c + 0) * (kBwTile + 4) + j] = u.x;
+        dut[(c + 1) * (kBwTile + 4) + j] = u.y;
+        dut[(c + 2) * (kBwTile + 4) + j] = u.z;
+        dut[(c + 3) * (kBwTile + 4) + j] = u.w;
+      }
     }
-    dHprev[(size_t)m * F + k] += s;
+    __syncthreads();
+    float acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[i][c] = 0.f;
+#pragma unroll 4
+    for (int o = 0; o < F; ++o) {
+      const float4 w = *reinterpret_cast<const float4*>(wsm + o * 2 * F + col);
+      const float4 u0 = *reinterpret_cast<const float4*>(dut + o * (kBwTile + 4) + row);
+      const float4 u1 = *reinterpret_cast<const float4*>(dut + o * (kBwTile + 4) + row + 4);
+      const float u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        acc[i][0] = fmaf(u[i], w.x, acc[i][0]);
+        acc[i][1] = fmaf(u[i], w.y, acc[i][1]);
+        acc[i][2] = fmaf(u[i], w.z, acc[i][2]);
+        acc[i][3] = fmaf(u[i], w.w, acc[i][3]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int n = base + row + i;
+      if (n >= N) break;
+      if (col < F) {
+        const float4 d = *reinterpret_cast<const float4*>(dhs + (row + i) * (F + 4) + col);
+        *reinterpret_cast<float4*>(dHout + (size_t)n * F + col) =
+            make_float4(d.x + acc[i][0], d.y + acc[i][1], d.z + acc[i][2], d.w + acc[i][3]);
+      } else {
+        const int deg = node_ptr[n + 1] - node_ptr[n] - 1;  // (the node itself is in its row)
+        const float f = (float)deg;
+        *reinterpret_cast<float4*>(dAsOut + (size_t)n * F + col - F) =
+            deg > 0 ? make_float4(acc[i][0] / f, acc[i][1] / f, acc[i][2] / f, acc[i][3] / f)
+                    : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
   }
 }
 
@@ -1567,8 +1665,8 @@ __global__ void __launch_bounds__(256) k_mp_wgrad(int N, const float* __restrict
                                                   const __nv_bfloat16* __restrict__ X1,
                                                   const __nv_bfloat16* __restrict__ X2, float* __restrict__ part) {
   constexpr int KQ = KW / 4;
-  constexpr int CH = 32;  // nodes per staged chunk
-  __shared__ float sdu[CH][F];
+  constexpr int CH = KW == 2 * F ? 32 : 64;  // nodes per staged chunk
+  __shared__ __align__(16) float sdu[CH][F];
   __shared__ float sx[CH][KW];
   const int o = threadIdx.x >> 2, q = threadIdx.x & 3;
   float acc[KQ];
@@ -1579,9 +1677,10 @@ __global__ void __launch_bounds__(256) k_mp_wgrad(int N, const float* __restrict
   const int n0 = blockIdx.x * per, n1 = min(N, n0 + per);
   for (int c0 = n0; c0 < n1; c0 += CH) {
     __syncthreads();
-    for (int i = threadIdx.x; i < CH * F; i += 256) {
-      const int j = i / F, f = i % F, n = c0 + j;
-      sdu[j][f] = n < n1 ? dU[(size_t)n * F + f] : 0.f;
+    for (int i = threadIdx.x; i < CH * F / 4; i += 256) {
+      const int j = i / (F / 4), f = i % (F / 4) * 4, n = c0 + j;
+      *reinterpret_cast<float4*>(&sdu[j][f]) = n < n1 ? *reinterpret_cast<const float4*>(dU + (size_t)n * F + f)
+                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     for (int i = threadIdx.x; i < CH * KW; i += 256) {
       const int j = i / KW, f = i % KW, n = c0 + j;
@@ -1610,20 +1709,28 @@ __global__ void __launch_bounds__(256) k_mp_wgrad(int N, const float* __restrict
 
 // Weight gradient of a message-passing layer on the tensor cores:
 //   dW^T[k][o] = sum_n Xc[n][k] dU[n][o]  (k < 128: Xc = [Hprev | A], o < 64),  db[o] = sum_n dU[n][o].
-// One CTA of 256 threads per contiguous node range (the same ranges as k_mp_wgrad, so the
-// partial sums per block keep their block order). Per chunk of 128 nodes: the Xc rows (BF16) and
+// One CTA of 256 threads per contiguous node range and layer (blockIdx.y): the layers wait for nothing of one another and fill
+// the gaps of each other's copies, transposes and MMA waits (18 us each in turn, 34 together). Per chunk of 128 nodes: the Xc rows (BF16) and
 // the dU rows (FP32, rounded to BF16; db summed in FP32 on the CUDA cores in node order) are
 // staged row-major, transposed into the K-major core-matrix layouts of the MMA operands
 // (A = Xc^T: 128 features x 128 nodes, B = dU^T: 64 outputs x 128 nodes; 8 nodes per 16-byte unit),
 // and one thread issues 8 tcgen05.mma (M=128, N=64, K=16) accumulating into 64 TMEM columns over
 // all chunks. Each warp of the first four then reads its 32 feature rows x 64 outputs.
 constexpr int kWgNodes = 128;
+constexpr int kWgBlocks = 98;  // per layer: three layers' blocks are one wave of two per SM
 constexpr int kWgSmem = kWgNodes * 2 * F * 2 /*Xc rows*/ + kWgNodes * F * 2 /*dU rows*/ + kASmem + kBSmem + 1024;
 
-__global__ void __launch_bounds__(256, 1) k_mp_wgrad_tc(int N, const float* __restrict__ dU,
-                                                        const __nv_bfloat16* __restrict__ X1,
-                                                        const __nv_bfloat16* __restrict__ X2, long long spin_limit,
-                                                        float* __restrict__ part, int* err) {
+struct WgradLayers {
+  const float* dU[kMpL];
+  const __nv_bfloat16 *H[kMpL], *A[kMpL];
+};
+
+__global__ void __launch_bounds__(256, 2) k_mp_wgrad_tc(int N, const WgradLayers L, long long spin_limit,
+                                                        float* __restrict__ parts, int* err) {
+  const float* __restrict__ dU = L.dU[blockIdx.y];
+  const __nv_bfloat16* __restrict__ X1 = L.H[blockIdx.y];
+  const __nv_bfloat16* __restrict__ X2 = L.A[blockIdx.y];
+  float* __restrict__ part = parts + (size_t)blockIdx.y * gridDim.x * kMpPartStride;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t mbar;
   __shared__ uint32_t tmem_slot;
@@ -1764,22 +1871,50 @@ __global__ void __launch_bounds__(256, 1) k_mp_wgrad_tc(int N, const float* __re
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(F));
 }
 
-// Encoder backward: dU0 = dH0 (H0 > 0)
-__global__ void __launch_bounds__(256) k_mp_enc_bwd(int N, const float* __restrict__ dH,
+// Encoder backward: dU0 = dH0 (H0 > 0), dH0 gathered as in the layers; 16 threads per node
+__global__ void __launch_bounds__(256) k_mp_enc_bwd(int N, const int* __restrict__ node_ptr,
+                                                    const int* __restrict__ nbr, const float* __restrict__ dHin,
+                                                    const float* __restrict__ dAsIn,
                                                     const __nv_bfloat16* __restrict__ H0, float* __restrict__ dU) {
-  const size_t total = (size_t)N * F;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x)
-    dU[i] = bf(H0[i]) > 0.f ? dH[i] : 0.f;
+  const long long total = (long long)N * (F / 4);
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const int n = (int)(i / (F / 4)), c = (int)(i % (F / 4)) * 4;
+    const int nd[1] = {n};
+    float4 d[1];
+    gathered<1>(dHin, dAsIn, node_ptr, nbr, nd, c, d);
+    *reinterpret_cast<float4*>(dU + (size_t)n * F + c) = masked(d[0], H0 + (size_t)n * F + c);
+  }
 }
 
-// grad[dst + i] += sum over blocks b (in order) of part[b][src + i], for i < count
-__global__ void k_mp_reduce_parts(const float* __restrict__ part, int nblocks, int stride, int src, int count,
-                                  float* __restrict__ grad, int dst) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int b = 0; b < nblocks; ++b) s += part[(size_t)b * stride + src + i];
-    grad[dst + i] += s;
+// grad[dst + i] += sum over blocks b of part[b][i], for i < count: one segment per blockIdx.y (decoder,
+// the layers, encoder). Four threads share an element: each adds a quarter of the blocks in order, and
+// the quarters are added in a fixed tree.
+struct PartSegments {
+  const float* part[kMpL + 2];
+  int blocks[kMpL + 2], stride[kMpL + 2], count[kMpL + 2], dst[kMpL + 2];
+};
+
+__global__ void __launch_bounds__(256) k_mp_reduce_parts(const PartSegments g, float* __restrict__ grad) {
+  const float* __restrict__ part = g.part[blockIdx.y];
+  const int stride = g.stride[blockIdx.y], count = g.count[blockIdx.y], nb = g.blocks[blockIdx.y];
+  // lanes 0-7: eight consecutive elements of quarter 0, lanes 8-15 of quarter 1, ...
+  const int lane = threadIdx.x & 31, quarter = lane >> 3;
+  const int i = (blockIdx.x * 256 + (int)threadIdx.x - lane) / 4 + (lane & 7);
+  const int b0 = nb * quarter / 4, b1 = nb * (quarter + 1) / 4;
+  float s = 0.f;
+  if (i < count) {
+    constexpr int kU = 16;  // blocks whose loads are in flight together
+    for (int b = b0; b < b1; b += kU) {
+      float v[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) v[u] = b + u < b1 ? part[(size_t)(b + u) * stride + i] : 0.f;
+#pragma unroll
+      for (int u = 0; u < kU; ++u) s += v[u];
+    }
   }
+  s += __shfl_xor_sync(0xffffffffu, s, 8);
+  s += __shfl_xor_sync(0xffffffffu, s, 16);
+  if (quarter == 0 && i < count) grad[g.dst[blockIdx.y] + i] += s;
 }
 
 // Adam (decoupled weight decay off): master FP32 parameters, BF16 copies for the kernels.
@@ -1913,7 +2048,9 @@ cudaError_t mpnn_prepare_device() {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !wg_done[dev]) {
-    const cudaError_t ew = cudaFuncSetAttribute(k_mp_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem);
+    cudaError_t ew = cudaFuncSetAttribute(k_mp_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem);
+    if (ew == cudaSuccess)
+      ew = cudaFuncSetAttribute(k_mp_layer_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwSmem);
     if (ew != cudaSuccess) return ew;
     wg_done[dev] = true;
   }
@@ -2065,32 +2202,47 @@ cudaError_t launch_mp_backward(const MpnnGraph& g, const MpnnParams& P, MpnnWork
   const int N = g.n_nodes;
   if (N <= 0) return cudaSuccess;
   const int G = kMpPartBlocks;
+  // partial sums of the layers, the decoder and the encoder, added at the end in one launch
+  PartSegments seg;
+  const size_t layer_part = (size_t)kWgBlocks * kMpPartStride;
+  float* dec_part = w.part + kMpL * layer_part;
+  float* enc_part = dec_part + (size_t)G * (2 * F + 2);
   // decoder
-  k_mp_dec_bwd<<<G, 256, 0, s>>>(N, w.H[kMpL], P, w.dY, w.dH, w.part);
-  k_mp_reduce_parts<<<1, 256, 0, s>>>(w.part, G, 2 * F + 2, 0, 2 * F, grad, kMpOffWout);
-  k_mp_reduce_parts<<<1, 32, 0, s>>>(w.part, G, 2 * F + 2, 2 * F, 2, grad, kMpOffBout);
-  long long k = 3;
-  // layers 3..1
-  float* dh = w.dH;
-  float* dprev = w.dH2;
+  k_mp_dec_bwd<<<G, 64 * kDecLanes, 0, s>>>(N, w.H[kMpL], P, w.dY, w.dH, dec_part);
+  seg.part[0] = dec_part;
+  seg.blocks[0] = G;
+  seg.stride[0] = seg.count[0] = 2 * F + 2;  // (b_out follows W_out in the parameters too)
+  seg.dst[0] = kMpOffWout;
+  // layers 3..1: each gathers the mean's transpose of the one above as it reads it
+  const float *din = w.dH, *as = nullptr;
+  WgradLayers wl;
+  const int grid = std::min((N + kBwTile - 1) / kBwTile, 148 * 3);
   for (int l = kMpL - 1; l >= 0; --l) {
-    k_mp_layer_bwd_a<<<grid_nodes(N, 4), 256, F * 2 * F * sizeof(float), s>>>(N, g.node_ptr, g.nbr, P, l, dh,
-                                                                               w.G[l], w.dU, dprev, w.dAs);
-    k_mp_wgrad_tc<<<G, 256, kWgSmem, s>>>(N, w.dU, w.H[l], w.A[l], spin_limit, w.part, err);
-    k_mp_layer_bwd_b<<<grid_nodes(N, 4), 256, 0, s>>>(N, g.node_ptr, g.nbr, w.dAs, dprev);
-    const int off = kMpOffL0 + l * kMpLStride;
-    k_mp_reduce_parts<<<grid_nodes(F * 2 * F + F, 256), 256, 0, s>>>(w.part, G, F * 2 * F + F, 0, F * 2 * F + F,
-                                                                      grad, off);
-    std::swap(dh, dprev);
-    k += 4;
+    float* dout = din == w.dH ? w.dH2 : w.dH;
+    float* aout = as == w.dAs ? w.dAs2 : w.dAs;
+    float* du = w.dU + (size_t)l * N * F;
+    k_mp_layer_bwd<<<grid, 256, kBwSmem, s>>>(N, g.node_ptr, g.nbr, P, l, din, as, w.G[l], du, dout, aout);
+    wl.dU[l] = du;
+    wl.H[l] = w.H[l];
+    wl.A[l] = w.A[l];
+    seg.part[1 + l] = w.part + l * layer_part;
+    seg.blocks[1 + l] = kWgBlocks;
+    seg.stride[1 + l] = seg.count[1 + l] = kMpPartStride;
+    seg.dst[1 + l] = kMpOffL0 + l * kMpLStride;
+    din = dout;
+    as = aout;
   }
+  k_mp_wgrad_tc<<<dim3(kWgBlocks, kMpL), 256, kWgSmem, s>>>(N, wl, spin_limit, w.part, err);
   // encoder
-  k_mp_enc_bwd<<<grid_nodes((long long)N * F, 256), 256, 0, s>>>(N, dh, w.H[0], w.dU);
-  k_mp_wgrad<kMpIn><<<G, 256, 0, s>>>(N, w.dU, w.X, nullptr, w.part);
-  k_mp_reduce_parts<<<grid_nodes(F * kMpIn + F, 256), 256, 0, s>>>(w.part, G, F * kMpIn + F, 0, F * kMpIn + F,
-                                                                    grad, kMpOffWin);
-  k += 3;
-  count_launches(k);
+  float* du0 = w.dU + (size_t)kMpL * N * F;
+  k_mp_enc_bwd<<<grid_nodes((long long)N * (F / 4), 256), 256, 0, s>>>(N, g.node_ptr, g.nbr, din, as, w.H[0], du0);
+  k_mp_wgrad<kMpIn><<<G, 256, 0, s>>>(N, du0, w.X, nullptr, enc_part);
+  seg.part[1 + kMpL] = enc_part;
+  seg.blocks[1 + kMpL] = G;
+  seg.stride[1 + kMpL] = seg.count[1 + kMpL] = F * kMpIn + F;
+  seg.dst[1 + kMpL] = kMpOffWin;
+  k_mp_reduce_parts<<<dim3((kMpPartStride + 63) / 64, kMpL + 2), 256, 0, s>>>(seg, grad);
+  count_launches(5 + kMpL);
   return cudaGetLastError();
 }
 
