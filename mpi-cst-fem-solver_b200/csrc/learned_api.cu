@@ -385,9 +385,13 @@ int cstg_host::run_fcg(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg
 struct cstg_trainer {
   int device = 0;
   cudaStream_t stream = nullptr;
+  // Samples in flight: the backward pass of one runs on `back` beside the forward pass of the next, so
+  // what the forward pass leaves for it exists twice.
+  cudaStream_t back = nullptr;
+  cudaEvent_t fwd_done[2] = {}, bwd_done[2] = {};
   std::string err;
-  DevBuf p32, m, v, grad, pb, pf, sc, az, z;
-  DevBuf H[kMpL + 1], G[kMpL], A[kMpL], X, Y, dY, dH, dH2, dU, dAs, dAs2, part;
+  DevBuf p32, m, v, grad, pb, pf, sc[2], az, z, losses;
+  DevBuf H[2][kMpL + 1], G[2][kMpL], A[2][kMpL], X[2], Y, dY[2], dH, dH2, dU, dAs, dAs2, part;
   int step = 0;
   int cap_nodes = 0;
 };
@@ -430,16 +434,13 @@ int tensure(cstg_trainer* tr, DevBuf& b, size_t bytes) {
     if (rc_) return rc_;                           \
   } while (0)
 
-int trainer_work(cstg_trainer* tr, int N, MpnnWork& w) {
+// Two samples are in flight on systems of up to this many nodes (above it one sample's kernels fill the
+// GPU, and a second set of activations, 2 KB a node, would buy nothing).
+constexpr int kPipelineNodes = 200000;
+
+int trainer_work(cstg_trainer* tr, int N, int sets, MpnnWork (&w)[2]) {
   const size_t nf = (size_t)N * kMpF;
-  for (int l = 0; l <= kMpL; ++l) TENSURE(tr->H[l], sizeof(__nv_bfloat16) * nf);
-  for (int l = 0; l < kMpL; ++l) {
-    TENSURE(tr->G[l], sizeof(__nv_bfloat16) * nf);
-    TENSURE(tr->A[l], sizeof(__nv_bfloat16) * nf);
-  }
-  TENSURE(tr->X, sizeof(__nv_bfloat16) * (size_t)N * kMpIn);
   TENSURE(tr->Y, sizeof(float) * 2 * (size_t)N);
-  TENSURE(tr->dY, sizeof(float) * 2 * (size_t)N);
   TENSURE(tr->dH, sizeof(float) * nf);
   TENSURE(tr->dH2, sizeof(float) * nf);
   TENSURE(tr->dU, sizeof(float) * nf * (kMpL + 1));
@@ -448,20 +449,88 @@ int trainer_work(cstg_trainer* tr, int N, MpnnWork& w) {
   TENSURE(tr->part, sizeof(float) * (size_t)kMpPartBlocks * kMpPartStride * (kMpL + 1));
   TENSURE(tr->az, sizeof(double) * 2 * (size_t)N);
   TENSURE(tr->z, sizeof(double) * 2 * (size_t)N);
-  for (int l = 0; l <= kMpL; ++l) w.H[l] = static_cast<__nv_bfloat16*>(tr->H[l].p);
-  for (int l = 0; l < kMpL; ++l) {
-    w.G[l] = static_cast<__nv_bfloat16*>(tr->G[l].p);
-    w.A[l] = static_cast<__nv_bfloat16*>(tr->A[l].p);
+  for (int k = 0; k < sets; ++k) {
+    for (int l = 0; l <= kMpL; ++l) TENSURE(tr->H[k][l], sizeof(__nv_bfloat16) * nf);
+    for (int l = 0; l < kMpL; ++l) {
+      TENSURE(tr->G[k][l], sizeof(__nv_bfloat16) * nf);
+      TENSURE(tr->A[k][l], sizeof(__nv_bfloat16) * nf);
+    }
+    TENSURE(tr->X[k], sizeof(__nv_bfloat16) * (size_t)N * kMpIn);
+    TENSURE(tr->dY[k], sizeof(float) * 2 * (size_t)N);
   }
-  w.X = static_cast<__nv_bfloat16*>(tr->X.p);
-  w.Y = static_cast<float*>(tr->Y.p);
-  w.dY = static_cast<float*>(tr->dY.p);
-  w.dH = static_cast<float*>(tr->dH.p);
-  w.dH2 = static_cast<float*>(tr->dH2.p);
-  w.dU = static_cast<float*>(tr->dU.p);
-  w.dAs = static_cast<float*>(tr->dAs.p);
-  w.dAs2 = static_cast<float*>(tr->dAs2.p);
-  w.part = static_cast<float*>(tr->part.p);
+  for (int k = 0; k < 2; ++k) {
+    const int j = k < sets ? k : 0;
+    for (int l = 0; l <= kMpL; ++l) w[k].H[l] = static_cast<__nv_bfloat16*>(tr->H[j][l].p);
+    for (int l = 0; l < kMpL; ++l) {
+      w[k].G[l] = static_cast<__nv_bfloat16*>(tr->G[j][l].p);
+      w[k].A[l] = static_cast<__nv_bfloat16*>(tr->A[j][l].p);
+    }
+    w[k].X = static_cast<__nv_bfloat16*>(tr->X[j].p);
+    w[k].Y = static_cast<float*>(tr->Y.p);
+    w[k].dY = static_cast<float*>(tr->dY[j].p);
+    w[k].dH = static_cast<float*>(tr->dH.p);
+    w[k].dH2 = static_cast<float*>(tr->dH2.p);
+    w[k].dU = static_cast<float*>(tr->dU.p);
+    w[k].dAs = static_cast<float*>(tr->dAs.p);
+    w[k].dAs2 = static_cast<float*>(tr->dAs2.p);
+    w[k].part = static_cast<float*>(tr->part.p);
+  }
+  return CSTG_OK;
+}
+
+// The samples' forward passes on stream s (forward(r, z, work, scratch)), their losses, and the backward
+// passes on the trainer's second stream, in sample order, so the gradient's sums keep their order.
+// winvd: the weights of the loss's step. Returns with both streams finished.
+template <class Forward>
+int accumulate_samples(cstg_trainer* tr, cstg_ctx* ctx, int n_samples, const double* d_R, const double* d_E,
+                       double* losses, const double* winvd, cudaStream_t s, const MpnnGraph& g, const MpnnParams& P,
+                       Forward forward) {
+  const int N = ctx->n_nodes, n = ctx->n_rows;
+  const int sets = N <= kPipelineNodes && n_samples > 1 ? 2 : 1;
+  MpnnWork w[2];
+  const int rc = trainer_work(tr, N, sets, w);
+  if (rc) return rc;
+  TENSURE(tr->losses, sizeof(double) * (size_t)std::max(n_samples, 1));
+  const BlockMatrix bm = block_view(ctx);
+  double* z = static_cast<double*>(tr->z.p);
+  double* az = static_cast<double*>(tr->az.p);
+  double* d_loss = static_cast<double*>(tr->losses.p);
+  float* grad = static_cast<float*>(tr->grad.p);
+  int* err = buf_ptr<int>(ctx->err_word);
+  TK(cudaMemsetAsync(err, 0x7f, sizeof(int) * kErrSlots, s));
+  int rf = CSTG_OK;
+  cudaError_t e = cudaSuccess;
+  const auto ok = [&](cudaError_t x) {
+    if (e == cudaSuccess) e = x;
+    return e == cudaSuccess;
+  };
+  for (int i = 0; i < n_samples && e == cudaSuccess && !rf; ++i) {
+    const int k = i % sets;
+    const double* r = d_R + (size_t)i * n;
+    MpScratch* sc = static_cast<MpScratch*>(tr->sc[k].p);
+    if (i >= sets) ok(cudaStreamWaitEvent(s, tr->bwd_done[k], 0));  // its buffers are free again
+    rf = forward(r, z, w[k], sc);
+    if (rf) break;
+    ok(launch_spmv(&bm, nullptr, z, az, s));
+    ok(launch_mp_loss(N, z, az, r, d_E + (size_t)i * n, winvd, sc, w[k], s));
+    ok(cudaMemcpyAsync(d_loss + i, &sc->loss, sizeof(double), cudaMemcpyDeviceToDevice, s));
+    ok(cudaEventRecord(tr->fwd_done[k], s));
+    ok(cudaStreamWaitEvent(tr->back, tr->fwd_done[k], 0));
+    ok(launch_mp_backward(g, P, w[k], grad, ctx->mbar_spin, err, tr->back));
+    ok(cudaEventRecord(tr->bwd_done[k], tr->back));
+  }
+  // both streams have finished before anything returns, an error too
+  const cudaError_t eb = cudaStreamSynchronize(tr->back);
+  int h_err[kErrSlots];
+  ok(cudaMemcpyAsync(h_err, err, sizeof h_err, cudaMemcpyDeviceToHost, s));
+  if (losses && n_samples > 0 && !rf)
+    ok(cudaMemcpyAsync(losses, d_loss, sizeof(double) * (size_t)n_samples, cudaMemcpyDeviceToHost, s));
+  const cudaError_t es = cudaStreamSynchronize(s);
+  if (rf) return rf;
+  TK(e);
+  TK(eb);
+  TK(es);
+  if (h_err[kErrTimeout] != kErrNone) return tfail(tr, CSTG_ERR_TIMEOUT, "trainer: a tensor-core wait timed out");
   return CSTG_OK;
 }
 
@@ -549,20 +618,28 @@ cstg_trainer* cstg_trainer_create(int device, const float* params, int* status) 
   cstg_trainer* tr = new cstg_trainer();
   tr->device = device;
   int rc = CSTG_OK;
-  if (cudaStreamCreateWithFlags(&tr->stream, cudaStreamNonBlocking) != cudaSuccess) rc = CSTG_ERR_CUDA;
+  if (cudaStreamCreateWithFlags(&tr->stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&tr->back, cudaStreamNonBlocking) != cudaSuccess)
+    rc = CSTG_ERR_CUDA;
+  for (int k = 0; k < 2 && !rc; ++k)
+    if (cudaEventCreateWithFlags(&tr->fwd_done[k], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&tr->bwd_done[k], cudaEventDisableTiming) != cudaSuccess)
+      rc = CSTG_ERR_CUDA;
   if (!rc) rc = tensure(tr, tr->p32, sizeof(float) * kMpParams);
   if (!rc) rc = tensure(tr, tr->m, sizeof(float) * kMpParams);
   if (!rc) rc = tensure(tr, tr->v, sizeof(float) * kMpParams);
   if (!rc) rc = tensure(tr, tr->grad, sizeof(float) * kMpParams);
   if (!rc) rc = tensure(tr, tr->pb, sizeof(__nv_bfloat16) * kMpParams);
   if (!rc) rc = tensure(tr, tr->pf, sizeof(float) * kMpParams);
-  if (!rc) rc = tensure(tr, tr->sc, sizeof(MpScratch));
+  for (DevBuf& b : tr->sc)
+    if (!rc) rc = tensure(tr, b, sizeof(MpScratch));
   if (!rc && mpnn_prepare_device() != cudaSuccess) rc = CSTG_ERR_CUDA;
   if (!rc && (cudaMemcpyAsync(tr->p32.p, params, sizeof(float) * kMpParams, cudaMemcpyHostToDevice, tr->stream) ||
               cudaMemsetAsync(tr->m.p, 0, sizeof(float) * kMpParams, tr->stream) ||
               cudaMemsetAsync(tr->v.p, 0, sizeof(float) * kMpParams, tr->stream) ||
               cudaMemsetAsync(tr->grad.p, 0, sizeof(float) * kMpParams, tr->stream) ||
-              cudaMemsetAsync(tr->sc.p, 0, sizeof(MpScratch), tr->stream) ||
+              cudaMemsetAsync(tr->sc[0].p, 0, sizeof(MpScratch), tr->stream) ||
+              cudaMemsetAsync(tr->sc[1].p, 0, sizeof(MpScratch), tr->stream) ||
               launch_mp_params(static_cast<float*>(tr->p32.p), static_cast<__nv_bfloat16*>(tr->pb.p),
                                static_cast<float*>(tr->pf.p), tr->stream) ||
               cudaStreamSynchronize(tr->stream)))
@@ -580,13 +657,22 @@ void cstg_trainer_destroy(cstg_trainer* tr) {
   if (!tr) return;
   cudaSetDevice(tr->device);
   if (tr->stream) cudaStreamSynchronize(tr->stream);
-  DevBuf* all[] = {&tr->p32, &tr->m, &tr->v, &tr->grad, &tr->pb, &tr->pf, &tr->sc, &tr->az, &tr->z,
-                   &tr->X,   &tr->Y, &tr->dY, &tr->dH,  &tr->dH2, &tr->dU, &tr->dAs, &tr->dAs2, &tr->part};
+  if (tr->back) cudaStreamSynchronize(tr->back);
+  DevBuf* all[] = {&tr->p32, &tr->m, &tr->v, &tr->grad, &tr->pb, &tr->pf, &tr->az, &tr->z, &tr->losses,
+                   &tr->Y,   &tr->dH,  &tr->dH2, &tr->dU, &tr->dAs, &tr->dAs2, &tr->part};
   for (DevBuf* b : all) free_buf(*b);
-  for (auto& b : tr->H) free_buf(b);
-  for (auto& b : tr->G) free_buf(b);
-  for (auto& b : tr->A) free_buf(b);
+  for (int k = 0; k < 2; ++k) {
+    free_buf(tr->sc[k]);
+    free_buf(tr->X[k]);
+    free_buf(tr->dY[k]);
+    for (auto& b : tr->H[k]) free_buf(b);
+    for (auto& b : tr->G[k]) free_buf(b);
+    for (auto& b : tr->A[k]) free_buf(b);
+    if (tr->fwd_done[k]) cudaEventDestroy(tr->fwd_done[k]);
+    if (tr->bwd_done[k]) cudaEventDestroy(tr->bwd_done[k]);
+  }
   if (tr->stream) cudaStreamDestroy(tr->stream);
+  if (tr->back) cudaStreamDestroy(tr->back);
   delete tr;
 }
 
@@ -605,39 +691,20 @@ int cstg_trainer_accumulate(cstg_trainer* tr, cstg_ctx* ctx, int n_samples, cons
     return tfail(tr, CSTG_ERR_INVALID_ARGUMENT, "trainer_accumulate: bad samples");
   if (!aligned16(d_R) || !aligned16(d_E))
     return tfail(tr, CSTG_ERR_INVALID_ARGUMENT, "trainer_accumulate: samples must be 16-byte aligned");
-  const int N = ctx->n_nodes, n = ctx->n_rows;
-  MpnnWork w;
-  int rc = trainer_work(tr, N, w);
-  if (rc) return rc;
   TK(cudaStreamSynchronize(ctx->stream));  // the context's matrix and inputs are ready
   const MpnnGraph g = graph_view(ctx);
   MpnnParams P;
   P.pb = static_cast<const __nv_bfloat16*>(tr->pb.p);
   P.pf = static_cast<const float*>(tr->pf.p);
-  MpScratch* sc = static_cast<MpScratch*>(tr->sc.p);
-  const BlockMatrix bm = block_view(ctx);
   const double* invd = buf_ptr<double>(ctx->inv_diag);
-  double* z = static_cast<double*>(tr->z.p);
-  double* az = static_cast<double*>(tr->az.p);
-  float* grad = static_cast<float*>(tr->grad.p);
-  int* err = buf_ptr<int>(ctx->err_word);
-  TK(cudaMemsetAsync(err, 0x7f, sizeof(int) * kErrSlots, tr->stream));
-  for (int i = 0; i < n_samples; ++i) {
-    const double* r = d_R + (size_t)i * n;
-    const double* e = d_E + (size_t)i * n;
-    TK(launch_mp_rr(n, r, sc, tr->stream));
-    TK(launch_mp_forward(g, P, r, invd, &sc->rr, buf_ptr<float>(ctx->lp_sf), nullptr, w, true, nullptr, z,
-                         ctx->mbar_spin, err, tr->stream));
-    TK(launch_spmv(&bm, nullptr, z, az, tr->stream));
-    TK(launch_mp_loss(N, z, az, r, e, invd, sc, w, tr->stream));
-    if (losses) TK(cudaMemcpyAsync(&losses[i], &sc->loss, sizeof(double), cudaMemcpyDeviceToHost, tr->stream));
-    TK(launch_mp_backward(g, P, w, grad, ctx->mbar_spin, err, tr->stream));
-  }
-  int h_err[kErrSlots];
-  TK(cudaMemcpyAsync(h_err, err, sizeof h_err, cudaMemcpyDeviceToHost, tr->stream));
-  TK(cudaStreamSynchronize(tr->stream));
-  if (h_err[kErrTimeout] != kErrNone) return tfail(tr, CSTG_ERR_TIMEOUT, "trainer: a tensor-core wait timed out");
-  return CSTG_OK;
+  return accumulate_samples(tr, ctx, n_samples, d_R, d_E, losses, invd, tr->stream, g, P,
+                            [&](const double* r, double* z, MpnnWork& w, MpScratch* sc) -> int {
+                              TK(launch_mp_rr(ctx->n_rows, r, sc, tr->stream));
+                              TK(launch_mp_forward(g, P, r, invd, &sc->rr, buf_ptr<float>(ctx->lp_sf), nullptr, w, true,
+                                                   nullptr, z, ctx->mbar_spin, buf_ptr<int>(ctx->err_word),
+                                                   tr->stream));
+                              return CSTG_OK;
+                            });
 }
 
 int cstg_trainer_step(cstg_trainer* tr, float lr, float grad_scale) {
@@ -744,40 +811,18 @@ int cstg_trainer_accumulate_cycle(cstg_trainer* tr, cstg_ctx* ctx, int n_samples
     const int rc = cycle_ready(ctx);  // (the context's own error text on failure)
     if (rc) return tfail(tr, rc, "trainer_accumulate: %s", ctx->err.c_str());
   }
-  const int N = ctx->n_nodes, n = ctx->n_rows;
-  MpnnWork w;
-  int rc = trainer_work(tr, N, w);
-  if (rc) return rc;
-  // everything runs on the context's stream, where the hierarchy and the samples' producers are
+  // the forward passes run on the context's stream, where the hierarchy and the samples' producers are
   TK(cudaStreamSynchronize(tr->stream));
-  cudaStream_t s = ctx->stream;
   const MpnnGraph g = graph_view(ctx);
   MpnnParams P;
   P.pb = static_cast<const __nv_bfloat16*>(tr->pb.p);
   P.pf = static_cast<const float*>(tr->pf.p);
-  MpScratch* sc = static_cast<MpScratch*>(tr->sc.p);
-  const BlockMatrix bm = block_view(ctx);
   const double* winvd = buf_ptr<double>(ctx->lm_winvd);
-  double* z = static_cast<double*>(tr->z.p);
-  double* az = static_cast<double*>(tr->az.p);
-  float* grad = static_cast<float*>(tr->grad.p);
-  int* err = buf_ptr<int>(ctx->err_word);
-  TK(cudaMemsetAsync(err, 0x7f, sizeof(int) * kErrSlots, s));
-  for (int i = 0; i < n_samples; ++i) {
-    const double* r = d_R + (size_t)i * n;
-    const double* e = d_E + (size_t)i * n;
-    rc = cycle_apply(ctx, g, P, w, sc, winvd, r, z, nullptr, true, s);
-    if (rc) return tfail(tr, rc, "trainer_accumulate: %s", ctx->err.c_str());
-    TK(launch_spmv(&bm, nullptr, z, az, s));
-    TK(launch_mp_loss(N, z, az, r, e, winvd, sc, w, s));
-    if (losses) TK(cudaMemcpyAsync(&losses[i], &sc->loss, sizeof(double), cudaMemcpyDeviceToHost, s));
-    TK(launch_mp_backward(g, P, w, grad, ctx->mbar_spin, err, s));
-  }
-  int h_err[kErrSlots];
-  TK(cudaMemcpyAsync(h_err, err, sizeof h_err, cudaMemcpyDeviceToHost, s));
-  TK(cudaStreamSynchronize(s));
-  if (h_err[kErrTimeout] != kErrNone) return tfail(tr, CSTG_ERR_TIMEOUT, "trainer: a tensor-core wait timed out");
-  return CSTG_OK;
+  return accumulate_samples(tr, ctx, n_samples, d_R, d_E, losses, winvd, ctx->stream, g, P,
+                            [&](const double* r, double* z, MpnnWork& w, MpScratch* sc) -> int {
+                              const int rc = cycle_apply(ctx, g, P, w, sc, winvd, r, z, nullptr, true, ctx->stream);
+                              return rc ? tfail(tr, rc, "trainer_accumulate: %s", ctx->err.c_str()) : CSTG_OK;
+                            });
 }
 
 }  // extern "C"
