@@ -1465,7 +1465,7 @@ __global__ void __launch_bounds__(256) k_mp_dy(int n, const double* __restrict__
 // ---- training: backward ------------------------------------------------------------------------
 
 // dH3 = W_out' dY; partial gradients of W_out (2 x 64) and b_out (2) per block
-constexpr int kDecLanes = 16;  // node lanes of a block
+constexpr int kDecLanes = 4;  // node lanes of a block
 
 __global__ void __launch_bounds__(64 * kDecLanes) k_mp_dec_bwd(int N, const __nv_bfloat16* __restrict__ H3, MpnnParams P,
                                                     const float* __restrict__ dY, float* __restrict__ dH,
@@ -1710,14 +1710,13 @@ __global__ void __launch_bounds__(256) k_mp_wgrad(int N, const float* __restrict
 // Weight gradient of a message-passing layer on the tensor cores:
 //   dW^T[k][o] = sum_n Xc[n][k] dU[n][o]  (k < 128: Xc = [Hprev | A], o < 64),  db[o] = sum_n dU[n][o].
 // One CTA of 256 threads per contiguous node range and layer (blockIdx.y): the layers wait for nothing of one another and fill
-// the gaps of each other's copies, transposes and MMA waits (18 us each in turn, 34 together). Per chunk of 128 nodes: the Xc rows (BF16) and
+// the gaps of each other's copies, transposes and MMA waits (18 us each in turn, 45 us together). Per chunk of 128 nodes: the Xc rows (BF16) and
 // the dU rows (FP32, rounded to BF16; db summed in FP32 on the CUDA cores in node order) are
 // staged row-major, transposed into the K-major core-matrix layouts of the MMA operands
 // (A = Xc^T: 128 features x 128 nodes, B = dU^T: 64 outputs x 128 nodes; 8 nodes per 16-byte unit),
 // and one thread issues 8 tcgen05.mma (M=128, N=64, K=16) accumulating into 64 TMEM columns over
 // all chunks. Each warp of the first four then reads its 32 feature rows x 64 outputs.
 constexpr int kWgNodes = 128;
-constexpr int kWgBlocks = 98;  // per layer: three layers' blocks are one wave of two per SM
 constexpr int kWgSmem = kWgNodes * 2 * F * 2 /*Xc rows*/ + kWgNodes * F * 2 /*dU rows*/ + kASmem + kBSmem + 1024;
 
 struct WgradLayers {
@@ -1886,35 +1885,28 @@ __global__ void __launch_bounds__(256) k_mp_enc_bwd(int N, const int* __restrict
   }
 }
 
-// grad[dst + i] += sum over blocks b of part[b][i], for i < count: one segment per blockIdx.y (decoder,
-// the layers, encoder). Four threads share an element: each adds a quarter of the blocks in order, and
-// the quarters are added in a fixed tree.
+// grad[dst + i] += sum over blocks b (in order) of part[b][i], for i < count: one segment per
+// blockIdx.y (decoder, the layers, encoder), a thread per element with a quarter of its loads in flight.
 struct PartSegments {
   const float* part[kMpL + 2];
-  int blocks[kMpL + 2], stride[kMpL + 2], count[kMpL + 2], dst[kMpL + 2];
+  int stride[kMpL + 2], dst[kMpL + 2];  // (elements per block, place in the gradient)
 };
 
-__global__ void __launch_bounds__(256) k_mp_reduce_parts(const PartSegments g, float* __restrict__ grad) {
+__global__ void __launch_bounds__(64) k_mp_reduce_parts(const PartSegments g, float* __restrict__ grad) {
   const float* __restrict__ part = g.part[blockIdx.y];
-  const int stride = g.stride[blockIdx.y], count = g.count[blockIdx.y], nb = g.blocks[blockIdx.y];
-  // lanes 0-7: eight consecutive elements of quarter 0, lanes 8-15 of quarter 1, ...
-  const int lane = threadIdx.x & 31, quarter = lane >> 3;
-  const int i = (blockIdx.x * 256 + (int)threadIdx.x - lane) / 4 + (lane & 7);
-  const int b0 = nb * quarter / 4, b1 = nb * (quarter + 1) / 4;
+  const int stride = g.stride[blockIdx.y], i = blockIdx.x * 64 + (int)threadIdx.x;
+  if (i >= stride) return;
+  constexpr int kU = kMpPartBlocks / 4;
+  static_assert(kMpPartBlocks % kU == 0, "no remainder");
   float s = 0.f;
-  if (i < count) {
-    constexpr int kU = 16;  // blocks whose loads are in flight together
-    for (int b = b0; b < b1; b += kU) {
-      float v[kU];
+  for (int b = 0; b < kMpPartBlocks; b += kU) {
+    float v[kU];
 #pragma unroll
-      for (int u = 0; u < kU; ++u) v[u] = b + u < b1 ? part[(size_t)(b + u) * stride + i] : 0.f;
+    for (int u = 0; u < kU; ++u) v[u] = part[(size_t)(b + u) * stride + i];
 #pragma unroll
-      for (int u = 0; u < kU; ++u) s += v[u];
-    }
+    for (int u = 0; u < kU; ++u) s += v[u];
   }
-  s += __shfl_xor_sync(0xffffffffu, s, 8);
-  s += __shfl_xor_sync(0xffffffffu, s, 16);
-  if (quarter == 0 && i < count) grad[g.dst[blockIdx.y] + i] += s;
+  grad[g.dst[blockIdx.y] + i] += s;
 }
 
 // Adam (decoupled weight decay off): master FP32 parameters, BF16 copies for the kernels.
@@ -2204,14 +2196,13 @@ cudaError_t launch_mp_backward(const MpnnGraph& g, const MpnnParams& P, MpnnWork
   const int G = kMpPartBlocks;
   // partial sums of the layers, the decoder and the encoder, added at the end in one launch
   PartSegments seg;
-  const size_t layer_part = (size_t)kWgBlocks * kMpPartStride;
+  const size_t layer_part = (size_t)kMpPartBlocks * kMpPartStride;
   float* dec_part = w.part + kMpL * layer_part;
   float* enc_part = dec_part + (size_t)G * (2 * F + 2);
   // decoder
   k_mp_dec_bwd<<<G, 64 * kDecLanes, 0, s>>>(N, w.H[kMpL], P, w.dY, w.dH, dec_part);
   seg.part[0] = dec_part;
-  seg.blocks[0] = G;
-  seg.stride[0] = seg.count[0] = 2 * F + 2;  // (b_out follows W_out in the parameters too)
+  seg.stride[0] = 2 * F + 2;  // (b_out follows W_out in the parameters too)
   seg.dst[0] = kMpOffWout;
   // layers 3..1: each gathers the mean's transpose of the one above as it reads it
   const float *din = w.dH, *as = nullptr;
@@ -2226,22 +2217,20 @@ cudaError_t launch_mp_backward(const MpnnGraph& g, const MpnnParams& P, MpnnWork
     wl.H[l] = w.H[l];
     wl.A[l] = w.A[l];
     seg.part[1 + l] = w.part + l * layer_part;
-    seg.blocks[1 + l] = kWgBlocks;
-    seg.stride[1 + l] = seg.count[1 + l] = kMpPartStride;
+    seg.stride[1 + l] = kMpPartStride;
     seg.dst[1 + l] = kMpOffL0 + l * kMpLStride;
     din = dout;
     as = aout;
   }
-  k_mp_wgrad_tc<<<dim3(kWgBlocks, kMpL), 256, kWgSmem, s>>>(N, wl, spin_limit, w.part, err);
+  k_mp_wgrad_tc<<<dim3(kMpPartBlocks, kMpL), 256, kWgSmem, s>>>(N, wl, spin_limit, w.part, err);
   // encoder
   float* du0 = w.dU + (size_t)kMpL * N * F;
   k_mp_enc_bwd<<<grid_nodes((long long)N * (F / 4), 256), 256, 0, s>>>(N, g.node_ptr, g.nbr, din, as, w.H[0], du0);
   k_mp_wgrad<kMpIn><<<G, 256, 0, s>>>(N, du0, w.X, nullptr, enc_part);
   seg.part[1 + kMpL] = enc_part;
-  seg.blocks[1 + kMpL] = G;
-  seg.stride[1 + kMpL] = seg.count[1 + kMpL] = F * kMpIn + F;
+  seg.stride[1 + kMpL] = F * kMpIn + F;
   seg.dst[1 + kMpL] = kMpOffWin;
-  k_mp_reduce_parts<<<dim3((kMpPartStride + 63) / 64, kMpL + 2), 256, 0, s>>>(seg, grad);
+  k_mp_reduce_parts<<<dim3((kMpPartStride + 63) / 64, kMpL + 2), 64, 0, s>>>(seg, grad);
   count_launches(5 + kMpL);
   return cudaGetLastError();
 }
