@@ -121,6 +121,23 @@ int scan_total(cstg_ctx* ctx, const int* in, int n, int* out, int* total) {
   return read_int(ctx, out + n, total);
 }
 
+// lambda_max(D^-1 A) of level l on the FP32 operators the smoother applies: the finest level's difference
+// form, else this level's entry-major copy, built with the Galerkin product of the level above.
+int level_lambda(cstg_ctx* ctx, AmgData* d, int l) {
+  AmgLevel& lv = d->L[l];
+  const size_t m = (size_t)lv.n * lv.B;
+  ENSURE(lv.lam, sizeof(double));
+  ENSURE(d->part, amg_lambda_scratch());
+  ENSURE(d->vx, sizeof(double) * m);
+  ENSURE(d->vy, sizeof(double) * m);
+  const MixedMatrix mm = l == 0 ? mixed_view(ctx) : MixedMatrix{};
+  const AmgBsr32 a32 = lv.A32();
+  CK(amg_lambda_f32(l == 0 ? &mm : nullptr, l == 0 ? nullptr : &a32, buf_ptr<double>(lv.dinv), buf_ptr<double>(d->vx),
+                    buf_ptr<double>(d->vy), buf_ptr<double>(d->part), buf_ptr<double>(lv.lam), kPowerIters,
+                    ctx->stream));
+  return CSTG_OK;
+}
+
 // One coarsening step from level l (matrix and nullspace Bf set) to level l + 1.
 // theta: strength-of-connection threshold of the aggregation (0: every connection)
 int coarsen(cstg_ctx* ctx, AmgData* d, int l, double theta, bool* stop) {
@@ -138,21 +155,9 @@ int coarsen(cstg_ctx* ctx, AmgData* d, int l, double theta, bool* stop) {
   ENSURE(d->agg1, sizeof(int) * (size_t)n);
   ENSURE(d->agg2, sizeof(int) * (size_t)n);
   ENSURE(d->members, sizeof(int) * (size_t)n);
-  // lambda_max(D^-1 A)
-  ENSURE(lv.lam, sizeof(double));
-  ENSURE(d->part, amg_lambda_scratch());
-  ENSURE(d->vx, sizeof(double) * (size_t)n * B);
-  ENSURE(d->vy, sizeof(double) * (size_t)n * B);
-  // (on the FP32 operators the smoother applies: the finest level's difference form, else this
-  // level's entry-major copy, built with the Galerkin product of the level above)
-  if (l == 0) {
-    const MixedMatrix mm = mixed_view(ctx);
-    CK(amg_lambda_f32(&mm, nullptr, buf_ptr<double>(lv.dinv), buf_ptr<double>(d->vx), buf_ptr<double>(d->vy),
-                      buf_ptr<double>(d->part), buf_ptr<double>(lv.lam), kPowerIters, ctx->stream));
-  } else {
-    const AmgBsr32 a32 = lv.A32();
-    CK(amg_lambda_f32(nullptr, &a32, buf_ptr<double>(lv.dinv), buf_ptr<double>(d->vx), buf_ptr<double>(d->vy),
-                      buf_ptr<double>(d->part), buf_ptr<double>(lv.lam), kPowerIters, ctx->stream));
+  {
+    const int rc = level_lambda(ctx, d, l);
+    if (rc) return rc;
   }
   // the strong connections the aggregation follows (none dropped at theta 0)
   const unsigned char* strong = nullptr;
@@ -364,6 +369,9 @@ int amg_build(cstg_ctx* ctx) {
         CK(cudaMemsetAsync(buf_ptr<int>(ctx->err_word) + kErrAmg, 0x7f, sizeof(int), ctx->stream));
         rc = coarsen(ctx, d, l, 0.0, &stop);
       }
+      if (rc) return rc;
+    } else if (l == 0 && lv.n > 0) {  // (a finest level that is the coarsest too: the learned cycle's step needs it)
+      const int rc = level_lambda(ctx, d, 0);
       if (rc) return rc;
     }
     if (stop) break;
