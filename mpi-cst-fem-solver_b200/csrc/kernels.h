@@ -183,19 +183,20 @@ struct MpnnParams {  // device copies of the packed parameters
 };
 
 // Per-tile gather plan of the message-passing layers (built on the GPU from the pattern, once
-// per matrix): for each tile of 128 consecutive nodes, the rows its nodes read (their own and
-// their neighbours') as at most kPlanMaxRuns runs of consecutive nodes holding at most
-// kPlanMaxUnion rows, and per node its degree (neighbours without itself) and the positions of
-// its neighbours' rows (ascending pattern order) in that union; an unused position holds
-// kPlanNone, the row after the union (which the layers keep at -0.0, so a padded sum needs no
+// per matrix): for each tile of 128 consecutive nodes, the other rows its nodes' neighbours have as
+// at most kPlanMaxRuns runs of consecutive nodes holding at most kPlanMaxUnion rows, and per node its
+// degree (neighbours without itself) and its neighbours' places (ascending pattern order) in a stage of
+// the layer kernel, in 16-byte units: the tile's own rows first (128 bytes a row, chunk c of row m at
+// unit 8 m + (c ^ (m & 7)): place 8 m + (m & 7)), then the union's rows (plain). An unused place is
+// kPlanNone16, the row after the union (which the layers keep at -0.0, so a padded sum needs no
 // branch). A tile that does not fit is marked and its neighbours are gathered from global memory
-// instead.
-constexpr int kPlanMaxRuns = 8, kPlanMaxUnion = 400, kPlanMaxLocal = 7, kPlanSpan = 4096;
-constexpr int kPlanNone = kPlanMaxUnion;
+// instead. (279 other rows are what three stages leave room for; a tile of an O-grid has 260.)
+constexpr int kPlanMaxRuns = 9, kPlanMaxUnion = 279, kPlanMaxLocal = 7, kPlanSpan = 4096;
+constexpr int kPlanUnion16 = 128 * 8, kPlanNone16 = kPlanUnion16 + kPlanMaxUnion * 8;
 struct MpTilePlan {
-  const int4* hdr = nullptr;    // [tiles]: (runs, union rows, fallback, 0)
+  const int4* hdr = nullptr;    // [tiles]: (runs, union rows, fallback, a node lists 7 others)
   const int2* runs = nullptr;   // [tiles][kPlanMaxRuns]: (first node, rows)
-  const uint4* local = nullptr; // [nodes]: 8 uint16: [0] degree, [1..deg] neighbours, kPlanNone unused
+  const uint4* local = nullptr; // [nodes]: 8 uint16: [0] degree, [1..deg] places, kPlanNone16 unused
 };
 struct MpnnGraph {  // the node-block pattern (self included; the network skips self)
   int n_nodes = 0;

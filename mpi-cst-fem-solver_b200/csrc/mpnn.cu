@@ -211,14 +211,14 @@ __global__ void __launch_bounds__(256) k_mp_tile_plan(int N, const int* __restri
   constexpr int W = kPlanSpan / 32;
   __shared__ unsigned bits[W];
   __shared__ int wpre[W + 1], spre[W + 1], epre[W + 1];
-  __shared__ int s_lo, s_hi, s_fail;
+  __shared__ int s_lo, s_hi, s_fail, s_wide;
   __shared__ int rs[kPlanMaxRuns], re[kPlanMaxRuns];
   const int t = threadIdx.x, tile = blockIdx.x;
   const int a = tile * kTile, b = min(N, a + kTile);
   if (t == 0) {
     s_lo = INT_MAX;
     s_hi = -1;
-    s_fail = 0;
+    s_fail = s_wide = 0;
   }
   for (int w = t; w < W; w += blockDim.x) bits[w] = 0u;
   __syncthreads();
@@ -236,6 +236,7 @@ __global__ void __launch_bounds__(256) k_mp_tile_plan(int N, const int* __restri
   if (t < b - a) {  // every node lists itself (first the own row) and at most kPlanMaxLocal others
     const int d = node_ptr[a + t + 1] - node_ptr[a + t];
     if (d < 1 || d - 1 > kPlanMaxLocal) s_fail = 1;
+    if (d - 1 > kPlanMaxLocal - 1) s_wide = 1;
   }
   __syncthreads();
   const int wlo = s_lo;
@@ -244,8 +245,8 @@ __global__ void __launch_bounds__(256) k_mp_tile_plan(int N, const int* __restri
     return;
   }
   for (int e = e0 + t; e < e1; e += blockDim.x) {
-    const int d = nbr[e] - wlo;
-    atomicOr(&bits[d >> 5], 1u << (d & 31));
+    const int v = nbr[e], d = v - wlo;
+    if (v < a || v >= b) atomicOr(&bits[d >> 5], 1u << (d & 31));
   }
   __syncthreads();
   if (t == 0) {  // word prefix counts of the set bits, the run starts and the run ends
@@ -285,20 +286,21 @@ __global__ void __launch_bounds__(256) k_mp_tile_plan(int N, const int* __restri
   const int nruns = spre[W];
   if (t < kPlanMaxRuns)
     runs[(size_t)tile * kPlanMaxRuns + t] = t < nruns ? make_int2(rs[t], re[t] - rs[t] + 1) : make_int2(0, 0);
-  if (t == 0) hdr[tile] = make_int4(nruns, wpre[W], 0, 0);
-  if (t < b - a) {  // the node's own row first, then its neighbours in pattern order
+  if (t == 0) hdr[tile] = make_int4(nruns, wpre[W], 0, s_wide);
+  if (t < b - a) {  // the node's degree, then its neighbours in pattern order
     const int n = a + t;
-    auto rank = [&](int v) {
+    auto place = [&](int v) {  // 16-byte units; the own rows lie in the 128-byte swizzle
+      if (v >= a && v < b) return (v - a) * 8 | ((v - a) & 7);
       const int d = v - wlo;
-      return wpre[d >> 5] + __popc(bits[d >> 5] & ((1u << (d & 31)) - 1u));
+      return kPlanUnion16 + 8 * (wpre[d >> 5] + __popc(bits[d >> 5] & ((1u << (d & 31)) - 1u)));
     };
     uint16_t slot[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) slot[j] = (uint16_t)kPlanNone;
+    for (int j = 0; j < 8; ++j) slot[j] = (uint16_t)kPlanNone16;
     int k = 1;
     for (int e = node_ptr[n]; e < node_ptr[n + 1]; ++e) {
       const int v = nbr[e];
-      if (v != n) slot[k++] = (uint16_t)rank(v);
+      if (v != n) slot[k++] = (uint16_t)place(v);
     }
     slot[0] = (uint16_t)(k - 1);  // the degree (the layers read their own rows elsewhere)
     local[n] = make_uint4((uint32_t)slot[0] | ((uint32_t)slot[1] << 16), (uint32_t)slot[2] | ((uint32_t)slot[3] << 16),
@@ -579,31 +581,39 @@ __global__ void __launch_bounds__(kEncT, kEncCtasPerSm) k_mp_encode(int N, const
 }
 
 
-// Neighbour sums in FP32: acc[j] += feature j of the chunk v (8 BF16) with the mixed-precision
-// add.rn.f32.bf16 (the BF16 operand widened exactly, one IEEE round-to-nearest add: the same result
-// as widening and a scalar add, in one instruction per feature).
-__device__ __forceinline__ void add_chunk_bf(float (&acc)[8], const uint4 v) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-    asm("{\n\t.reg .b16 lo, hi;\n\t"
-        "mov.b32 {lo, hi}, %2;\n\t"
-        "add.rn.f32.bf16 %0, lo, %0;\n\t"
-        "add.rn.f32.bf16 %1, hi, %1;\n\t}\n"
-        : "+f"(acc[2 * q]), "+f"(acc[2 * q + 1])
-        : "r"(w[q]));
-}
-// g + the low / high BF16 of w, widened exactly: one IEEE round-to-nearest add (the bits of
-// bf_lo(w) + g, in one instruction).
-__device__ __forceinline__ float add_bf_lo(uint32_t w, float g) {
-  float d;
-  asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %1;\n\tadd.rn.f32.bf16 %0, lo, %2;\n\t}\n" : "=f"(d) : "r"(w), "f"(g));
+// Two FP32 values in one 64-bit register, and the packed adds and products on them: one instruction
+// for two IEEE round-to-nearest operations (the bits of the scalar ones).
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack_f2(uint32_t lo, uint32_t hi) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(d) : "r"(lo), "r"(hi));
   return d;
 }
-__device__ __forceinline__ float add_bf_hi(uint32_t w, float g) {
-  float d;
-  asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %1;\n\tadd.rn.f32.bf16 %0, hi, %2;\n\t}\n" : "=f"(d) : "r"(w), "f"(g));
+__device__ __forceinline__ float2 unpack_f2(f32x2 v) {
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(d.x), "=f"(d.y) : "l"(v));
   return d;
+}
+__device__ __forceinline__ f32x2 add_f2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul_f2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// The two BF16 of w, widened exactly (low one first).
+__device__ __forceinline__ f32x2 widen_bf2(uint32_t w) { return pack_f2(w << 16, w & 0xFFFF0000u); }
+
+// Neighbour sums in FP32: acc[q] += features 2q, 2q + 1 of the chunk v (8 BF16), the BF16 operands
+// widened exactly.
+__device__ __forceinline__ void add_chunk_bf(f32x2 (&acc)[4], const uint4 v) {
+  acc[0] = add_f2(acc[0], widen_bf2(v.x));
+  acc[1] = add_f2(acc[1], widen_bf2(v.y));
+  acc[2] = add_f2(acc[2], widen_bf2(v.z));
+  acc[3] = add_f2(acc[3], widen_bf2(v.w));
 }
 // Eight BF16 -0.0: the chunk a missing neighbour contributes. x + (-0) = x exactly for every x
 // (both zeros included), so a sum padded with it has the bits of the sum without it, and the
@@ -624,14 +634,21 @@ __device__ __forceinline__ float inv_deg(int deg) {
   return r;
 }
 // The chunk's mean as 8 BF16: each sum times inv, rounded to nearest.
-__device__ __forceinline__ uint4 mean_chunk(const float (&acc)[8], float inv) {
-  return make_uint4(pack_bf2(acc[0] * inv, acc[1] * inv), pack_bf2(acc[2] * inv, acc[3] * inv),
-                    pack_bf2(acc[4] * inv, acc[5] * inv), pack_bf2(acc[6] * inv, acc[7] * inv));
+__device__ __forceinline__ uint4 mean_chunk(const f32x2 (&acc)[4], float inv) {
+  const f32x2 ii = pack_f2(__float_as_uint(inv), __float_as_uint(inv));
+  const float2 a = unpack_f2(mul_f2(acc[0], ii)), b = unpack_f2(mul_f2(acc[1], ii)),
+               c = unpack_f2(mul_f2(acc[2], ii)), d = unpack_f2(mul_f2(acc[3], ii));
+  return make_uint4(pack_bf2(a.x, a.y), pack_bf2(b.x, b.y), pack_bf2(c.x, c.y), pack_bf2(d.x, d.y));
+}
+// The residual add of two features: the BF16 pair w of the node's own row, widened exactly, plus g.
+__device__ __forceinline__ uint32_t residual_bf2(uint32_t w, float g0, float g1) {
+  const float2 h = unpack_f2(add_f2(widen_bf2(w), pack_f2(__float_as_uint(g0), __float_as_uint(g1))));
+  return pack_bf2(h.x, h.y);
 }
 
 // A tile the plan takes: its union fits one stage in at most kPlanMaxRuns runs.
 __device__ __forceinline__ bool plan_takes(const int4 h) {
-  return h.z == 0 && h.x >= 1 && h.x <= kPlanMaxRuns && h.y >= 1 && h.y <= kPlanMaxUnion;
+  return h.z == 0 && h.x <= kPlanMaxRuns && h.y <= kPlanMaxUnion;
 }
 
 template <bool TRAIN, bool LAST>
@@ -740,7 +757,7 @@ __global__ void __launch_bounds__(kLT, kLayerCtasPerSm) k_mp_layer_tc(const MpLa
         const int k0 = __shfl_sync(0xffffffffu, np, li) - np0;
         const int k1 = __shfl_sync(0xffffffffu, np, li + 1) - np0;
         uint4 own = make_uint4(0u, 0u, 0u, 0u);
-        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        f32x2 acc[4] = {0ull, 0ull, 0ull, 0ull};
         int deg = 0;
         if (n < N) {
           own = __ldg(reinterpret_cast<const uint4*>(a.Hin + (size_t)n * F) + c);
@@ -928,65 +945,55 @@ __global__ void __launch_bounds__(kLT, kLayerCtasPerSm) k_mp_layer_tc(const MpLa
 //
 // The same layer as k_mp_layer_tc (same operands, same order of every addition: the same bits),
 // arranged as a pipeline of roles over the CTA's tiles so that the copies, the gathers, the MMAs
-// and the epilogues of consecutive tiles overlap. Shared memory holds a ring of three stages of the
-// tiles' own rows in the layout the MMA reads (used by the MMA and the epilogue), a ring of two
-// stages of the tiles' unions in plain layout (used by the gathers alone, so a stage is refilled as
-// soon as its gathers are done), two buffers of the A operand's mean half and, in tensor memory,
-// two accumulators of 64 columns.
-//  own producer (warp 20): copies a tile's own 128 rows with one 2-D tensor copy
-//            (cp.async.bulk.tensor, no multicast) in the 128-byte swizzle (K-major: the A operand's
-//            own half needs no copy through registers) into a stage its previous tile's epilogue has
-//            released.
-//  union producer (warp 22): copies the tile's union, one bulk copy per run of consecutive rows
-//            (cp.async.bulk), and the node slots with one more, into a stage its previous tile's
-//            gathers have released. Row kPlanNone of every stage holds -0.0 (the unused slots'
-//            row). A tile the plan does not take gets no union: its neighbours come from global
-//            memory.
+// and the epilogues of consecutive tiles overlap. Shared memory holds three stages, each with a tile's
+// own 128 rows in the layout the MMA reads, the other rows its nodes read (plain), and the mean half of
+// its A operand; tensor memory holds two accumulators of 64 columns.
+//  own producer (warp 24): copies a tile's own rows with one 2-D tensor copy (cp.async.bulk.tensor, no
+//            multicast) in the 128-byte swizzle (K-major: the A operand's own half needs no copy through
+//            registers) into a stage whose previous tile has left it.
+//  union producer (warp 26): copies the other rows, one bulk copy per run of consecutive rows
+//            (cp.async.bulk), as soon as the stage's previous gathers are done. The row after them holds
+//            -0.0 (the unused places' row). A tile the plan does not take gets none: its neighbours
+//            come from global memory.
 //  gather (warps 0..15): 8 nodes per warp, four at once with 8 lanes per node (lane c: features
-//            8c..8c+7); each node's 7 neighbour slots read (row address = one multiply-add, unused
-//            slots at the -0.0 row) and summed in pattern order with add.rn.f32.bf16, times 1/deg,
-//            rounded to BF16 into the mean half (K-major, 128-byte swizzle); one arrival per warp on
-//            the union stage (free) and on the mean half (ready).
-//  MMA (warp 21, one thread): 8 x tcgen05.mma (M=128, N=64, K=16: four K-slices of the own rows,
+//            8c..8c+7); the rows at a node's six places (the seventh only in tiles that have such a node)
+//            are read and summed in pattern order with packed FP32 adds, times 1/deg, rounded to BF16 into
+//            the mean half (K-major, 128-byte swizzle); one arrival per warp on the union (free) and on
+//            the mean half (ready). The next tile's places are loaded a tile ahead.
+//  MMA (warp 25, one thread): 8 x tcgen05.mma (M=128, N=64, K=16: four K-slices of the own rows,
 //            four of the means) and the bias slice (ones x the FP32 bias split into three BF16
-//            parts) into the accumulator; tcgen05.commit arrives on the accumulator's barrier,
-//            which frees the mean half and starts the epilogue.
-//  epilogue (warps 16..19, warp 16+q on TMEM lanes 32q..32q+31, one thread per node): reads the
-//            node's own row (the residual; its first half while the MMA runs) and the accumulator
-//            (2 x tcgen05.ld.32x32b.x32), applies ReLU and the residual, writes each chunk into a
-//            128-byte swizzled staging buffer, releases the accumulator and the own stage, and
-//            stores the warp's 32 rows with one 2-D tensor store. The last layer runs the decoder per thread (features
-//            0..63 in order) and writes z.
+//            parts) into the accumulator; tcgen05.commit arrives on the accumulator's barrier.
+//  epilogue (two groups of four warps, group g on accumulator g; a group's warp q on TMEM lanes
+//            32q..32q+31, one thread per node): reads the node's own row (the residual; its first half
+//            while the MMA runs) and the accumulator (2 x tcgen05.ld.32x32b.x32), applies ReLU and the
+//            residual, writes each chunk over the own row it came from, and stores the warp's 32 rows with
+//            one 2-D tensor store. The last layer runs the decoder per thread (features 0..63 in order)
+//            and writes z.
 // Waits suspend in the hardware between polls (a 2 us hint), so the waiting warps take few
 // issue slots; each is bounded (spin_limit polls). A role that gives up records the timeout and
 // raises the CTA's abort flag, which every other wait polls. Before the CTA leaves, the copies and
 // MMAs already issued have completed (bounded waits) and the tensor stores have read their staging.
-// Measured on the 2M-DOF plate (120.8 us for the previous two-CTA kernel whose tile warps gathered,
-// issued and ran the epilogue in turn): 8 gather warps and a union in swizzled 8-row boxes 186 us,
-// one own box and bulk runs 154 us; the gather was the limit, two warps per scheduler with a
-// swizzled-or-plain address per neighbour and a branch around each neighbour's adds. This layout
-// (16 gather warps, plain union addressing, no branches) ran at 106 us, and at 88 us (0.47 of the
-// measured HBM bandwidth) once the tile headers and runs were loaded a tile ahead; it is then
-// bound by instruction issue and shared-memory latency, not by HBM.
+// Bound by the gathers' instructions (73 % of the issue slots; shared memory 61 %), not by HBM. Measured on
+// the 2M-DOF plate, 86 us a layer and 100 us the last (41 at the measured HBM bandwidth). Before: 89 and
+// 107 us with the own rows copied twice, two stages, a barrier per kind of copy, seven places summed with
+// scalar adds, and four epilogue warps, which were the last layer's limit. A third stage, other rows alone in the
+// union, or fewer adds gave nothing by themselves; dropping waits from the gather warps' path did (each costs
+// ~270 cycles behind their loads). 16 gather warps and plain rows without branches were worth 186 -> 106 us.
 constexpr int kWsGatherWarps = 16, kWsEpiWarps = 4;
 constexpr int kWsEpi0 = kWsGatherWarps;                    // warps 16..19 (TMEM lane quarters 0..3)
-constexpr int kWsOwnProd = kWsEpi0 + kWsEpiWarps;          // warp 20
-constexpr int kWsMma = kWsOwnProd + 1;                     // warp 21
-constexpr int kWsUnionProd = kWsMma + 1;                   // warp 22
-constexpr int kWsT = (kWsUnionProd + 1) * 32;              // 736 threads (at most 88 registers each)
-constexpr int kWsOwnStages = 3, kWsUStages = 2;
-constexpr int kWsOwn = kTile * 128;                        // own stage: 128 rows
-constexpr int kWsSlots = (kPlanMaxUnion + 1) * 128;        // union stage: the rows, the -0.0 row,
-constexpr int kWsUStage = kWsSlots + kTile * 16;           // then the tile's node slots
-constexpr int kWsStore = 32 * 128;                         // staging: a warp's 32 rows
+constexpr int kWsOwnProd = kWsEpi0 + 2 * kWsEpiWarps;      // warp 24
+constexpr int kWsMma = kWsOwnProd + 1;                     // warp 25
+constexpr int kWsUnionProd = kWsMma + 1;                   // warp 26
+constexpr int kWsT = (kWsUnionProd + 1) * 32;              // 864 threads (at most 72 registers each)
+constexpr int kWsStages = 3;
+constexpr int kWsOwn = kTile * 128;                        // a stage: the own rows, the union's rows,
+constexpr int kWsMean = kWsOwn + (kPlanMaxUnion + 1) * 128;   // the -0.0 row, the mean half
+constexpr int kWsStage = kWsMean + kTile * 128;
+static_assert(kPlanUnion16 * 16 == kWsOwn && kPlanNone16 * 16 == kWsMean - 128, "the plan's places");
 constexpr int kWsOffOwn = kBSmem + kBiasSmem;              // after B, the ones and the bias parts
-constexpr int kWsOffMean = kWsOffOwn + kWsOwnStages * kWsOwn;
-constexpr int kWsOffSt = kWsOffMean + 2 * kTile * 128;
-constexpr int kWsOffU = kWsOffSt + kWsEpiWarps * kWsStore;
-constexpr int kWsSmem = kWsOffU + kWsUStages * kWsUStage + 1024;  // (+ the 1024-byte alignment)
-static_assert(kWsOffOwn % 1024 == 0 && kWsOffMean % 1024 == 0 && kWsOffSt % 1024 == 0,
+constexpr int kWsSmem = kWsOffOwn + kWsStages * kWsStage + 1024;  // (+ the 1024-byte alignment)
+static_assert(kWsOffOwn % 1024 == 0 && kWsStage % 1024 == 0 && kWsMean % 1024 == 0 && kWsEpi0 % 4 == 0,
               "the 128-byte swizzle's atoms start on 1024-byte boundaries");
-static_assert(kWsOffU % 16 == 0 && kWsUStage % 16 == 0, "bulk copies land on 16-byte boundaries");
 static_assert(kWsSmem + 1024 <= 227 * 1024, "one CTA per SM");
 constexpr uint32_t kWsSuspendNs = 2000;  // suspend hint of a wait's poll
 
@@ -1020,35 +1027,52 @@ __device__ __forceinline__ void sts128(uint32_t addr, const uint4 v) {
                : "memory");
 }
 
-// Bounded wait that suspends between polls (up to kWsSuspendNs each); false when `limit` polls
-// ran out or another role raised `abort_flag`.
-__device__ __forceinline__ bool ws_poll(uint32_t bar, uint32_t parity, long long limit, const volatile int* abort_flag) {
-  for (long long i = 0; i < limit; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(kWsSuspendNs)
-        : "memory");
-    if (ok) return true;
-    if (*abort_flag) return false;
-  }
-  return false;
+// One poll of an mbarrier's phase; a poll that fails has been suspended for up to kWsSuspendNs.
+__device__ __forceinline__ bool ws_try(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(kWsSuspendNs)
+      : "memory");
+  return ok != 0;
 }
-// A role's wait: true when the phase completed; false when another role stopped first or the limit
-// ran out (then the timeout is recorded and every role told to stop). `warp_wide`: the whole warp
-// waits and takes the same decision.
-__device__ __forceinline__ bool ws_wait(uint32_t bar, uint32_t parity, long long limit, volatile int* abort_v,
-                                        int* err, int tile, bool warp_wide = true) {
-  const bool ok = ws_poll(bar, parity, limit, abort_v);
-  if (!ok && !*abort_v) {
+// Bounded wait; false when `limit` polls ran out (then the timeout is recorded and every role told to
+// stop) or another role raised `abort_v`.
+__device__ __noinline__ bool ws_poll(uint32_t bar, uint32_t parity, long long limit, volatile int* abort_v, int* err,
+                                     int tile) {
+  for (long long i = 1; i < limit; ++i) {
+    if (ws_try(bar, parity)) return true;
+    if (*abort_v) return false;
+  }
+  if (!*abort_v) {
     if (err) atomicMin(&err[kErrTimeout], tile);
     *abort_v = 1;
   }
-  return warp_wide ? __all_sync(0xffffffffu, ok) : ok;
+  return false;
 }
+// A role's wait: true when the phase completed (most waits at their first poll). `warp_wide`: the whole
+// warp waits and takes the same decision.
+__device__ __forceinline__ bool ws_wait(uint32_t bar, uint32_t parity, long long limit, volatile int* abort_v,
+                                        int* err, int tile, bool warp_wide = true) {
+  bool ok = limit > 0 && ws_try(bar, parity);
+  if (!warp_wide) return ok || ws_poll(bar, parity, limit, abort_v, err, tile);
+  if (__all_sync(0xffffffffu, ok)) return true;
+  if (!ok) ok = ws_poll(bar, parity, limit, abort_v, err, tile);
+  return __all_sync(0xffffffffu, ok);
+}
+// Stage k % 3 and phase (k / 3) & 1 of a role's tile k, stepped without divisions.
+struct WsStage {
+  uint32_t s = 0, phase = 0;
+  __device__ __forceinline__ void next() {
+    if (++s == (uint32_t)kWsStages) {
+      s = 0;
+      phase ^= 1u;
+    }
+  }
+};
 
 template <bool TRAIN, bool LAST>
 __global__ void __launch_bounds__(kWsT, 1)
@@ -1061,10 +1085,10 @@ __global__ void __launch_bounds__(kWsT, 1)
     return;
   }
   extern __shared__ uint8_t smem_raw[];
-  // own ring (3): full / empty; union ring (2): full / empty; mean halves and accumulators (2):
-  // mean ready, MMA done, accumulator empty
-  __shared__ uint64_t o_full[kWsOwnStages], o_empty[kWsOwnStages], u_full[kWsUStages], u_empty[kWsUStages];
-  __shared__ uint64_t m_full[2], mma_done[2], acc_empty[2];
+  // stages: full (both producers), union and own rows free, mean ready; accumulators (2): MMA done,
+  // free
+  __shared__ uint64_t full[kWsStages], o_empty[kWsStages], u_empty[kWsStages], m_full[kWsStages];
+  __shared__ uint64_t mma_done[2], acc_empty[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   __shared__ __align__(16) float wout[2 * F];
@@ -1074,10 +1098,7 @@ __global__ void __launch_bounds__(kWsT, 1)
   uint8_t* sB = base;  // element (n, k): (k/8)*1024 + (n/8)*128 + (n%8)*16 + (k%8)*2
   uint8_t* sOnes = base + kBSmem;
   uint8_t* sBias = sOnes + 4096;
-  uint8_t* sOwn = base + kWsOffOwn;    // own stage s: row m at m*128, 128-byte swizzle
-  uint8_t* sMean = base + kWsOffMean;  // mean half b: row m at m*128, 128-byte swizzle
-  uint8_t* sSt = base + kWsOffSt;      // epilogue warp q's staging: 32 rows, 128-byte swizzle
-  uint8_t* sU = base + kWsOffU;        // union stage s: slot j at j*128 (plain), then the node slots
+  uint8_t* sOwn = base + kWsOffOwn;    // stage s: own row m at m*128 (128-byte swizzle), the union, the mean half
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const __nv_bfloat16* W = a.P.pb + kMpOffL0 + a.layer * kMpLStride;
   if (t < kTile) {
@@ -1094,9 +1115,9 @@ __global__ void __launch_bounds__(kWsT, 1)
     *reinterpret_cast<uint4*>(sBias + (n >> 3) * 128 + (n & 7) * 16) =
         make_uint4(w0, (uint32_t)__bfloat16_as_ushort(b2), 0u, 0u);
     *reinterpret_cast<uint4*>(sBias + 1024 + (n >> 3) * 128 + (n & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
-  } else if (t < kTile + F + 8 * kWsUStages) {  // the -0.0 row of each union stage
+  } else if (t < kTile + F + 8 * kWsStages) {  // the -0.0 row of each stage
     const int j = t - kTile - F;
-    *reinterpret_cast<uint4*>(sU + (size_t)(j >> 3) * kWsUStage + kPlanNone * 128 + (j & 7) * 16) =
+    *reinterpret_cast<uint4*>(sOwn + (size_t)(j >> 3) * kWsStage + (kPlanNone16 + (j & 7)) * 16) =
         make_uint4(kNegZero2, kNegZero2, kNegZero2, kNegZero2);
   }
   for (int idx = t; idx < F * 16; idx += blockDim.x) {  // 64 rows x 16 chunks of 8 BF16
@@ -1117,16 +1138,13 @@ __global__ void __launch_bounds__(kWsT, 1)
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
   if (t == 0) {
-    for (int j = 0; j < kWsOwnStages; ++j) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&o_full[j])), "r"(1));
+    for (int j = 0; j < kWsStages; ++j) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&full[j])), "r"(2));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&o_empty[j])), "r"(kWsEpiWarps));
-    }
-    for (int j = 0; j < kWsUStages; ++j) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&u_full[j])), "r"(1));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&u_empty[j])), "r"(kWsGatherWarps));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&m_full[j])), "r"(kWsGatherWarps));
     }
     for (int j = 0; j < 2; ++j) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&m_full[j])), "r"(kWsGatherWarps));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&mma_done[j])), "r"(1));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&acc_empty[j])), "r"(kWsEpiWarps));
     }
@@ -1139,51 +1157,54 @@ __global__ void __launch_bounds__(kWsT, 1)
   const uint32_t tmem = tmem_slot;
   volatile int* abort_v = &abort_flag;
   const long long lim = a.spin_limit;
-  const uint32_t ofull0 = smem_u32(&o_full[0]), oempty0 = smem_u32(&o_empty[0]), ufull0 = smem_u32(&u_full[0]),
-                 uempty0 = smem_u32(&u_empty[0]), mfull0 = smem_u32(&m_full[0]), mdone0 = smem_u32(&mma_done[0]),
-                 aempty0 = smem_u32(&acc_empty[0]);
-  // tile k of this CTA: own stage k % 3 (use k / 3); union stage, mean half and accumulator k % 2
-  // (use k / 2)
+  const uint32_t full0 = smem_u32(&full[0]), oempty0 = smem_u32(&o_empty[0]), uempty0 = smem_u32(&u_empty[0]),
+                 mfull0 = smem_u32(&m_full[0]), mdone0 = smem_u32(&mma_done[0]), aempty0 = smem_u32(&acc_empty[0]);
+  // tile k of this CTA: stage k % 3 (use k / 3); accumulator and epilogue group k % 2 (use k / 2)
 
   if (warp < kWsGatherWarps) {
     // ---- gather: the mean half of the A operand
     const int g = lane >> 3, c = lane & 7;
-    int kt = 0;
+    const uint32_t c2 = (uint32_t)c * 0x10001u;
     int4 ph = (int)blockIdx.x * kTile < N ? __ldg(&a.plan.hdr[blockIdx.x]) : make_int4(0, 0, 1, 0);
-    for (int tile = blockIdx.x; tile * kTile < N; tile += gridDim.x, ++kt) {
-      const int hs = kt & 1;
-      const uint32_t hpar = (uint32_t)(kt >> 1) & 1u;
-      const bool planned = plan_takes(ph);
-      const int next = tile + (int)gridDim.x;  // its header arrives during this tile
-      ph = next * kTile < N ? __ldg(&a.plan.hdr[next]) : make_int4(0, 0, 1, 0);
-      if (!ws_wait(ufull0 + 8u * hs, hpar, lim, abort_v, a.err, tile)) break;
-      if (kt >= 2 && !ws_wait(mdone0 + 8u * hs, hpar ^ 1u, lim, abort_v, a.err, tile)) break;  // mean half free
-      const uint32_t row_a = smem_u32(sU + (size_t)hs * kWsUStage) + ((uint32_t)c << 4);  // chunk c of slot 0
-      const uint32_t slot_a = smem_u32(sU + (size_t)hs * kWsUStage + kWsSlots);
-      const uint32_t mean_a = smem_u32(sMean + (size_t)hs * kTile * 128);
-      uint4 lp[2];  // both rounds' slots first
+    uint4 lnext[2];  // both rounds' places
+    auto places = [&](int tl) {
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int m = warp * 8 + u * 4 + g;
-        constexpr uint32_t kNone2 = (uint32_t)kPlanNone * 0x10001u;
-        lp[u] = planned && tile * kTile + m < N ? lds128(slot_a + (uint32_t)m * 16u)
-                                                : make_uint4((uint32_t)kPlanNone << 16, kNone2, kNone2, kNone2);
-      }
+      for (int u = 0; u < 2; ++u)
+        lnext[u] = __ldg(&a.plan.local[min(tl * kTile + warp * 8 + u * 4 + g, N - 1)]);
+    };
+    places(blockIdx.x);
+    WsStage at;
+    for (int tile = blockIdx.x; tile * kTile < N; tile += gridDim.x, at.next()) {
+      const uint32_t us = at.s;
+      const bool planned = plan_takes(ph), wide = ph.w != 0;
+      const uint4 lp[2] = {lnext[0], lnext[1]};
+      const int next = tile + (int)gridDim.x;  // its header and places arrive during this tile
+      ph = next * kTile < N ? __ldg(&a.plan.hdr[next]) : make_int4(0, 0, 1, 0);
+      places(next);
+      // full: the tile's rows have landed, and (the own rows' place was free) the MMA of the stage's
+      // previous tile has read its mean half
+      if (!ws_wait(full0 + 8u * us, at.phase, lim, abort_v, a.err, tile)) break;
+      const uint32_t stage_a = smem_u32(sOwn + (size_t)us * kWsStage);
+      const uint32_t mean_a = stage_a + kWsMean;
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int m = warp * 8 + u * 4 + g;
         const int n = tile * kTile + m;
-        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        f32x2 acc[4] = {0ull, 0ull, 0ull, 0ull};
         int deg = 0;
-        if (planned) {
-          const uint32_t sl[7] = {lp[u].x >> 16, lp[u].y & 0xFFFFu, lp[u].y >> 16, lp[u].z & 0xFFFFu,
-                                  lp[u].z >> 16, lp[u].w & 0xFFFFu, lp[u].w >> 16};
-          uint4 v[7];
+        if (planned && n < N) {
+          // chunk c of the row at place e is at unit e ^ c: own rows carry their swizzle key in e's
+          // low bits, the union's are plain
+          const uint32_t w[4] = {lp[u].x ^ (c2 & 0xFFFF0000u), lp[u].y ^ c2, lp[u].z ^ c2, lp[u].w ^ c2};
+          const uint32_t sl[7] = {w[0] >> 16, w[1] & 0xFFFFu, w[1] >> 16, w[2] & 0xFFFFu,
+                                  w[2] >> 16, w[3] & 0xFFFFu, w[3] >> 16};
+          uint4 v[6];
 #pragma unroll
-          for (int j = 0; j < 7; ++j) v[j] = lds128(row_a + sl[j] * 128u);  // (unused: the -0.0 row)
+          for (int j = 0; j < 6; ++j) v[j] = lds128(stage_a + sl[j] * 16u);  // (unused: the -0.0 row)
           deg = (int)(lp[u].x & 0xFFFFu);
 #pragma unroll
-          for (int j = 0; j < 7; ++j) add_chunk_bf(acc, v[j]);
+          for (int j = 0; j < 6; ++j) add_chunk_bf(acc, v[j]);
+          if (wide) add_chunk_bf(acc, lds128(stage_a + sl[6] * 16u));
         } else if (n < N) {  // neighbours from global memory, in pattern order
           const int k0 = __ldg(&a.node_ptr[n]), k1 = __ldg(&a.node_ptr[n + 1]);
           for (int k = k0; k < k1; k += 8) {
@@ -1210,20 +1231,22 @@ __global__ void __launch_bounds__(kWsT, 1)
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(uempty0 + 8u * hs);  // the union stage is free
-        mbar_arrive(mfull0 + 8u * hs);   // the mean half is ready
+        mbar_arrive(uempty0 + 8u * us);  // the stage's union is free
+        mbar_arrive(mfull0 + 8u * us);   // the mean half is ready
       }
     }
   } else if (warp < kWsOwnProd) {
-    // ---- epilogue: one node per thread, its row chunk by chunk
-    const int q = warp - kWsEpi0;
+    // ---- epilogue: one node per thread, its row chunk by chunk; group hs takes the tiles of
+    // accumulator hs
+    const int q = (warp - kWsEpi0) & 3, hs = (warp - kWsEpi0) >> 2;
     const int m = q * 32 + lane;
     const double sc = LAST ? sqrt(*a.rr * a.inv_n) : 0.0;
-    const uint32_t st = smem_u32(sSt + (size_t)q * kWsStore) + (uint32_t)lane * 128u;  // the thread's staged row
-    int kt = 0;
-    for (int tile = blockIdx.x; tile * kTile < N; tile += gridDim.x, ++kt) {
-      const int os = kt % kWsOwnStages, hs = kt & 1;
-      const uint32_t opar = (uint32_t)(kt / kWsOwnStages) & 1u, hpar = (uint32_t)(kt >> 1) & 1u;
+    WsStage at;
+    if (hs) at.next();
+    uint32_t hpar = 1;  // tile k: phase (k / 2) & 1
+    for (int tile = blockIdx.x + hs * (int)gridDim.x; tile * kTile < N; tile += 2 * (int)gridDim.x, at.next(), at.next()) {
+      const uint32_t os = at.s, opar = at.phase;
+      hpar ^= 1u;
       const int n = tile * kTile + m;
       const int row0 = tile * kTile + q * 32;
       const bool store = a.Hout && row0 < N;  // warp-uniform
@@ -1234,11 +1257,10 @@ __global__ void __launch_bounds__(kWsT, 1)
         dn_e = reinterpret_cast<const double2*>(a.invd)[n];
         if (a.zbase) zb_e = reinterpret_cast<const double2*>(a.zbase)[n];
       }
-      if (store && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");  // staging free
-      if (!ws_wait(ofull0 + 8u * os, opar, lim, abort_v, a.err, tile)) break;
+      if (!ws_wait(full0 + 8u * os, opar, lim, abort_v, a.err, tile)) break;
       // the residual (the node's own row): the first half read while the MMA runs, the second
       // while the accumulator's second half is read
-      const uint32_t own_a = smem_u32(sOwn + (size_t)os * kWsOwn) + (uint32_t)m * 128u;
+      const uint32_t own_a = smem_u32(sOwn + (size_t)os * kWsStage) + (uint32_t)m * 128u;
       uint4 res[4];
 #pragma unroll
       for (int cc = 0; cc < 4; ++cc) res[cc] = lds128(own_a + ((uint32_t)(cc ^ (m & 7)) << 4));
@@ -1262,7 +1284,7 @@ __global__ void __launch_bounds__(kWsT, 1)
           for (int j = 0; j < 4; ++j) {  // (the accumulator holds the bias already)
             const float g0 = fmaxf(__uint_as_float(v[cc * 8 + 2 * j]), 0.f);
             const float g1 = fmaxf(__uint_as_float(v[cc * 8 + 2 * j + 1]), 0.f);
-            hw[j] = pack_bf2(add_bf_lo(ow[j], g0), add_bf_hi(ow[j], g1));
+            hw[j] = residual_bf2(ow[j], g0, g1);
             gw[j] = pack_bf2(g0, g1);
           }
           if (TRAIN && n < N)
@@ -1282,14 +1304,14 @@ __global__ void __launch_bounds__(kWsT, 1)
               if (o) y1 = y; else y0 = y;
             }
           }
-          if (store) sts128(st + ((uint32_t)(ch ^ (lane & 7)) << 4), make_uint4(hw[0], hw[1], hw[2], hw[3]));
+          if (store) sts128(own_a + ((uint32_t)(ch ^ (m & 7)) << 4), make_uint4(hw[0], hw[1], hw[2], hw[3]));
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(aempty0 + 8u * hs);  // the accumulator is free
-        mbar_arrive(oempty0 + 8u * os);  // the own stage is free (its MMA has completed)
+        if (!store) mbar_arrive(oempty0 + 8u * os);  // the own rows are free (their MMA has completed)
       }
       if (LAST && n < N) {
         if (TRAIN) reinterpret_cast<float2*>(a.Yout)[n] = make_float2(y0, y1);
@@ -1304,8 +1326,10 @@ __global__ void __launch_bounds__(kWsT, 1)
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         __syncwarp();
         if (lane == 0) {
-          tma_store_rows(&tout, row0, smem_u32(sSt + (size_t)q * kWsStore));
+          tma_store_rows(&tout, row0, smem_u32(sOwn + (size_t)os * kWsStage + (size_t)q * 32 * 128));
           asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+          asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+          mbar_arrive(oempty0 + 8u * os);  // the own rows' place is free
         }
       }
     }
@@ -1316,42 +1340,43 @@ __global__ void __launch_bounds__(kWsT, 1)
     if (lane == 0) {
       asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&tin)) : "memory");
       for (int tile = blockIdx.x; tile * kTile < N; tile += gridDim.x, ++kt) {
-        const int os = kt % kWsOwnStages;
-        if (kt >= kWsOwnStages &&
-            !ws_wait(oempty0 + 8u * os, (uint32_t)(kt / kWsOwnStages - 1) & 1u, lim, abort_v, a.err, tile, false))
+        const int os = kt % kWsStages;
+        if (kt >= kWsStages &&
+            !ws_wait(oempty0 + 8u * os, (uint32_t)(kt / kWsStages - 1) & 1u, lim, abort_v, a.err, tile, false))
           break;
-        const uint32_t fb = ofull0 + 8u * os;
+        const uint32_t fb = full0 + 8u * os;
         // the epilogue's generic reads of this stage are ordered before the copy's writes
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb), "r"((uint32_t)kWsOwn)
                      : "memory");
-        tma_load_rows(smem_u32(sOwn + (size_t)os * kWsOwn), &tin, tile * kTile, fb);  // (past N: zeros)
+        tma_load_rows(smem_u32(sOwn + (size_t)os * kWsStage), &tin, tile * kTile, fb);  // (past N: zeros)
       }
       // the copies issued land before the CTA leaves (bounded)
-      for (int j = max(0, kt - kWsOwnStages); j < kt; ++j)
-        mbar_wait(ofull0 + 8u * (j % kWsOwnStages), (uint32_t)(j / kWsOwnStages) & 1u, kMbarSpinLimit);
+      for (int j = max(0, kt - kWsStages); j < kt; ++j)
+        mbar_wait(full0 + 8u * (j % kWsStages), (uint32_t)(j / kWsStages) & 1u, kMbarSpinLimit);
     }
   } else if (warp == kWsUnionProd) {
     // ---- union producer: each tile's union and its node slots
     int kt = 0;
-    // lane j: run j (first node, rows) of the tile; the next tile's header and runs are loaded
-    // while this tile waits for its stage
-    auto tile_runs = [&](int tl, int4& h, int2& r) {
-      h = tl * kTile < N ? __ldg(&a.plan.hdr[tl]) : make_int4(0, 0, 1, 0);
-      r = plan_takes(h) && lane < h.x ? __ldg(&a.plan.runs[(size_t)tl * kPlanMaxRuns + lane]) : make_int2(0, 0);
+    // lane j: run j (first node, rows) of the tile; headers are loaded two tiles ahead, runs one
+    auto tile_hdr = [&](int tl) { return tl * kTile < N ? __ldg(&a.plan.hdr[tl]) : make_int4(0, 0, 1, 0); };
+    auto tile_runs = [&](int tl, const int4 h) {
+      return plan_takes(h) && lane < h.x ? __ldg(&a.plan.runs[(size_t)tl * kPlanMaxRuns + lane]) : make_int2(0, 0);
     };
-    int4 ph_next;
-    int2 rn_next;
-    tile_runs(blockIdx.x, ph_next, rn_next);
-    for (int tile = blockIdx.x; tile * kTile < N; tile += gridDim.x, ++kt) {
-      const int us = kt & 1;
+    const int step = (int)gridDim.x;
+    int4 ph_next = tile_hdr(blockIdx.x), ph_far = tile_hdr(blockIdx.x + step);
+    int2 rn_next = tile_runs(blockIdx.x, ph_next);
+    for (int tile = blockIdx.x; tile * kTile < N; tile += step, ++kt) {
+      const int us = kt % kWsStages;
       const int4 ph = ph_next;
       const int2 rn = rn_next;
-      tile_runs(tile + (int)gridDim.x, ph_next, rn_next);
-      if (kt >= kWsUStages && !ws_wait(uempty0 + 8u * us, (uint32_t)((kt >> 1) - 1) & 1u, lim, abort_v, a.err, tile))
+      ph_next = ph_far;
+      rn_next = tile_runs(tile + step, ph_next);
+      ph_far = tile_hdr(tile + 2 * step);
+      if (kt >= kWsStages &&
+          !ws_wait(uempty0 + 8u * us, (uint32_t)(kt / kWsStages - 1) & 1u, lim, abort_v, a.err, tile))
         break;
       const bool planned = plan_takes(ph);
-      const int cnt = min(kTile, N - tile * kTile);
       int off = rn.y;  // inclusive prefix of the run lengths over the lanes
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
@@ -1359,45 +1384,40 @@ __global__ void __launch_bounds__(kWsT, 1)
         if (lane >= d) off += v;
       }
       off -= rn.y;
-      const uint32_t stg = smem_u32(sU + (size_t)us * kWsUStage);
-      const uint32_t fb = ufull0 + 8u * us;
+      const uint32_t stg = smem_u32(sOwn + (size_t)us * kWsStage);
+      const uint32_t fb = full0 + 8u * us;
       if (lane == 0) {
         // the gathers' generic reads of this stage are ordered before the copies' writes
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb),
-                     "r"(planned ? (uint32_t)ph.y * 128u + (uint32_t)cnt * 16u : 0u)
+                     "r"(planned ? (uint32_t)ph.y * 128u : 0u)
                      : "memory");
-        if (planned)
-          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                           stg + kWsSlots),
-                       "l"(a.plan.local + (size_t)tile * kTile), "r"((uint32_t)cnt * 16u), "r"(fb)
-                       : "memory");
       }
       __syncwarp();
       if (rn.y > 0)  // run j lands after the earlier runs
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                         stg + (uint32_t)off * 128u),
+                         stg + (uint32_t)kWsOwn + (uint32_t)off * 128u),
                      "l"(a.Hin + (size_t)rn.x * F), "r"((uint32_t)rn.y * 128u), "r"(fb)
                      : "memory");
     }
     // the copies issued land before the CTA leaves (bounded)
     if (lane == 0)
-      for (int j = max(0, kt - kWsUStages); j < kt; ++j)
-        mbar_wait(ufull0 + 8u * (j & 1), (uint32_t)(j >> 1) & 1u, kMbarSpinLimit);
+      for (int j = max(0, kt - kWsStages); j < kt; ++j)
+        mbar_wait(full0 + 8u * (j % kWsStages), (uint32_t)(j / kWsStages) & 1u, kMbarSpinLimit);
   } else if (lane == 0) {
     // ---- MMA: one thread
     const uint32_t b_addr = smem_u32(sB);
     int kt = 0;
-    for (int tile = blockIdx.x; tile * kTile < N; tile += gridDim.x, ++kt) {
-      const int os = kt % kWsOwnStages, hs = kt & 1;
-      const uint32_t opar = (uint32_t)(kt / kWsOwnStages) & 1u, hpar = (uint32_t)(kt >> 1) & 1u;
-      if (!ws_wait(mfull0 + 8u * hs, hpar, lim, abort_v, a.err, tile, false) ||
-          !ws_wait(ofull0 + 8u * os, opar, lim, abort_v, a.err, tile, false) ||
-          (kt >= 2 && !ws_wait(aempty0 + 8u * hs, hpar ^ 1u, lim, abort_v, a.err, tile, false)))
+    WsStage at;
+    for (int tile = blockIdx.x; tile * kTile < N; tile += gridDim.x, ++kt, at.next()) {
+      const uint32_t os = at.s, opar = at.phase, hs = kt & 1, hpar = (uint32_t)(kt >> 1) & 1u;
+      if (!ws_wait(full0 + 8u * os, opar, lim, abort_v, a.err, tile, false) ||
+          (kt >= 2 && !ws_wait(aempty0 + 8u * hs, hpar ^ 1u, lim, abort_v, a.err, tile, false)) ||
+          !ws_wait(mfull0 + 8u * os, opar, lim, abort_v, a.err, tile, false))
         break;
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       const uint32_t d = tmem + (uint32_t)(hs * F);
-      const uint32_t own = smem_u32(sOwn + (size_t)os * kWsOwn), mean = smem_u32(sMean + (size_t)hs * kTile * 128);
+      const uint32_t own = smem_u32(sOwn + (size_t)os * kWsStage), mean = own + kWsMean;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {  // K = 128 in slices of 16: four of the own rows, four of the means
         const uint64_t ad = umma_desc_sw128((j < 4 ? own : mean) + (uint32_t)(j & 3) * 32u, 1024u);
