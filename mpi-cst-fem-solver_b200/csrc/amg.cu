@@ -860,11 +860,9 @@ struct SweepCoef {
   double a0, beta, gamma, cd;
 };
 
-template <int MODE>
-__device__ __forceinline__ SweepCoef sweep_coef(const double* lam, int cheb) {
+__device__ SweepCoef sweep_coef_of(int mode, double l, int cheb) {
   SweepCoef c{0.0, 1.0, 0.0, 0.0};
-  if (MODE == kSweepResidual) return c;
-  const double l = *lam;
+  if (mode == kSweepResidual) return c;
   if (!cheb) {
     const double w = 4.0 / (3.0 * l);
     c.a0 = w;
@@ -874,17 +872,36 @@ __device__ __forceinline__ SweepCoef sweep_coef(const double* lam, int cheb) {
   const double hi = kChebHi * l, lo = hi / kChebRatio;
   const double theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo), sigma = theta / delta;
   const double rho1 = 1.0 / sigma, rho2 = 1.0 / (2.0 * sigma - rho1);
-  if (MODE == kSweepFirst) {
+  if (mode == kSweepFirst) {
     c.a0 = 1.0 / theta;
     c.beta = 1.0 + rho2 * rho1;
     c.gamma = 2.0 * rho2 / delta;
-  } else if (MODE == kSweepSmooth) {
+  } else if (mode == kSweepSmooth) {
     c.gamma = 1.0 / theta;
   } else {
     c.cd = rho2 * rho1;
     c.gamma = 2.0 * rho2 / delta;
   }
   return c;
+}
+
+// The coefficients of every step follow lambda_max in its buffer (kAmgLamDoubles), computed once per
+// setup: in the sweeps every thread spent five dependent FP64 divisions on them, more than on its node.
+__global__ void k_amg_sweep_coef(double* lam) {
+  const int t = threadIdx.x;  // 4 steps x (Jacobi, Chebyshev)
+  const SweepCoef c = sweep_coef_of(t & 3, lam[0], t >> 2);
+  double* o = lam + 1 + 4 * t;
+  o[0] = c.a0;
+  o[1] = c.beta;
+  o[2] = c.gamma;
+  o[3] = c.cd;
+}
+
+template <int MODE>
+__device__ __forceinline__ SweepCoef sweep_coef(const double* lam, int cheb) {
+  if (MODE == kSweepResidual) return SweepCoef{0.0, 1.0, 0.0, 0.0};
+  const double* o = lam + 1 + 4 * (MODE + (cheb ? 4 : 0));
+  return SweepCoef{__ldg(&o[0]), __ldg(&o[1]), __ldg(&o[2]), __ldg(&o[3])};
 }
 
 // the update of component i given its current value xi (and previous value xpi for kSweepSecond)
@@ -1177,12 +1194,33 @@ __global__ void k_amg_gemv(const int* skip, int n, const double* __restrict__ M,
 // cluster barriers (release/acquire at cluster scope; vectors written in a phase are read in the
 // next through L2). The same row functions and orders of addition as the per-level launches, so
 // the result is bit-identical to them; only the ~13 launch latencies of these small levels go.
+__device__ __forceinline__ void prefetch_l2(const void* p, size_t bytes, int tid, int nt) {
+  const char* c = static_cast<const char*>(p);
+  for (size_t o = (size_t)tid * 128; o < bytes; o += (size_t)nt * 128)
+    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(c + o));
+}
+
 __global__ void __launch_bounds__(kAmgTailThreads, 1) k_amg_tail(const int* skip, const __grid_constant__ AmgTail T) {
   if (skipped(skip)) return;  // (uniform over the cluster: every CTA leaves before any barrier)
   const cg::cluster_group cl = cg::this_cluster();
   const int tid = (int)cl.block_rank() * blockDim.x + threadIdx.x;
   const int nt = (int)cl.num_blocks() * blockDim.x;
   const int lane = threadIdx.x & 31, warp = tid >> 5, nw = nt >> 5;
+  // the rest of the cycle has pushed the levels' operators out of L2: their DRAM latencies all at once
+  for (int l = 0; l + 1 < T.nl; ++l) {
+    const AmgTailLevel& v = T.L[l];
+    prefetch_l2(v.A.ptr, sizeof(int) * (size_t)(v.A.n + 1), tid, nt);
+    prefetch_l2(v.A.col, sizeof(int) * (size_t)v.A.nnzb, tid, nt);
+    prefetch_l2(v.A.val, sizeof(float) * 9 * (size_t)v.A.nnzb, tid, nt);
+    prefetch_l2(v.dinv, sizeof(double) * 3 * (size_t)v.A.n, tid, nt);
+    prefetch_l2(v.pt_ptr, sizeof(int) * (size_t)(v.nc + 1), tid, nt);
+    prefetch_l2(v.p_ptr, sizeof(int) * (size_t)(v.A.n + 1), tid, nt);
+    prefetch_l2(v.pt_row, sizeof(int) * (size_t)v.nnz_p, tid, nt);
+    prefetch_l2(v.p_col, sizeof(int) * (size_t)v.nnz_p, tid, nt);
+    prefetch_l2(v.pt32, sizeof(float) * 9 * (size_t)v.nnz_p, tid, nt);
+    prefetch_l2(v.p32, sizeof(float) * 9 * (size_t)v.nnz_p, tid, nt);
+  }
+  prefetch_l2(T.Minv, sizeof(double) * (size_t)T.n_coarse * T.n_coarse, tid, nt);
   for (int l = 0; l + 1 < T.nl; ++l) {
     const AmgTailLevel& v = T.L[l];
     sweep3_rows<kSweepFirst, true>(v.A, v.dinv, sweep_coef<kSweepFirst>(v.lam, T.cheb), v.b, nullptr, nullptr, v.x,
@@ -1492,7 +1530,8 @@ cudaError_t amg_lambda_f32(const MixedMatrix* fine, const AmgBsr32* coarse, cons
     k_amg_norm<<<1, kThreads, 0, s>>>(part, kLamGrid, lam, sc);
     std::swap(x, y);
   }
-  count_launches(1 + 2LL * iters);
+  k_amg_sweep_coef<<<1, 8, 0, s>>>(lam);
+  count_launches(2 + 2LL * iters);
   return cudaGetLastError();
 }
 

@@ -126,7 +126,7 @@ int scan_total(cstg_ctx* ctx, const int* in, int n, int* out, int* total) {
 int level_lambda(cstg_ctx* ctx, AmgData* d, int l) {
   AmgLevel& lv = d->L[l];
   const size_t m = (size_t)lv.n * lv.B;
-  ENSURE(lv.lam, sizeof(double));
+  ENSURE(lv.lam, sizeof(double) * kAmgLamDoubles);
   ENSURE(d->part, amg_lambda_scratch());
   ENSURE(d->vx, sizeof(double) * m);
   ENSURE(d->vy, sizeof(double) * m);
@@ -322,6 +322,7 @@ int setup_tail(cstg_ctx* ctx, AmgData* d) {
     v.xa = buf_ptr<double>(lv.xa);
     v.r = buf_ptr<double>(lv.r);
     v.nc = lv.nc;
+    v.nnz_p = lv.nnz_p;
     v.pt_ptr = buf_ptr<int>(lv.pt_ptr);
     v.pt_row = buf_ptr<int>(lv.pt_row);
     v.pt32 = buf_ptr<float>(lv.pt32);

@@ -365,6 +365,7 @@ cudaError_t amg_coarsest(int B, const AmgBsr& A, double* M, double* piv, cudaStr
 // smoother steps (amg.cu): x + gamma D^-1 (b - A x); b - A x; the two steps from x = 0 in one
 // launch (x not read); the second Chebyshev step (reads the previous iterate xp). cheb: Chebyshev
 // coefficients (else damped Jacobi), computed in the kernel from lambda_max.
+constexpr int kAmgLamDoubles = 1 + 2 * 4 * 4;  // lambda_max, then the coefficients of the steps
 constexpr int kSweepSmooth = 0, kSweepResidual = 1, kSweepFirst = 2, kSweepSecond = 3;
 void amg_prepare_launch_shapes();  // occupancy queries of the one-wave launches (call outside a capture)
 // skip (all cycle launchers): a device flag; non-zero makes the launch return at once (may be null)
@@ -404,6 +405,7 @@ struct AmgTailLevel {
   double* xa = nullptr;  // sweep scratch
   double* r = nullptr;   // residual
   int nc = 0;            // transfer to the next level
+  int nnz_p = 0;
   const int* pt_ptr = nullptr;
   const int* pt_row = nullptr;
   const float* pt32 = nullptr;
