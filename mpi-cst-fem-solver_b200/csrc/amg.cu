@@ -73,20 +73,16 @@ __device__ __forceinline__ int row_find(const int* cols, int lo, int hi, int v) 
 
 // ---- fine-level conversion: the node-run layout -> BSR 2x2 --------------------------------------
 
+// Eight lanes per node, 16 bytes each, so that reads and writes are runs (a thread per node: 122 us for
+// 1,003,302 DOFs; 39 so).
 __global__ void k_amg_bsr2(int N, const int* __restrict__ node_ptr, const double* __restrict__ vals,
                            double* __restrict__ out) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3);
   if (n >= N) return;
   const int b0 = node_ptr[n], deg = node_ptr[n + 1] - b0;
-  const double* ra = vals + 4L * b0;
-  const double* rb = ra + 2 * deg;
-  for (int k = 0; k < deg; ++k) {
-    double* o = out + 4L * (b0 + k);
-    o[0] = ra[2 * k];
-    o[1] = ra[2 * k + 1];
-    o[2] = rb[2 * k];
-    o[3] = rb[2 * k + 1];
-  }
+  const double2* in = reinterpret_cast<const double2*>(vals) + 2 * (size_t)b0;
+  double2* o = reinterpret_cast<double2*>(out) + 2 * (size_t)b0;
+  for (int u = threadIdx.x & 7; u < 2 * deg; u += 8) o[u] = in[(u & 1) * deg + (u >> 1)];
 }
 
 template <int B>
@@ -280,70 +276,97 @@ __global__ void k_sort_segments(int m, const int* __restrict__ ptr, int* __restr
 
 // ---- tentative prolongator: per aggregate, QR (modified Gram-Schmidt) of the stacked B x 3 blocks ----
 
+// Eight lanes per aggregate, its stacked blocks in shared memory: the lanes take the rows' updates, and
+// each lane runs the sums over the rows (in order) for itself. A chain of dependent FP64 operations per
+// aggregate bounds it (a thread per aggregate in global memory: 306 us for 48,233 aggregates of ten
+// nodes; the coarse levels, with few aggregates, 80 to 95 us; 74 and 18 so).
+constexpr int kTentLanes = 8, kTentWarps = 2;
+
 template <int B>
-__global__ void k_amg_tentative(int n_agg, const int* __restrict__ agg_ptr, const int* __restrict__ members,
-                                const double* __restrict__ Bf, double* __restrict__ P0, double* __restrict__ Bc,
-                                int* err) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= n_agg) return;
+__global__ void __launch_bounds__(32 * kTentWarps) k_amg_tentative(int n_agg, const int* __restrict__ agg_ptr,
+                                                                   const int* __restrict__ members,
+                                                                   const double* __restrict__ Bf,
+                                                                   double* __restrict__ P0, double* __restrict__ Bc,
+                                                                   int* err) {
+  constexpr int kGroups = 32 * kTentWarps / kTentLanes;
+  __shared__ double sm[kGroups][kAmgMaxAgg * B * 3];  // Q in place: row r of the stacked matrix at 3 r
+  const int g = threadIdx.x / kTentLanes, l = threadIdx.x % kTentLanes;
+  const unsigned mask = 0xffu << ((threadIdx.x & 31) / kTentLanes * kTentLanes);
+  const int a = blockIdx.x * kGroups + g;
+  if (a >= n_agg) return;  // (uniform over a group; groups synchronise alone)
   const int lo = agg_ptr[a], hi = agg_ptr[a + 1], m = hi - lo;
   if (m > kAmgMaxAgg) {
-    atomicMin(&err[kErrAmg], a);
+    if (l == 0) atomicMin(&err[kErrAmg], a);
     return;
   }
   const int rows = m * B;
-  double R[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  // Q is written in place into P0 (node-major B x 3 blocks): column c of the stacked matrix
-  // lives at P0[node * B*3 + r * 3 + c]
-  for (int q = 0; q < m; ++q) {
-    const int node = members[lo + q];
-    for (int k = 0; k < B * 3; ++k) P0[(size_t)node * B * 3 + k] = Bf[(size_t)node * B * 3 + k];
-  }
-  auto at = [&](int row, int c) -> double& {
-    const int node = members[lo + row / B];
-    return P0[(size_t)node * B * 3 + (row % B) * 3 + c];
-  };
+  double* q = sm[g];
   double scale = 0.0;
-  for (int r = 0; r < rows; ++r)
-    for (int c = 0; c < 3; ++c) scale = fmax(scale, fabs(at(r, c)));
+  for (int e = l; e < rows * 3; e += kTentLanes) {
+    const double v = Bf[(size_t)members[lo + e / (B * 3)] * B * 3 + e % (B * 3)];
+    q[e] = v;
+    scale = fmax(scale, fabs(v));
+  }
+#pragma unroll
+  for (int o = kTentLanes / 2; o > 0; o >>= 1) scale = fmax(scale, __shfl_xor_sync(mask, scale, o));
+  __syncwarp(mask);
+  double R[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
   for (int c = 0; c < 3; ++c) {
+#pragma unroll
     for (int p = 0; p < c; ++p) {
       double d = 0.0;
-      for (int r = 0; r < rows; ++r) d += at(r, p) * at(r, c);
+      for (int r = 0; r < rows; ++r) d = fma(q[3 * r + p], q[3 * r + c], d);
       R[p * 3 + c] = d;
-      for (int r = 0; r < rows; ++r) at(r, c) -= d * at(r, p);
+      __syncwarp(mask);
+      for (int r = l; r < rows; r += kTentLanes) q[3 * r + c] = fma(-d, q[3 * r + p], q[3 * r + c]);
+      __syncwarp(mask);
     }
     double nrm = 0.0;
-    for (int r = 0; r < rows; ++r) nrm += at(r, c) * at(r, c);
+    for (int r = 0; r < rows; ++r) nrm = fma(q[3 * r + c], q[3 * r + c], nrm);
     nrm = sqrt(nrm);
-    if (nrm <= 1e-10 * (scale > 0.0 ? scale : 1.0)) {  // dependent column (tiny aggregate): drop it
-      R[c * 3 + c] = 0.0;
-      for (int r = 0; r < rows; ++r) at(r, c) = 0.0;
-    } else {
-      R[c * 3 + c] = nrm;
-      for (int r = 0; r < rows; ++r) at(r, c) /= nrm;
-    }
+    const bool drop = nrm <= 1e-10 * (scale > 0.0 ? scale : 1.0);  // dependent column (tiny aggregate)
+    R[c * 3 + c] = drop ? 0.0 : nrm;
+    __syncwarp(mask);
+    for (int r = l; r < rows; r += kTentLanes) q[3 * r + c] = drop ? 0.0 : q[3 * r + c] / nrm;
+    __syncwarp(mask);
   }
-  for (int k = 0; k < 9; ++k) Bc[(size_t)a * 9 + k] = R[k];
+  for (int e = l; e < rows * 3; e += kTentLanes)
+    P0[(size_t)members[lo + e / (B * 3)] * B * 3 + e % (B * 3)] = q[e];
+  for (int k = l; k < 9; k += kTentLanes) {
+    double v = R[0];
+#pragma unroll
+    for (int u = 1; u < 9; ++u) v = k == u ? R[u] : v;
+    Bc[(size_t)a * 9 + k] = v;
+  }
 }
 
 // ---- lambda_max(D^-1 A) by power iteration ----------------------------------------------------------
 // Each step y = s D^-1 A x with s = 1 / ||x|| from the previous step (1 on the first) writes
 // per-block partial sums of ||y||^2 on a fixed grid (k_amg_dinva_fine / _coarse, after the cycle
-// kernels); k_amg_norm adds the partials in block order.
+// kernels); the last block by ticket adds them in block order (a launch of its own took 3 us a step).
 constexpr int kLamGrid = 148 * 8;
 
-// lam = sqrt(sum of the partials, in block order), sc = 1 / lam (one block)
-__global__ void __launch_bounds__(kThreads) k_amg_norm(const double* __restrict__ part, int nparts, double* lam,
-                                                       double* sc) {
-  double s = 0.0;
-  for (int b = threadIdx.x; b < nparts; b += blockDim.x) s += part[b];
-  __shared__ double sm[kWarps];
-  const double t = block_sum<kThreads>(s, sm);
+// t: the block's sum (thread 0). The last block: lam = sqrt(sum of the partials), sc = 1 / lam.
+__device__ __forceinline__ void amg_norm_epilogue(double t, double* part, double* lam, double* sc, unsigned* ticket,
+                                                  double* sm) {
+  __shared__ bool am_last;
   if (threadIdx.x == 0) {
-    const double nrm = sqrt(t);
+    part[blockIdx.x] = t;
+    __threadfence();
+    am_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!am_last) return;
+  __threadfence();
+  double s = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) s += __ldcg(&part[b]);
+  const double sum = block_sum<kThreads>(s, sm);
+  if (threadIdx.x == 0) {
+    const double nrm = sqrt(sum);
     *lam = nrm;
     *sc = nrm > 0.0 ? 1.0 / nrm : 0.0;
+    *ticket = 0u;
   }
 }
 
@@ -403,64 +426,18 @@ __global__ void k_amg_ap_count(int n, AmgBsr A, AmgBsr P, int* __restrict__ cnt,
   cnt[i] = m;
 }
 
-// The fill of a Galerkin factor runs in two kernels: a thread per row writes the row's sorted
-// column set (as the count kernel found it), then a warp per row sums the row's block products.
-// The warp takes the row's candidate products (one per pair of input blocks) 32 at a time in
-// their fixed order, each lane computes one product into shared memory, and each lane then adds,
-// in candidate order, the products that fall on the two output blocks it owns (lane, lane + 32).
-// Every output block thus sees the same additions in the same order on every run.
+// The fill of a Galerkin factor runs in two kernels: one writes the rows' sorted column sets (as the
+// count kernel found them), then G lanes per row sum the row's block products. Each lane owns the output
+// blocks lane, lane + G, ... (a pass per G blocks) and goes through the row's candidate products (one per
+// pair of input blocks) in their fixed order, computing those that fall on its block: every output block
+// sees the same additions in the same order on every run, and nothing goes through shared memory (a warp
+// per row that left the products there for their owners took 719 us for AP, 561 for P and 317 for A_c of
+// 1,003,302 DOFs, most lanes idle in the additions; these take 204, 100 and 197). Latency of the chain of
+// indices bounds them; G fits the rows' usual number of output blocks.
 constexpr int kGalWarps = 8;
 
-template <int NV>
-struct GalerkinSmem {
-  int cols[kGalWarps][kAmgMaxRow];
-  int ofs[kGalWarps][33];
-  int slot[kGalWarps][32];
-  double prod[kGalWarps][32][NV];
-};
-
-// owner-lane accumulation of one chunk of `cnt` candidate products
-template <int NV>
-__device__ __forceinline__ void gal_accumulate(const int* slot, const double (*prod)[NV], int cnt, int lane,
-                                               double (&a0)[NV], double (&a1)[NV]) {
-  for (int u = 0; u < cnt; ++u) {
-    const int su = slot[u];
-    if (su == lane) {
-#pragma unroll
-      for (int v = 0; v < NV; ++v) a0[v] += prod[u][v];
-    } else if (su == lane + 32) {
-#pragma unroll
-      for (int v = 0; v < NV; ++v) a1[v] += prod[u][v];
-    }
-  }
-}
-
-// inclusive warp scan of `len` into ofs[1..32] (ofs[0] = 0); returns the total
-__device__ __forceinline__ int gal_offsets(int len, int lane, int* ofs) {
-  int incl = len;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  ofs[lane + 1] = incl;
-  if (lane == 0) ofs[0] = 0;
-  __syncwarp();
-  return __shfl_sync(0xffffffffu, incl, 31);
-}
-
-// the group member g (0..ng-1) whose candidate range [ofs[g], ofs[g+1]) holds t
-__device__ __forceinline__ int gal_member(const int* ofs, int ng, int t) {
-  int lo = 0, hi = ng - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (ofs[mid] <= t)
-      lo = mid;
-    else
-      hi = mid - 1;
-  }
-  return lo;
-}
+// The largest value over the warp.
+__device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(0xffffffffu, v); }
 
 // Prolongator smoothing weight w = kProlongOmega / lambda_max(D^-1 A). 1.6 rather than the usual
 // 4/3: on the plates it gives 3-4 % fewer cycle iterations and slightly smaller coarse levels.
@@ -469,65 +446,59 @@ constexpr double kProlongOmega = 1.6;
 // P = P0 - w D^-1 A P0: values, warp per row i. Candidates: the blocks k of A's row i in order,
 // each the B x 3 product -w D_i^-1 A_k P0_{A.col[k]}; then P0_i is added to the node's own
 // aggregate's block.
-template <int B>
+template <int B, int G>
 __global__ void __launch_bounds__(32 * kGalWarps) k_amg_p_vals(int n, AmgBsr A, const int* __restrict__ agg,
                                                                const double* __restrict__ P0,
                                                                const double* __restrict__ dinv,
                                                                const double* __restrict__ wp, AmgBsr P) {
-  constexpr int NV = B * 3;
-  __shared__ GalerkinSmem<NV> sm;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int warp = blockIdx.x * kGalWarps + w, nw = gridDim.x * kGalWarps;
+  constexpr int NV = B * 3, R = 32 / G;
+  const int lane = threadIdx.x & 31, gl = lane % G;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
   const double om = kProlongOmega / *wp;
-  for (int i = warp; i < n; i += nw) {
-    const int c0 = P.ptr[i], m = P.ptr[i + 1] - c0;
-    for (int t = lane; t < m; t += 32) sm.cols[w][t] = P.col[c0 + t];
-    __syncwarp();
+  for (int base = warp * R; base < n; base += nw * R) {
+    const int i = base + lane / G;
+    const bool on = i < n;
+    const int c0 = on ? P.ptr[i] : 0, m = on ? P.ptr[i + 1] - c0 : 0;
+    const int k0 = on ? A.ptr[i] : 0, k1 = on ? A.ptr[i + 1] : 0;
+    const int own = on ? agg[i] : -1;
     double f[B];
 #pragma unroll
-    for (int r = 0; r < B; ++r) f[r] = -om * dinv[(size_t)i * B + r];
-    double a0[NV], a1[NV];
+    for (int r = 0; r < B; ++r) f[r] = on ? -om * dinv[(size_t)i * B + r] : 0.0;
+    const int passes = warp_max(m), span = warp_max(k1 - k0);
+    for (int p = 0; p < passes; p += G) {
+      const int mine = p + gl < m ? P.col[c0 + p + gl] : -1;
+      double acc[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) a0[v] = a1[v] = 0.0;
-    const int k0 = A.ptr[i], k1 = A.ptr[i + 1];
-    for (int kb = k0; kb < k1; kb += 32) {
-      const int k = kb + lane;
-      if (k < k1) {
-        const int j = A.col[k];
-        const double* blk = A.val + (size_t)k * B * B;
-        const double* p0 = P0 + (size_t)j * B * 3;
+      for (int v = 0; v < NV; ++v) acc[v] = 0.0;
+      for (int kb = 0; kb < span; kb += G) {
+        int j = 0, to = -2;  // the candidates' nodes and aggregates, one per lane
+        if (k0 + kb + gl < k1) {
+          j = A.col[k0 + kb + gl];
+          to = agg[j];
+        }
+        const int us = min(G, span - kb);
+        for (int u = 0; u < us; ++u) {
+          const int ju = __shfl_sync(0xffffffffu, j, u, G);
+          if (__shfl_sync(0xffffffffu, to, u, G) != mine) continue;
+          const double* blk = A.val + (size_t)(k0 + kb + u) * B * B;
+          const double* p0 = P0 + (size_t)ju * NV;
 #pragma unroll
-        for (int r = 0; r < B; ++r)
+          for (int r = 0; r < B; ++r)
 #pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            double t = 0.0;
+            for (int c = 0; c < 3; ++c) {
+              double t = 0.0;
 #pragma unroll
-            for (int q = 0; q < B; ++q) t = fma(blk[r * B + q], p0[q * 3 + c], t);
-            sm.prod[w][lane][r * 3 + c] = f[r] * t;
-          }
-        sm.slot[w][lane] = row_find(sm.cols[w], 0, m, agg[j]);
+              for (int q = 0; q < B; ++q) t = fma(blk[r * B + q], p0[q * 3 + c], t);
+              acc[r * 3 + c] = __dadd_rn(acc[r * 3 + c], __dmul_rn(f[r], t));
+            }
+        }
       }
-      __syncwarp();
-      gal_accumulate<NV>(sm.slot[w], sm.prod[w], min(32, k1 - kb), lane, a0, a1);
-      __syncwarp();
+      if (p + gl < m) {
+        double* out = const_cast<double*>(P.val) + (size_t)(c0 + p + gl) * NV;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) out[v] = own == mine ? acc[v] + P0[(size_t)i * NV + v] : acc[v];
+      }
     }
-    const int own = row_find(sm.cols[w], 0, m, agg[i]);
-    const double* p0i = P0 + (size_t)i * B * 3;
-    if (own == lane) {
-#pragma unroll
-      for (int v = 0; v < NV; ++v) a0[v] += p0i[v];
-    } else if (own == lane + 32) {
-#pragma unroll
-      for (int v = 0; v < NV; ++v) a1[v] += p0i[v];
-    }
-    double* out = const_cast<double*>(P.val) + (size_t)c0 * NV;
-    if (lane < m)
-#pragma unroll
-      for (int v = 0; v < NV; ++v) out[(size_t)lane * NV + v] = a0[v];
-    if (lane + 32 < m)
-#pragma unroll
-      for (int v = 0; v < NV; ++v) out[(size_t)(lane + 32) * NV + v] = a1[v];
-    __syncwarp();
   }
 }
 
@@ -546,68 +517,70 @@ __global__ void k_amg_ap_cols(int n, AmgBsr A, AmgBsr P, AmgBsr AP) {
   for (int q = 0; q < m; ++q) cols[q] = s[q];
 }
 
+// The block of a sorted row (columns col[beg .. beg + len)) whose column is `mine`, or -1: the lanes of a
+// group share the row and load its columns together.
+template <int G>
+__device__ __forceinline__ int gal_hit(const int* __restrict__ col, int beg, int len, int mine, int gl) {
+  int hit = -1;
+  const int most = warp_max(len);
+  for (int x0 = 0; x0 < most; x0 += G) {
+    const int c = x0 + gl < len ? col[beg + x0 + gl] : -2;
+    const int xs = min(G, most - x0);
+    for (int x = 0; x < xs; ++x)
+      if (__shfl_sync(0xffffffffu, c, x, G) == mine) hit = beg + x0 + x;
+  }
+  return hit;
+}
+
 // AP = A P: values. Row i's candidates: for each block k of A's row i (ascending), for each block
 // q of P's row A.col[k] (ascending), the B x 3 product A_k P_q.
-template <int B>
+template <int B, int G>
 __global__ void __launch_bounds__(32 * kGalWarps) k_amg_ap_vals(int n, AmgBsr A, AmgBsr P, AmgBsr AP) {
-  constexpr int NV = B * 3;
-  __shared__ GalerkinSmem<NV> sm;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int warp = blockIdx.x * kGalWarps + w, nw = gridDim.x * kGalWarps;
-  for (int i = warp; i < n; i += nw) {
-    const int c0 = AP.ptr[i], m = AP.ptr[i + 1] - c0;
-    for (int t = lane; t < m; t += 32) sm.cols[w][t] = AP.col[c0 + t];
-    double a0[NV], a1[NV];
+  constexpr int NV = B * 3, R = 32 / G;
+  const int lane = threadIdx.x & 31, gl = lane % G;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  for (int base = warp * R; base < n; base += nw * R) {
+    const int i = base + lane / G;
+    const bool on = i < n;
+    const int c0 = on ? AP.ptr[i] : 0, m = on ? AP.ptr[i + 1] - c0 : 0;
+    const int k0 = on ? A.ptr[i] : 0, k1 = on ? A.ptr[i + 1] : 0;
+    const int passes = warp_max(m), span = warp_max(k1 - k0);
+    for (int p = 0; p < passes; p += G) {
+      const int mine = p + gl < m ? AP.col[c0 + p + gl] : -1;
+      double acc[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) a0[v] = a1[v] = 0.0;
-    const int k0 = A.ptr[i], k1 = A.ptr[i + 1];
-    for (int kb = k0; kb < k1; kb += 32) {
-      const int ng = min(32, k1 - kb);
-      int pbeg = 0, len = 0;
-      if (lane < ng) {
-        const int j = A.col[kb + lane];
-        pbeg = P.ptr[j];
-        len = P.ptr[j + 1] - pbeg;
-      }
-      const int total = gal_offsets(len, lane, sm.ofs[w]);
-      for (int cb = 0; cb < total; cb += 32) {
-        const int t = cb + lane;
-        const int g = gal_member(sm.ofs[w], ng, min(t, total - 1));
-        const int qb = __shfl_sync(0xffffffffu, pbeg, g);
-        if (t < total) {
-          const int k = kb + g, q = qb + (t - sm.ofs[w][g]);
-          const double* blk = A.val + (size_t)k * B * B;
-          const double* pb = P.val + (size_t)q * B * 3;
-          double a[B * B], p[B * 3];
-#pragma unroll
-          for (int v = 0; v < B * B; ++v) a[v] = blk[v];
-#pragma unroll
-          for (int v = 0; v < B * 3; ++v) p[v] = pb[v];
+      for (int v = 0; v < NV; ++v) acc[v] = 0.0;
+      for (int kb = 0; kb < span; kb += G) {
+        int pbeg = 0, len = 0;
+        if (k0 + kb + gl < k1) {
+          const int j = A.col[k0 + kb + gl];
+          pbeg = P.ptr[j];
+          len = P.ptr[j + 1] - pbeg;
+        }
+        const int us = min(G, span - kb);
+        for (int u = 0; u < us; ++u) {
+          const int hit = gal_hit<G>(P.col, __shfl_sync(0xffffffffu, pbeg, u, G), __shfl_sync(0xffffffffu, len, u, G),
+                                     mine, gl);
+          if (hit < 0) continue;
+          const double* a = A.val + (size_t)(k0 + kb + u) * B * B;
+          const double* pb = P.val + (size_t)hit * NV;
 #pragma unroll
           for (int r = 0; r < B; ++r)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
               double x = 0.0;
 #pragma unroll
-              for (int z = 0; z < B; ++z) x = fma(a[r * B + z], p[z * 3 + c], x);
-              sm.prod[w][lane][r * 3 + c] = x;
+              for (int z = 0; z < B; ++z) x = fma(a[r * B + z], pb[z * 3 + c], x);
+              acc[r * 3 + c] = __dadd_rn(acc[r * 3 + c], x);
             }
-          sm.slot[w][lane] = row_find(sm.cols[w], 0, m, P.col[q]);
         }
-        __syncwarp();
-        gal_accumulate<NV>(sm.slot[w], sm.prod[w], min(32, total - cb), lane, a0, a1);
-        __syncwarp();
       }
-      __syncwarp();
+      if (p + gl < m) {
+        double* out = const_cast<double*>(AP.val) + (size_t)(c0 + p + gl) * NV;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) out[v] = acc[v];
+      }
     }
-    double* out = const_cast<double*>(AP.val) + (size_t)c0 * NV;
-    if (lane < m)
-#pragma unroll
-      for (int v = 0; v < NV; ++v) out[(size_t)lane * NV + v] = a0[v];
-    if (lane + 32 < m)
-#pragma unroll
-      for (int v = 0; v < NV; ++v) out[(size_t)(lane + 32) * NV + v] = a1[v];
-    __syncwarp();
   }
 }
 
@@ -647,7 +620,8 @@ __device__ __forceinline__ unsigned ac_slot(int c) {
 template <bool FILL>
 __global__ void __launch_bounds__(32 * kAcWarps) k_amg_ac_pattern(int nc, const int* __restrict__ pt_ptr,
                                                                   const int* __restrict__ pt_idx,
-                                                                  const int* __restrict__ p_row, AmgBsr AP,
+                                                                  const int* __restrict__ p_row /* null: rows pt_idx */,
+                                                                  AmgBsr AP,
                                                                   int* __restrict__ cnt, AmgBsr Ac, int* err) {
   __shared__ int set[kAcWarps][kAcSet];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -657,7 +631,7 @@ __global__ void __launch_bounds__(32 * kAcWarps) k_amg_ac_pattern(int nc, const 
     int full = 0;
     const int t1 = pt_ptr[J + 1];
     for (int t = pt_ptr[J] + lane; t < t1; t += 32) {
-      const int i = p_row[pt_idx[t]];
+      const int i = p_row ? p_row[pt_idx[t]] : pt_idx[t];
       for (int q = AP.ptr[i]; q < AP.ptr[i + 1]; ++q) {
         const int c = AP.col[q];
         unsigned h = ac_slot(c);
@@ -671,14 +645,16 @@ __global__ void __launch_bounds__(32 * kAcWarps) k_amg_ac_pattern(int nc, const 
       }
     }
     __syncwarp();
-    int v[kAcSet / 32];
+    // the distinct columns, packed to the front of the set
+    int v[kAcSet / 32], at[kAcSet / 32];
     int m = 0;
 #pragma unroll
     for (int u = 0; u < kAcSet / 32; ++u) {
       v[u] = set[w][lane + 32 * u];
-      m += v[u] >= 0 ? 1 : 0;
+      const unsigned on = __ballot_sync(0xffffffffu, v[u] >= 0);
+      at[u] = m + __popc(on & ((1u << lane) - 1u));
+      m += __popc(on);
     }
-    m = __reduce_add_sync(0xffffffffu, m);
     full = __any_sync(0xffffffffu, full);
     if (!FILL) {
       if (lane == 0) {
@@ -686,16 +662,16 @@ __global__ void __launch_bounds__(32 * kAcWarps) k_amg_ac_pattern(int nc, const 
         cnt[J] = m;
       }
     } else {
-      int* cols = const_cast<int*>(Ac.col) + Ac.ptr[J];
 #pragma unroll
-      for (int u = 0; u < kAcSet / 32; ++u) {
-        if (v[u] < 0) continue;
+      for (int u = 0; u < kAcSet / 32; ++u)
+        if (v[u] >= 0) set[w][at[u]] = v[u];
+      __syncwarp();
+      int* cols = const_cast<int*>(Ac.col) + Ac.ptr[J];
+      for (int e = lane; e < m; e += 32) {  // each at its rank among them
+        const int c = set[w][e];
         int r = 0;
-        for (int h = 0; h < kAcSet; ++h) {
-          const int o = set[w][h];
-          r += (o >= 0 && o < v[u]) ? 1 : 0;
-        }
-        cols[r] = v[u];
+        for (int h = 0; h < m; ++h) r += set[w][h] < c ? 1 : 0;
+        cols[r] = c;
       }
     }
     __syncwarp();
@@ -704,72 +680,58 @@ __global__ void __launch_bounds__(32 * kAcWarps) k_amg_ac_pattern(int nc, const 
 
 // A_c = P' (AP): values. Coarse row J's candidates: for each P block (i, J) in ascending fine row
 // i, for each block q of AP's row i (ascending), the 3 x 3 product P_iJ' (AP)_q.
-template <int B>
+template <int B, int G>
 __global__ void __launch_bounds__(32 * kGalWarps) k_amg_ac_vals(int nc, const int* __restrict__ pt_ptr,
                                                                 const int* __restrict__ pt_idx,
                                                                 const int* __restrict__ p_row, AmgBsr P, AmgBsr AP,
                                                                 AmgBsr Ac) {
-  constexpr int NV = 9;
-  __shared__ GalerkinSmem<NV> sm;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int warp = blockIdx.x * kGalWarps + w, nw = gridDim.x * kGalWarps;
-  for (int J = warp; J < nc; J += nw) {
-    const int c0 = Ac.ptr[J], m = Ac.ptr[J + 1] - c0;
-    for (int t = lane; t < m; t += 32) sm.cols[w][t] = Ac.col[c0 + t];
-    double a0[NV], a1[NV];
+  constexpr int NV = B * 3, R = 32 / G;
+  const int lane = threadIdx.x & 31, gl = lane % G;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  for (int base = warp * R; base < nc; base += nw * R) {
+    const int J = base + lane / G;
+    const bool on = J < nc;
+    const int c0 = on ? Ac.ptr[J] : 0, m = on ? Ac.ptr[J + 1] - c0 : 0;
+    const int t0 = on ? pt_ptr[J] : 0, t1 = on ? pt_ptr[J + 1] : 0;
+    const int passes = warp_max(m), span = warp_max(t1 - t0);
+    for (int p = 0; p < passes; p += G) {
+      const int mine = p + gl < m ? Ac.col[c0 + p + gl] : -1;
+      double acc[9];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) a0[v] = a1[v] = 0.0;
-    const int t0 = pt_ptr[J], t1 = pt_ptr[J + 1];
-    for (int tb = t0; tb < t1; tb += 32) {
-      const int ng = min(32, t1 - tb);
-      int pq = 0, abeg = 0, len = 0;
-      if (lane < ng) {
-        pq = pt_idx[tb + lane];
-        const int i = p_row[pq];
-        abeg = AP.ptr[i];
-        len = AP.ptr[i + 1] - abeg;
-      }
-      const int total = gal_offsets(len, lane, sm.ofs[w]);
-      for (int cb = 0; cb < total; cb += 32) {
-        const int t = cb + lane;
-        const int g = gal_member(sm.ofs[w], ng, min(t, total - 1));
-        const int qb = __shfl_sync(0xffffffffu, abeg, g);
-        const int pqg = __shfl_sync(0xffffffffu, pq, g);
-        if (t < total) {
-          const int q = qb + (t - sm.ofs[w][g]);
-          const double* pb = P.val + (size_t)pqg * B * 3;  // P_iJ (B x 3)
-          const double* ab = AP.val + (size_t)q * B * 3;   // (AP)_iK (B x 3)
-          double p[B * 3], a[B * 3];
-#pragma unroll
-          for (int v = 0; v < B * 3; ++v) {
-            p[v] = pb[v];
-            a[v] = ab[v];
-          }
+      for (int v = 0; v < 9; ++v) acc[v] = 0.0;
+      for (int tb = 0; tb < span; tb += G) {
+        int pq = 0, abeg = 0, len = 0;
+        if (t0 + tb + gl < t1) {
+          pq = pt_idx[t0 + tb + gl];
+          const int i = p_row[pq];
+          abeg = AP.ptr[i];
+          len = AP.ptr[i + 1] - abeg;
+        }
+        const int us = min(G, span - tb);
+        for (int u = 0; u < us; ++u) {
+          const int pu = __shfl_sync(0xffffffffu, pq, u, G);
+          const int hit = gal_hit<G>(AP.col, __shfl_sync(0xffffffffu, abeg, u, G),
+                                     __shfl_sync(0xffffffffu, len, u, G), mine, gl);
+          if (hit < 0) continue;
+          const double* pb = P.val + (size_t)pu * NV;    // P_iJ (B x 3)
+          const double* ab = AP.val + (size_t)hit * NV;  // (AP)_iK (B x 3)
 #pragma unroll
           for (int r = 0; r < 3; ++r)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
               double x = 0.0;
 #pragma unroll
-              for (int z = 0; z < B; ++z) x = fma(p[z * 3 + r], a[z * 3 + c], x);
-              sm.prod[w][lane][r * 3 + c] = x;
+              for (int z = 0; z < B; ++z) x = fma(pb[z * 3 + r], ab[z * 3 + c], x);
+              acc[r * 3 + c] = __dadd_rn(acc[r * 3 + c], x);
             }
-          sm.slot[w][lane] = row_find(sm.cols[w], 0, m, AP.col[q]);
         }
-        __syncwarp();
-        gal_accumulate<NV>(sm.slot[w], sm.prod[w], min(32, total - cb), lane, a0, a1);
-        __syncwarp();
       }
-      __syncwarp();
+      if (p + gl < m) {
+        double* out = const_cast<double*>(Ac.val) + (size_t)(c0 + p + gl) * 9;
+#pragma unroll
+        for (int v = 0; v < 9; ++v) out[v] = acc[v];
+      }
     }
-    double* out = const_cast<double*>(Ac.val) + (size_t)c0 * NV;
-    if (lane < m)
-#pragma unroll
-      for (int v = 0; v < NV; ++v) out[(size_t)lane * NV + v] = a0[v];
-    if (lane + 32 < m)
-#pragma unroll
-      for (int v = 0; v < NV; ++v) out[(size_t)(lane + 32) * NV + v] = a1[v];
-    __syncwarp();
   }
 }
 
@@ -835,6 +797,58 @@ __global__ void __launch_bounds__(1024) k_amg_gauss_jordan(int n, double* __rest
         M[(size_t)i * n + j] -= f * M[(size_t)k * n + j];
     }
   }
+}
+
+// The same for n <= 128, the matrix in the threads' registers (16 entries each, rows ti + 32 a, columns
+// tj + 32 b); a step publishes the pivot's row, column and reciprocal through shared memory (two sets,
+// one barrier a step). Latency: the kernel above meets five barriers and the caches at each step, 367 us
+// for 102 unknowns; this takes 152.
+constexpr int kGjMax = 128;
+
+__global__ void __launch_bounds__(1024) k_amg_gauss_jordan_regs(int n, double* __restrict__ M) {
+  constexpr int T = kGjMax / 32;
+  __shared__ double row[2][kGjMax], col[2][kGjMax], scale[2];
+  const int ti = threadIdx.x >> 5, tj = threadIdx.x & 31;
+  double m[T][T];
+#pragma unroll
+  for (int a = 0; a < T; ++a)
+#pragma unroll
+    for (int b = 0; b < T; ++b) {
+      const int i = ti + 32 * a, j = tj + 32 * b;
+      m[a][b] = i < n && j < n ? M[(size_t)i * n + j] : 0.0;
+    }
+  for (int k = 0; k < n; ++k) {
+    const int h = k & 1, ka = k >> 5, kt = k & 31;
+#pragma unroll
+    for (int a = 0; a < T; ++a)
+#pragma unroll
+      for (int b = 0; b < T; ++b) {
+        if (tj == kt && b == ka) col[h][ti + 32 * a] = m[a][b];
+        if (ti == kt && a == ka) row[h][tj + 32 * b] = m[a][b];
+        if (ti == kt && tj == kt && a == ka && b == ka) scale[h] = fabs(m[a][b]) > 0.0 ? 1.0 / m[a][b] : 0.0;
+      }
+    __syncthreads();
+    const double s = scale[h];
+    double f[T], r[T];
+#pragma unroll
+    for (int a = 0; a < T; ++a) f[a] = col[h][ti + 32 * a];
+#pragma unroll
+    for (int b = 0; b < T; ++b) r[b] = row[h][tj + 32 * b] * s;
+#pragma unroll
+    for (int a = 0; a < T; ++a)
+#pragma unroll
+      for (int b = 0; b < T; ++b) {
+        const bool ik = ti == kt && a == ka, jk = tj == kt && b == ka;
+        m[a][b] = ik ? (jk ? s : r[b]) : jk ? -f[a] * s : fma(-f[a], r[b], m[a][b]);
+      }
+  }
+#pragma unroll
+  for (int a = 0; a < T; ++a)
+#pragma unroll
+    for (int b = 0; b < T; ++b) {
+      const int i = ti + 32 * a, j = tj + 32 * b;
+      if (i < n && j < n) M[(size_t)i * n + j] = m[a][b];
+    }
 }
 
 // ---- cycle kernels ----------------------------------------------------------------------------------
@@ -1254,9 +1268,10 @@ __global__ void __launch_bounds__(kAmgTailThreads, 1) k_amg_tail(const int* skip
 // transpose of the rounded block (J, I) (the FP64 Galerkin product is symmetric only to rounding).
 // Stored entry-major: entry e of block k at val32[e * nnzb + k].
 __global__ void k_amg_coarse_f32(AmgBsr A, float* __restrict__ val32) {
-  const int I = blockIdx.x * blockDim.x + threadIdx.x;
+  const int I = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;  // eight lanes per row
   if (I >= A.n) return;
-  for (int k = A.ptr[I]; k < A.ptr[I + 1]; ++k) {
+  const size_t nb = (size_t)A.ptr[A.n];
+  for (int k = A.ptr[I] + (threadIdx.x & 7); k < A.ptr[I + 1]; k += 8) {
     const int J = A.col[k];
     int src = k;
     bool tr = false;
@@ -1268,7 +1283,6 @@ __global__ void k_amg_coarse_f32(AmgBsr A, float* __restrict__ val32) {
       }
     }
     const double* sv = A.val + (size_t)src * 9;
-    const size_t nb = (size_t)A.ptr[A.n];
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
@@ -1312,9 +1326,10 @@ __global__ void k_amg_rigid(int N, const double* __restrict__ xy, double* __rest
 // form (thread per node) and a coarse level's entry-major FP32 copy (8 lanes per row).
 
 __global__ void __launch_bounds__(kThreads) k_amg_dinva_fine(MixedMatrix M, const double* __restrict__ dinv,
-                                                             const double* sc, const double* __restrict__ x,
-                                                             double* __restrict__ y, double* __restrict__ part) {
-  const double s = sc ? *sc : 1.0;
+                                                             double* sc, int first, const double* __restrict__ x,
+                                                             double* __restrict__ y, double* part,
+                                                             double* lam, unsigned* ticket) {
+  const double s = first ? 1.0 : *sc;
   const double2* x2 = reinterpret_cast<const double2*>(x);
   double ss = 0.0;
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < M.n_nodes; n += gridDim.x * blockDim.x) {
@@ -1340,13 +1355,14 @@ __global__ void __launch_bounds__(kThreads) k_amg_dinva_fine(MixedMatrix M, cons
   }
   __shared__ double sm[kWarps];
   const double t = block_sum<kThreads>(ss, sm);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
+  amg_norm_epilogue(t, part, lam, sc, ticket, sm);
 }
 
 __global__ void __launch_bounds__(kThreads) k_amg_dinva_coarse(AmgBsr32 A, const double* __restrict__ dinv,
-                                                               const double* sc, const double* __restrict__ x,
-                                                               double* __restrict__ y, double* __restrict__ part) {
-  const double s = sc ? *sc : 1.0;
+                                                               double* sc, int first, const double* __restrict__ x,
+                                                               double* __restrict__ y, double* part,
+                                                             double* lam, unsigned* ticket) {
+  const double s = first ? 1.0 : *sc;
   const size_t nb = (size_t)A.nnzb;
   const int lane = threadIdx.x & 31, l8 = lane & 7, sub = lane >> 3;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
@@ -1382,7 +1398,7 @@ __global__ void __launch_bounds__(kThreads) k_amg_dinva_coarse(AmgBsr32 A, const
   }
   __shared__ double sm[kWarps];
   const double t = block_sum<kThreads>(ss, sm);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
+  amg_norm_epilogue(t, part, lam, sc, ticket, sm);
 }
 
 // One full wave of a grid-stride kernel: every SM gets as many blocks as it can hold at once
@@ -1425,8 +1441,14 @@ inline int gw(long long n) { return (int)std::max<long long>(1, std::min<long lo
 
 // ---- launchers ---------------------------------------------------------------------------------------
 
+// blocks of the Galerkin value kernels: `lanes` lanes per row, at most 16 blocks per SM
+inline int gal_grid(long long rows, int lanes) {
+  const long long b = (rows * lanes + 32 * kGalWarps - 1) / (32 * kGalWarps);
+  return (int)std::max<long long>(1, std::min<long long>(b, 148LL * 16));
+}
+
 cudaError_t amg_fine_bsr(int N, const int* node_ptr, const double* vals, double* out, cudaStream_t s) {
-  k_amg_bsr2<<<g1(N), 256, 0, s>>>(N, node_ptr, vals, out);
+  k_amg_bsr2<<<g1((long long)N * 8), 256, 0, s>>>(N, node_ptr, vals, out);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1510,9 +1532,9 @@ cudaError_t amg_group(int n, const int* key, int m, int* ptr, int* cnt, int* cur
 cudaError_t amg_tentative(int B, int n_agg, const int* agg_ptr, const int* members, const double* Bf, double* P0,
                           double* Bc, int* err, cudaStream_t s) {
   if (B == 2)
-    k_amg_tentative<2><<<g1(n_agg, 128), 128, 0, s>>>(n_agg, agg_ptr, members, Bf, P0, Bc, err);
+    k_amg_tentative<2><<<g1((long long)n_agg * kTentLanes, 32 * kTentWarps), 32 * kTentWarps, 0, s>>>(n_agg, agg_ptr, members, Bf, P0, Bc, err);
   else
-    k_amg_tentative<3><<<g1(n_agg, 128), 128, 0, s>>>(n_agg, agg_ptr, members, Bf, P0, Bc, err);
+    k_amg_tentative<3><<<g1((long long)n_agg * kTentLanes, 32 * kTentWarps), 32 * kTentWarps, 0, s>>>(n_agg, agg_ptr, members, Bf, P0, Bc, err);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1521,17 +1543,21 @@ cudaError_t amg_lambda_f32(const MixedMatrix* fine, const AmgBsr32* coarse, cons
                            double* part, double* lam, int iters, cudaStream_t s) {
   const int n = fine ? 2 * fine->n_nodes : 3 * coarse->n;
   double* sc = part + kLamGrid;  // the scale of the next step
+  unsigned* ticket = reinterpret_cast<unsigned*>(part + kLamGrid + 1);
+  const cudaError_t e = cudaMemsetAsync(ticket, 0, sizeof(unsigned), s);
+  if (e != cudaSuccess) return e;
   k_amg_init_vec<<<gw(n), 256, 0, s>>>(n, x);
+  // (a block without rows adds an exact zero: small levels leave those out)
+  const int grid = std::min(kLamGrid, fine ? g1(fine->n_nodes, kThreads) : g1(coarse->n * 8LL, kThreads));
   for (int t = 0; t < iters; ++t) {
     if (fine)
-      k_amg_dinva_fine<<<kLamGrid, kThreads, 0, s>>>(*fine, dinv, t ? sc : nullptr, x, y, part);
+      k_amg_dinva_fine<<<grid, kThreads, 0, s>>>(*fine, dinv, sc, t == 0, x, y, part, lam, ticket);
     else
-      k_amg_dinva_coarse<<<kLamGrid, kThreads, 0, s>>>(*coarse, dinv, t ? sc : nullptr, x, y, part);
-    k_amg_norm<<<1, kThreads, 0, s>>>(part, kLamGrid, lam, sc);
+      k_amg_dinva_coarse<<<grid, kThreads, 0, s>>>(*coarse, dinv, sc, t == 0, x, y, part, lam, ticket);
     std::swap(x, y);
   }
   k_amg_sweep_coef<<<1, 8, 0, s>>>(lam);
-  count_launches(2 + 2LL * iters);
+  count_launches(2LL + iters);
   return cudaGetLastError();
 }
 
@@ -1548,13 +1574,12 @@ cudaError_t amg_p_count(int B, const AmgBsr& A, const int* agg, int* cnt, int* e
 
 cudaError_t amg_p_fill(int B, const AmgBsr& A, const int* agg, const double* P0, const double* dinv, const double* lam,
                        const AmgBsr& P, cudaStream_t s) {
-  const int gv = (int)std::max<long long>(1, std::min<long long>(((long long)A.n + kGalWarps - 1) / kGalWarps, 148LL * 16));
   if (B == 2) {
     k_amg_p_cols<2><<<g1(A.n, 128), 128, 0, s>>>(A.n, A, agg, P);
-    k_amg_p_vals<2><<<gv, 32 * kGalWarps, 0, s>>>(A.n, A, agg, P0, dinv, lam, P);
+    k_amg_p_vals<2, 4><<<gal_grid(A.n, 4), 32 * kGalWarps, 0, s>>>(A.n, A, agg, P0, dinv, lam, P);
   } else {
     k_amg_p_cols<3><<<g1(A.n, 128), 128, 0, s>>>(A.n, A, agg, P);
-    k_amg_p_vals<3><<<gv, 32 * kGalWarps, 0, s>>>(A.n, A, agg, P0, dinv, lam, P);
+    k_amg_p_vals<3, 8><<<gal_grid(A.n, 8), 32 * kGalWarps, 0, s>>>(A.n, A, agg, P0, dinv, lam, P);
   }
   count_launches(2);
   return cudaGetLastError();
@@ -1564,19 +1589,18 @@ cudaError_t amg_ap_count(int B, const AmgBsr& A, const AmgBsr& P, int* cnt, int*
   if (B == 2)
     k_amg_ap_count<2><<<g1(A.n, 128), 128, 0, s>>>(A.n, A, P, cnt, err);
   else
-    k_amg_ap_count<3><<<g1(A.n, 128), 128, 0, s>>>(A.n, A, P, cnt, err);
+    k_amg_ac_pattern<false><<<ac_grid(A.n), 32 * kAcWarps, 0, s>>>(A.n, A.ptr, A.col, nullptr, P, cnt, AmgBsr{}, err);
   count_launches(1);
   return cudaGetLastError();
 }
 
 cudaError_t amg_ap_fill(int B, const AmgBsr& A, const AmgBsr& P, const AmgBsr& AP, cudaStream_t s) {
-  const int gv = (int)std::max<long long>(1, std::min<long long>(((long long)A.n + kGalWarps - 1) / kGalWarps, 148LL * 16));
   if (B == 2) {
     k_amg_ap_cols<2><<<g1(A.n, 128), 128, 0, s>>>(A.n, A, P, AP);
-    k_amg_ap_vals<2><<<gv, 32 * kGalWarps, 0, s>>>(A.n, A, P, AP);
+    k_amg_ap_vals<2, 8><<<gal_grid(A.n, 8), 32 * kGalWarps, 0, s>>>(A.n, A, P, AP);
   } else {
-    k_amg_ap_cols<3><<<g1(A.n, 128), 128, 0, s>>>(A.n, A, P, AP);
-    k_amg_ap_vals<3><<<gv, 32 * kGalWarps, 0, s>>>(A.n, A, P, AP);
+    k_amg_ac_pattern<true><<<ac_grid(A.n), 32 * kAcWarps, 0, s>>>(A.n, A.ptr, A.col, nullptr, P, nullptr, AP, nullptr);
+    k_amg_ap_vals<3, 16><<<gal_grid(A.n, 16), 32 * kGalWarps, 0, s>>>(A.n, A, P, AP);
   }
   count_launches(2);
   return cudaGetLastError();
@@ -1606,12 +1630,11 @@ cudaError_t amg_ac_count(int B, int nc, const int* pt_ptr, const int* pt_idx, co
 
 cudaError_t amg_ac_fill(int B, int nc, const int* pt_ptr, const int* pt_idx, const int* p_row, const AmgBsr& P,
                         const AmgBsr& AP, const AmgBsr& Ac, cudaStream_t s) {
-  const int gv = (int)std::max<long long>(1, std::min<long long>(((long long)nc + kGalWarps - 1) / kGalWarps, 148LL * 16));
   k_amg_ac_pattern<true><<<ac_grid(nc), 32 * kAcWarps, 0, s>>>(nc, pt_ptr, pt_idx, p_row, AP, nullptr, Ac, nullptr);
   if (B == 2)
-    k_amg_ac_vals<2><<<gv, 32 * kGalWarps, 0, s>>>(nc, pt_ptr, pt_idx, p_row, P, AP, Ac);
+    k_amg_ac_vals<2, 16><<<gal_grid(nc, 16), 32 * kGalWarps, 0, s>>>(nc, pt_ptr, pt_idx, p_row, P, AP, Ac);
   else
-    k_amg_ac_vals<3><<<gv, 32 * kGalWarps, 0, s>>>(nc, pt_ptr, pt_idx, p_row, P, AP, Ac);
+    k_amg_ac_vals<3, 32><<<gal_grid(nc, 32), 32 * kGalWarps, 0, s>>>(nc, pt_ptr, pt_idx, p_row, P, AP, Ac);
   count_launches(2);
   return cudaGetLastError();
 }
@@ -1623,7 +1646,10 @@ cudaError_t amg_coarsest(int B, const AmgBsr& A, double* M, double* piv, cudaStr
     k_amg_dense<2><<<g1(A.n), 256, 0, s>>>(A.n, A, M);
   else
     k_amg_dense<3><<<g1(A.n), 256, 0, s>>>(A.n, A, M);
-  k_amg_gauss_jordan<<<1, 1024, 0, s>>>(n, M, piv);
+  if (n <= kGjMax)
+    k_amg_gauss_jordan_regs<<<1, 1024, 0, s>>>(n, M);
+  else
+    k_amg_gauss_jordan<<<1, 1024, 0, s>>>(n, M, piv);
   count_launches(2);
   return cudaGetLastError();
 }
@@ -1704,7 +1730,7 @@ cudaError_t amg_prolong_f32(const int* skip, int B, int n, const int* p_ptr, con
 }
 
 cudaError_t amg_coarse_f32(const AmgBsr& A, float* val32, cudaStream_t s) {
-  k_amg_coarse_f32<<<g1(A.n), 256, 0, s>>>(A, val32);
+  k_amg_coarse_f32<<<g1((long long)A.n * 8), 256, 0, s>>>(A, val32);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -173,10 +173,15 @@ int coarsen(cstg_ctx* ctx, AmgData* d, int l, double theta, bool* stop) {
   // distance-2 maximal independent set of the strong-connection graph
   CK(cudaMemsetAsync(d->state.p, 0, sizeof(int) * (size_t)n, ctx->stream));
   int und = n;
-  for (int round = 0; und > 0; ++round) {
+  for (int round = 0; und > 0;) {
     if (round >= kMaxMisRounds) return fail(ctx, CSTG_ERR_UNSUPPORTED, "amg_setup: aggregation did not settle");
-    CK(amg_mis_round(A, strong, buf_ptr<int>(d->state), buf_ptr<unsigned long long>(d->m1), buf_ptr<int>(d->newroot),
-                     buf_ptr<int>(d->near), buf_ptr<int>(d->und), ctx->stream));
+    // four rounds before the first look at what is left (most levels take four to six; a round on a
+    // settled set changes nothing), then one at a time
+    const int batch = round == 0 ? 4 : 1;
+    for (int b = 0; b < batch; ++b)
+      CK(amg_mis_round(A, strong, buf_ptr<int>(d->state), buf_ptr<unsigned long long>(d->m1), buf_ptr<int>(d->newroot),
+                       buf_ptr<int>(d->near), buf_ptr<int>(d->und), ctx->stream));
+    round += batch;
     const int rc = read_int(ctx, buf_ptr<int>(d->und), &und);
     if (rc) return rc;
   }
