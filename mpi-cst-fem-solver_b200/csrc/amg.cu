@@ -858,7 +858,8 @@ __global__ void __launch_bounds__(1024) k_amg_gauss_jordan_regs(int n, double* _
 __device__ __forceinline__ bool skipped(const int* skip) { return skip && *(volatile const int*)skip != 0; }
 
 // Smoother steps. With r(x) = D^-1 (b - A x):
-//   kSweepFirst     xo = beta x0 + gamma r(x0), x0 = a0 D^-1 b formed on the fly (x not read)
+//   kSweepFirst     xo = beta x0 + gamma r(x0), x0 = a0 D^-1 b (finest level: formed on the fly, x not
+//                   read; below: x, written with b by the restriction)
 //   kSweepSmooth    xo = x + gamma r(x)
 //   kSweepSecond    xo = x + cd (x - xp) + gamma r(x)   (xp: the iterate before x)
 //   kSweepResidual  xo = b - A x
@@ -1065,9 +1066,7 @@ template <int MODE, bool COH>
 __device__ __forceinline__ void sweep3_rows(const AmgBsr32& A, const double* dinv, const SweepCoef& cf,
                                             const double* b, const double* x, const double* xp, double* xo, int warp,
                                             int nw, int lane) {
-  auto xval = [&](size_t d) -> double {
-    return MODE == kSweepFirst ? cf.a0 * __ldg(&dinv[d]) * ldv<COH>(&b[d]) : ldv<COH>(&x[d]);
-  };
+  auto xval = [&](size_t d) -> double { return ldv<COH>(&x[d]); };  // (kSweepFirst: x0, from the restriction)
   const size_t nb = (size_t)A.nnzb;
   const int l8 = lane & 7, sub = lane >> 3;
   for (int base = warp * 4; base < A.n; base += nw * 4) {
@@ -1114,32 +1113,78 @@ __global__ void __launch_bounds__(256, 8) k_amg_sweep3_f32(const int* skip, AmgB
   sweep3_rows<MODE, false>(A, dinv, cf, b, x, xp, xo, warp, nw, threadIdx.x & 31);
 }
 
+// The B x 3 entries of FP32 transfer block t (the finest level's as 8-byte loads: its blocks are 24 bytes,
+// and a load of a scattered word costs the load units as much as one of two).
+template <int B>
+__device__ __forceinline__ void load_transfer(const float* p32, size_t t, float (&v)[B * 3]) {
+  if (B == 2) {
+    const float2* q = reinterpret_cast<const float2*>(p32 + t * 6);
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      const float2 w = __ldg(&q[e]);
+      v[2 * e] = w.x;
+      v[2 * e + 1] = w.y;
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < B * 3; ++e) v[e] = __ldg(&p32[t * B * 3 + e]);
+  }
+}
+
 // bc_J = sum over the P blocks of column J of P_iJ' r_i, from the FP32 copy of P stored by coarse
-// row (pt32, pt_row): one warp per coarse row, lanes over the row's blocks, fixed shuffle tree.
+// row (pt32, pt_row): one warp per coarse row, lanes over the row's blocks, fixed shuffle tree. The next
+// row's extent is loaded a row ahead.
+// bc's level starts from x0 = a0 D^-1 bc, written here (x0 null: the dense coarsest level): its first
+// sweep formed it at every neighbour from dinv and b, 18.5 us on 287,703 DOFs where it now takes 13.8.
 template <int B, bool COH>
 __device__ __forceinline__ void restrict_rows(int nc, const int* pt_ptr, const int* pt_row, const float* pt32,
-                                              const double* r, double* bc, int warp, int nw, int lane) {
+                                              const double* r, double* bc, const RestrictStart& st, int warp, int nw,
+                                              int lane) {
+  const double first = st.x0 ? sweep_coef<kSweepFirst>(st.lam, st.cheb).a0 : 0.0;
+  int t0 = 0, t1 = 0;
+  if (warp < nc) {
+    t0 = __ldg(&pt_ptr[warp]);
+    t1 = __ldg(&pt_ptr[warp + 1]);
+  }
   for (int J = warp; J < nc; J += nw) {
+    int n0 = 0, n1 = 0;
+    if (J + nw < nc) {
+      n0 = __ldg(&pt_ptr[J + nw]);
+      n1 = __ldg(&pt_ptr[J + nw + 1]);
+    }
+    const double dv = st.x0 && lane < 3 ? __ldg(&st.dinv[3 * (size_t)J + lane]) : 0.0;
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    const int t1 = __ldg(&pt_ptr[J + 1]);
-    for (int t = __ldg(&pt_ptr[J]) + lane; t < t1; t += 32) {
+    for (int t = t0 + lane; t < t1; t += 32) {
       const int i = __ldg(&pt_row[t]);
-      const float* pb = pt32 + (size_t)t * B * 3;
       float v[B * 3];
+      load_transfer<B>(pt32, (size_t)t, v);
+      double rv[B];
+      if (B == 2 && !COH) {
+        const double2 w = reinterpret_cast<const double2*>(r)[i];
+        rv[0] = w.x;
+        rv[1] = w.y;
+      } else {
 #pragma unroll
-      for (int e = 0; e < B * 3; ++e) v[e] = __ldg(&pb[e]);
+        for (int z = 0; z < B; ++z) rv[z] = ldv<COH>(&r[(size_t)i * B + z]);
+      }
 #pragma unroll
       for (int z = 0; z < B; ++z) {
-        const double rv = ldv<COH>(&r[(size_t)i * B + z]);
-        a0 = fma((double)v[z * 3 + 0], rv, a0);
-        a1 = fma((double)v[z * 3 + 1], rv, a1);
-        a2 = fma((double)v[z * 3 + 2], rv, a2);
+        a0 = fma((double)v[z * 3 + 0], rv[z], a0);
+        a1 = fma((double)v[z * 3 + 1], rv[z], a1);
+        a2 = fma((double)v[z * 3 + 2], rv[z], a2);
       }
     }
     a0 = warp_sum(a0);
     a1 = warp_sum(a1);
     a2 = warp_sum(a2);
-    if (lane < 3) bc[3 * (size_t)J + lane] = lane == 0 ? a0 : lane == 1 ? a1 : a2;
+    if (lane < 3) {
+      const size_t d = 3 * (size_t)J + lane;
+      const double v = lane == 0 ? a0 : lane == 1 ? a1 : a2;
+      bc[d] = v;
+      if (st.x0) st.x0[d] = first * dv * v;
+    }
+    t0 = n0;
+    t1 = n1;
   }
 }
 
@@ -1147,32 +1192,56 @@ template <int B>
 __global__ void __launch_bounds__(256) k_amg_restrict_f32(const int* skip, int nc, const int* __restrict__ pt_ptr,
                                                           const int* __restrict__ pt_row,
                                                           const float* __restrict__ pt32, const double* r,
-                                                          double* bc) {
+                                                          double* bc, RestrictStart st) {
   if (skipped(skip)) return;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-  restrict_rows<B, false>(nc, pt_ptr, pt_row, pt32, r, bc, warp, nw, threadIdx.x & 31);
+  restrict_rows<B, false>(nc, pt_ptr, pt_row, pt32, r, bc, st, warp, nw, threadIdx.x & 31);
 }
 
-// x += P xc with the FP32 copy of P (thread per fine row)
+// x += P xc with the FP32 copy of P (thread per fine row). The loads of several blocks are in flight at
+// once; the additions follow in block order. Bound by the load units (scattered rows); 2,000,244 DOFs: 34
+// -> 25 us with 8-byte loads, three blocks at a time (15 at the measured HBM bandwidth).
 template <int B, bool COH>
 __device__ __forceinline__ void prolong_rows(int n, const int* p_ptr, const int* p_col, const float* p32,
                                              const double* xc, double* x, int tid, int nt) {
+  constexpr int U = B == 2 ? 3 : 2;
   for (int i = tid; i < n; i += nt) {
     double acc[B];
+    if (B == 2 && !COH) {
+      const double2 w = reinterpret_cast<const double2*>(x)[i];
+      acc[0] = w.x;
+      acc[1] = w.y;
+    } else {
 #pragma unroll
-    for (int r = 0; r < B; ++r) acc[r] = ldv<COH>(&x[(size_t)i * B + r]);
-    const int q1 = __ldg(&p_ptr[i + 1]);
-    for (int q = __ldg(&p_ptr[i]); q < q1; ++q) {
-      const float* pb = p32 + (size_t)q * B * 3;
-      const double* c = xc + 3 * (size_t)__ldg(&p_col[q]);
-      const double c0 = ldv<COH>(&c[0]), c1 = ldv<COH>(&c[1]), c2 = ldv<COH>(&c[2]);
-#pragma unroll
-      for (int r = 0; r < B; ++r)
-        acc[r] = fma((double)__ldg(&pb[r * 3 + 2]), c2,
-                     fma((double)__ldg(&pb[r * 3 + 1]), c1, fma((double)__ldg(&pb[r * 3]), c0, acc[r])));
+      for (int r = 0; r < B; ++r) acc[r] = ldv<COH>(&x[(size_t)i * B + r]);
     }
+    const int q1 = __ldg(&p_ptr[i + 1]);
+    for (int q = __ldg(&p_ptr[i]); q < q1; q += U) {
+      float v[U][B * 3];
+      double c[U][3];
 #pragma unroll
-    for (int r = 0; r < B; ++r) x[(size_t)i * B + r] = acc[r];
+      for (int u = 0; u < U; ++u) {
+        const int k = min(q + u, q1 - 1);
+        const double* xj = xc + 3 * (size_t)__ldg(&p_col[k]);
+        load_transfer<B>(p32, (size_t)k, v[u]);
+#pragma unroll
+        for (int e = 0; e < 3; ++e) c[u][e] = ldv<COH>(&xj[e]);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (q + u < q1) {
+#pragma unroll
+          for (int r = 0; r < B; ++r)
+            acc[r] = fma((double)v[u][r * 3 + 2], c[u][2],
+                         fma((double)v[u][r * 3 + 1], c[u][1], fma((double)v[u][r * 3], c[u][0], acc[r])));
+        }
+    }
+    if (B == 2) {
+      reinterpret_cast<double2*>(x)[i] = make_double2(acc[0], acc[1]);
+    } else {
+#pragma unroll
+      for (int r = 0; r < B; ++r) x[(size_t)i * B + r] = acc[r];
+    }
   }
 }
 
@@ -1237,13 +1306,15 @@ __global__ void __launch_bounds__(kAmgTailThreads, 1) k_amg_tail(const int* skip
   prefetch_l2(T.Minv, sizeof(double) * (size_t)T.n_coarse * T.n_coarse, tid, nt);
   for (int l = 0; l + 1 < T.nl; ++l) {
     const AmgTailLevel& v = T.L[l];
-    sweep3_rows<kSweepFirst, true>(v.A, v.dinv, sweep_coef<kSweepFirst>(v.lam, T.cheb), v.b, nullptr, nullptr, v.x,
+    sweep3_rows<kSweepFirst, true>(v.A, v.dinv, sweep_coef<kSweepFirst>(v.lam, T.cheb), v.b, v.xa, nullptr, v.x,
                                    warp, nw, lane);
     cl.sync();
     sweep3_rows<kSweepResidual, true>(v.A, v.dinv, SweepCoef{0.0, 1.0, 0.0, 0.0}, v.b, v.x, nullptr, v.r, warp, nw,
                                       lane);
     cl.sync();
-    restrict_rows<3, true>(v.nc, v.pt_ptr, v.pt_row, v.pt32, v.r, T.L[l + 1].b, warp, nw, lane);
+    const AmgTailLevel& w = T.L[l + 1];
+    restrict_rows<3, true>(v.nc, v.pt_ptr, v.pt_row, v.pt32, v.r, w.b,
+                           RestrictStart{l + 2 < T.nl ? w.xa : nullptr, w.dinv, w.lam, T.cheb}, warp, nw, lane);
     cl.sync();
   }
   gemv_rows<true>(T.n_coarse, T.Minv, T.L[T.nl - 1].b, T.L[T.nl - 1].x, warp, nw, lane);
@@ -1709,12 +1780,12 @@ cudaError_t amg_sweep3_f32(const int* skip, int mode, int cheb, const AmgBsr32& 
 }
 
 cudaError_t amg_restrict_f32(const int* skip, int B, int nc, const int* pt_ptr, const int* pt_row, const float* pt32,
-                             const double* r, double* bc, cudaStream_t s) {
+                             const double* r, double* bc, const RestrictStart& st, cudaStream_t s) {
   if (B == 2)
     k_amg_restrict_f32<2><<<one_wave((const void*)k_amg_restrict_f32<2>, (long long)nc * 32), 256, 0, s>>>(skip, nc, pt_ptr, pt_row,
-                                                                                            pt32, r, bc);
+                                                                                            pt32, r, bc, st);
   else
-    k_amg_restrict_f32<3><<<gw((long long)nc * 32), 256, 0, s>>>(skip, nc, pt_ptr, pt_row, pt32, r, bc);
+    k_amg_restrict_f32<3><<<gw((long long)nc * 32), 256, 0, s>>>(skip, nc, pt_ptr, pt_row, pt32, r, bc, st);
   count_launches(1);
   return cudaGetLastError();
 }

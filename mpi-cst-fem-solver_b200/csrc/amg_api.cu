@@ -410,6 +410,19 @@ int amg_build(cstg_ctx* ctx) {
   return CSTG_OK;
 }
 
+// What the restriction to level l writes besides its right-hand side: the first iterate, in xa, unless
+// the level is the dense coarsest.
+RestrictStart restrict_start(AmgData* d, size_t l) {
+  RestrictStart st;
+  if ((int)l + 1 == d->nl) return st;
+  AmgLevel& lv = d->L[l];
+  st.x0 = buf_ptr<double>(lv.xa);
+  st.dinv = buf_ptr<double>(lv.dinv);
+  st.lam = buf_ptr<double>(lv.lam);
+  st.cheb = d->cheb;
+  return st;
+}
+
 // V(2,2): x = cycle(l, b)
 // dots (finest level only, may be null): the flexible-CG scalars, taken in the last sweep
 int vcycle(cstg_ctx* ctx, AmgData* d, size_t l, const double* b, double* x, const int* skip,
@@ -441,10 +454,10 @@ int vcycle(cstg_ctx* ctx, AmgData* d, size_t l, const double* b, double* x, cons
     return fine ? amg_sweep_f32(skip, mode, cheb, mm, dinv, lam, b, xin, xp, xout, s, dk)
                 : amg_sweep3_f32(skip, mode, cheb, A32, dinv, lam, b, xin, xp, xout, s);
   };
-  CK(sweep(kSweepFirst, nullptr, nullptr, x));  // two pre-smoothing steps from x = 0
+  CK(sweep(kSweepFirst, fine ? nullptr : xa, nullptr, x));  // two pre-smoothing steps from x = 0
   CK(sweep(kSweepResidual, x, nullptr, r));
   CK(amg_restrict_f32(skip, lv.B, lv.nc, buf_ptr<int>(lv.pt_ptr), buf_ptr<int>(lv.pt_row), buf_ptr<float>(lv.pt32), r,
-                      buf_ptr<double>(nx.bc), s));
+                      buf_ptr<double>(nx.bc), restrict_start(d, l + 1), s));
   const int rc = vcycle(ctx, d, l + 1, buf_ptr<double>(nx.bc), buf_ptr<double>(nx.xb), skip, nullptr);
   if (rc) return rc;
   CK(amg_prolong_f32(skip, lv.B, lv.n, buf_ptr<int>(lv.p_ptr), buf_ptr<int>(lv.p_col), buf_ptr<float>(lv.p32),
@@ -474,7 +487,7 @@ int vcycle_pre(cstg_ctx* ctx, AmgData* d, const double* b, double* x, const int*
   CK(amg_sweep_f32(skip, kSweepFirst, d->cheb, mm, dinv, lam, b, nullptr, nullptr, x, s));
   CK(amg_sweep_f32(skip, kSweepResidual, d->cheb, mm, dinv, lam, b, x, nullptr, r, s));
   CK(amg_restrict_f32(skip, lv.B, lv.nc, buf_ptr<int>(lv.pt_ptr), buf_ptr<int>(lv.pt_row), buf_ptr<float>(lv.pt32), r,
-                      buf_ptr<double>(nx.bc), s));
+                      buf_ptr<double>(nx.bc), restrict_start(d, 1), s));
   const int rc = vcycle(ctx, d, 1, buf_ptr<double>(nx.bc), buf_ptr<double>(nx.xb), skip, nullptr);
   if (rc) return rc;
   CK(amg_prolong_f32(skip, lv.B, lv.n, buf_ptr<int>(lv.p_ptr), buf_ptr<int>(lv.p_col), buf_ptr<float>(lv.p32),

@@ -386,8 +386,14 @@ cudaError_t amg_transfer_f32(int B, const AmgBsr& P, int nnz_p, const int* pt_id
 cudaError_t amg_sweep3_f32(const int* skip, int mode, int cheb, const AmgBsr32& A, const double* dinv,
                            const double* lam, const double* b, const double* x, const double* xp, double* xo,
                            cudaStream_t s);
+// The restriction's second output: the first iterate of the level below (x0 null: none)
+struct RestrictStart {
+  double* x0 = nullptr;
+  const double *dinv = nullptr, *lam = nullptr;  // of that level
+  int cheb = 1;
+};
 cudaError_t amg_restrict_f32(const int* skip, int B, int nc, const int* pt_ptr, const int* pt_row, const float* pt32,
-                             const double* r, double* bc, cudaStream_t s);
+                             const double* r, double* bc, const RestrictStart& st, cudaStream_t s);
 cudaError_t amg_prolong_f32(const int* skip, int B, int n, const int* p_ptr, const int* p_col, const float* p32,
                             const double* xc, double* x, cudaStream_t s);
 cudaError_t amg_gemv(const int* skip, int n, const double* M, const double* b, double* x, cudaStream_t s);
