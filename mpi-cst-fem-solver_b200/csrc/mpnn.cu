@@ -406,6 +406,7 @@ __global__ void __launch_bounds__(kEncT, kEncCtasPerSm) k_mp_encode(int N, const
                                                      const int* skip, __nv_bfloat16* __restrict__ H0,
                                                      __nv_bfloat16* __restrict__ Xout, long long spin_limit,
                                                      int* err) {
+  start_next();  // (launched in the plain way: everything before has finished)
   if (skip && *skip) return;  // uniform: before any barrier or tensor-memory allocation
   __shared__ __align__(128) uint8_t stage[2][kEncStage];
   __shared__ __align__(128) uint8_t sX[4096];   // A: k 0..7 at +0, k 8..15 at +2048 (rows of 16 B)
@@ -653,6 +654,8 @@ __device__ __forceinline__ bool plan_takes(const int4 h) {
 
 template <bool TRAIN, bool LAST>
 __global__ void __launch_bounds__(kLT, kLayerCtasPerSm) k_mp_layer_tc(const MpLayerArgs a) {
+  wait_previous();
+  if (!LAST) start_next();
   const int N = a.N;
   if (a.skip && *a.skip) {  // uniform: before any barrier or tensor-memory allocation
     if (LAST)                 // the network is off: the Jacobi step
@@ -1079,6 +1082,7 @@ __global__ void __launch_bounds__(kWsT, 1)
     k_mp_layer_ws(const MpLayerArgs a, const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout) {
   const int N = a.N;
   if (a.skip && *a.skip) {  // uniform: before any barrier or tensor-memory allocation
+    wait_previous();
     if (LAST)               // the network is off: the Jacobi step
       for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * N; i += gridDim.x * blockDim.x)
         a.z[i] = (a.zbase ? a.zbase[i] : 0.0) + a.invd[i] * a.r[i];
@@ -1151,6 +1155,8 @@ __global__ void __launch_bounds__(kWsT, 1)
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     abort_flag = 0;
   }
+  wait_previous();  // (so far: parameters and flags that the kernel before does not write)
+  if (!LAST) start_next();
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -2034,14 +2040,14 @@ int tc_grid(int N, bool ws) {
 template <bool TRAIN, bool LAST>
 cudaError_t launch_layer_t(const MpLayerArgs& a, bool plan, cudaStream_t s) {
   if (!plan) {
-    k_mp_layer_tc<TRAIN, LAST><<<tc_grid(a.N, false), kLT, kTcSmem, s>>>(a);
+    launch_next(k_mp_layer_tc<TRAIN, LAST>, tc_grid(a.N, false), kLT, kTcSmem, s, a);
     return cudaSuccess;
   }
   CUtensorMap tin, tout;
   cudaError_t e = rows_map(&tin, a.Hin, a.N, kTile);
   if (e == cudaSuccess) e = rows_map(&tout, a.Hout ? a.Hout : a.Hin, a.N, 32);
   if (e != cudaSuccess) return e;
-  k_mp_layer_ws<TRAIN, LAST><<<tc_grid(a.N, true), kWsT, kWsSmem, s>>>(a, tin, tout);
+  launch_next(k_mp_layer_ws<TRAIN, LAST>, tc_grid(a.N, true), kWsT, kWsSmem, s, a, tin, tout);
   return cudaSuccess;
 }
 
