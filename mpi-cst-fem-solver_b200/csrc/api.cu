@@ -673,7 +673,7 @@ static int run_solve(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg_s
   PcgTeam team = n > 0 && even_rows && o.launch_mode != CSTG_LAUNCH_GRAPH && !instrumented && !snap
                      ? next_team(PcgTeam::kFirst)
                      : PcgTeam::kNone;
-  if (team != PcgTeam::kNone) ENSURE(ctx->pcg_work, pcg_persistent_work(n));
+  if (team < PcgTeam::kGrid) ENSURE(ctx->pcg_work, pcg_persistent_work(n));
   const int chunk = snap ? snap->every : instrumented ? kBdChunk : (o.check_interval > 0 ? o.check_interval : 50);
   // (Re)captures the chunk graph when a buffer, the shape or the method changed. The mixed
   // graph reads b (reliable updates), so it is also tied to the right-hand-side pointer.
@@ -735,7 +735,8 @@ static int run_solve(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg_s
       const int it0 = ctx->h_state->iter;
       if (team != PcgTeam::kNone) {
         // (rounded up to what a bulk copy reads)
-        if (mixed || team >= PcgTeam::kStream) ENSURE(ctx->pcg_slots, sizeof(unsigned short) * ((size_t)entries + 32));
+        if ((mixed || team >= PcgTeam::kStream) && team != PcgTeam::kGrid)
+          ENSURE(ctx->pcg_slots, sizeof(unsigned short) * ((size_t)entries + 32));
         CK(launch_pcg_persistent(team, w, pbm, mixed ? &mm : nullptr, pcm, ctx->pcg_work.p,
                                  buf_ptr<unsigned short>(ctx->pcg_slots), o.max_refinements, ctx->barrier_spin,
                                  ctx->stream));
@@ -771,7 +772,8 @@ static int run_solve(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg_s
       if (team != PcgTeam::kNone && ctx->h_state->no_halo)
         team = next_team(team);  // (the blocks' shares did not fit: nothing was done)
       else if (team != PcgTeam::kNone && ctx->h_state->done == 0)
-        team = PcgTeam::kNone;  // (a streamed mixed solve after its switch to FP64)
+        team = csr || team == PcgTeam::kGrid ? PcgTeam::kNone : PcgTeam::kGrid;  // (a streamed mixed solve after
+                                                                                 // its switch to FP64)
       if (ctx->h_state->done == CSTG_SOLVE_TIMEOUT + 1) {
         if (stats) {
           std::memset(stats, 0, sizeof *stats);

@@ -87,6 +87,8 @@ struct alignas(128) PcgState {
   int use_jacobi;       // learned: this iteration's z is D^-1 r (fallback or a non-descent z)
   int mp_skip;          // learned: the network kernels skip (done or fallback)
   int fb_it0;           // learned: iteration at the start of the stagnation window
+  unsigned int bar_count;  // persistent_grid.cu: blocks arrived at the current grid barrier
+  unsigned int bar_gen;    // persistent_grid.cu: barrier generation (bumped on release)
   int no_halo;             // persistent kernel: a block's halo does not fit (nothing was done)
   int bar_err;             // persistent kernel: a barrier wait ran out (the solve is abandoned)
   unsigned int ticket[8];  // last-block tickets, one per kernel kind
@@ -503,13 +505,16 @@ cudaError_t launch_true_residual(const PcgBuffers& w, bool restart, int max_repl
 // persistent.cu: every iteration of a solve in one kernel, run by a team of blocks; the state must be
 // initialised (launch_pcg_init / launch_mixed_init). Teams from the smallest systems up: one cluster;
 // one block per SM with the matrix in shared memory; one block per SM that streams it (by wide or
-// narrow groups of rows).
-enum class PcgTeam { kFirst = -1, kCluster = 0, kResident, kStream, kStreamNarrow, kNone };
+// narrow groups of rows); and, for the meshes that none of these holds, all vectors in global memory
+// (persistent_grid.cu).
+enum class PcgTeam { kFirst = -1, kCluster = 0, kResident, kStream, kStreamNarrow, kGrid, kNone };
 // spin_limit: polls of a wait between blocks before the solve gives up (kBarrierSpinDefault).
 constexpr long long kBarrierSpinDefault = 50000000LL;  // polls of ~40 ns: ~2 s
 // The first team after `after` that should hold the system (n nodes or CSR rows, entries in blocks or
 // CSR entries); small_ok: the cluster may be taken.
 PcgTeam pcg_persistent_team(int n, long long entries, bool mixed, bool csr, bool small_ok, PcgTeam after);
+cudaError_t launch_pcg_grid(const PcgBuffers& w, const BlockMatrix& A64, const MixedMatrix* A32,
+                            int max_final_checks, long long spin_limit, cudaStream_t s);
 size_t pcg_persistent_work(int n);  // bytes of `work` for n DOFs
 // Whether a CSR matrix's rows (the longest one given) are short and alike enough for it.
 inline bool pcg_persistent_rows(int n, long long nnz, int longest) {

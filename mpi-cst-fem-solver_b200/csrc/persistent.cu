@@ -1059,6 +1059,7 @@ PcgTeam pcg_persistent_team(int n, long long entries, bool mixed, bool csr, bool
       case PcgTeam::kResident: return resident(team_blocks(n));
       case PcgTeam::kStream: return stream(mixed ? 32 : 16, 12);
       case PcgTeam::kStreamNarrow: return stream(16, mixed ? 12 : 8);
+      case PcgTeam::kGrid: return !csr;
       default: return true;
     }
   };
@@ -1070,6 +1071,7 @@ PcgTeam pcg_persistent_team(int n, long long entries, bool mixed, bool csr, bool
 cudaError_t launch_pcg_persistent(PcgTeam team, const PcgBuffers& w, const BlockMatrix* A64, const MixedMatrix* A32,
                                   const CsrMatrixDev* csr, void* work, unsigned short* slots, int max_final_checks,
                                   long long spin_limit, cudaStream_t s) {
+  if (team == PcgTeam::kGrid) return launch_pcg_grid(w, *A64, A32, max_final_checks, spin_limit, s);
   SolveArgs a;
   const size_t n = (size_t)w.n;
   a.n = csr ? w.n : w.n / 2;
