@@ -26,8 +26,11 @@
 // its rows read) in shared memory for all load cases, forms p = z + beta p there itself, and so needs
 // two reductions an iteration and passes only z between blocks; r, Ap and x follow as far as they fit.
 // It is bound by the L2 traffic of what does not (x, the matrix) and the shared-memory gathers of p:
-// 38 us an iteration for 20,301 nodes x 4 cases on 8 SMs, against about 100 us for k_batch_pcg, which
-// gathers p through L2 and runs three phases (64 plates of n_r 20 .. 100: 177 against 382 ms). Larger
+// about 35 us an iteration for 20,301 nodes x 4 cases on 8 SMs, against about 100 us for k_batch_pcg, which
+// gathers p through L2 and runs three phases (64 plates of n_r 20 .. 100: 166 against 382 ms). The FP32
+// blocks are regrouped at a plate's start, the k-th blocks of a warp's 32 rows side by side, so that a load
+// is one run of 512 bytes instead of 32 sectors that the small L1 beside the vectors drops before their
+// second half is read (177 -> 166 ms). Larger
 // plates, whose p does not fit, run faster with all cases on k_batch_pcg than with a case or two
 // at a time here (n_r 20 .. 200: 2.1 against 3.6 s), so a batch that holds one goes there as a whole; a
 // single plate whose numbering makes its halo too large is put on a list for it.
@@ -499,6 +502,16 @@ __device__ __forceinline__ int case_pitch(int n) {
   return (n + 7) / 8 * 8 + (G == 1 ? 0 : 8 / G);
 }
 
+// The place of the k-th off-diagonal block of each lane's row among the regrouped blocks of a warp's 32
+// nodes (all first blocks, all second blocks, ...): `run` is the next free place, c the row's blocks (0: no
+// row). A lane without a k-th block gets a valid place.
+__device__ __forceinline__ int lane_place(int& run, int k, int c, int lane) {
+  const unsigned on = __ballot_sync(0xffffffffu, k < c);
+  const int at = run + __popc(on & ((1u << lane) - 1u));
+  run += __popc(on);
+  return k < c ? at : run - 1;
+}
+
 // All load cases of a plate; dyn: shared memory from the end of the halo's list on.
 template <int R, int T>
 __device__ __forceinline__ void solve_cases(const BatchArgs& a, const cg::cluster_group& cl, HaloShared<R, T>& sh,
@@ -633,7 +646,9 @@ __device__ __forceinline__ void solve_cases(const BatchArgs& a, const cg::cluste
 #pragma unroll
     for (int q = 0; q < G; ++q) pap[q] = 0.0;
     const bool fp64 = sh.fp64 != 0;
-    for (int i = tid; i < cnt; i += T) {
+    for (int i0 = tid - lane; i0 < cnt; i0 += T) {
+      const bool on = i0 + lane < cnt;  // (a lane past the end repeats the last row, and adds nothing)
+      const int i = on ? i0 + lane : cnt - 1;
       const int n = n0 + i;
       const int b0 = __ldg(&a.A64.node_ptr[n]), deg = __ldg(&a.A64.node_ptr[n + 1]) - b0;
       const unsigned short* sl = a.slots + (b0 - n);
@@ -657,17 +672,19 @@ __device__ __forceinline__ void solve_cases(const BatchArgs& a, const cg::cluste
           }
         }
       } else {
-        const int c = deg - 1;
-        const float4* f4 = a.A32.val32 + (b0 - n);
+        const int c = on ? deg - 1 : 0;
+        const int longest = __reduce_max_sync(0xffffffffu, c);
+        int run = __shfl_sync(0xffffffffu, b0 - n, 0);
         constexpr int kN = 3;  // neighbours whose matrix loads are in flight together
-        for (int k0 = 0; k0 < c; k0 += kN) {
+        for (int k0 = 0; k0 < longest; k0 += kN) {
           int slot[kN];
           float4 f[kN];
 #pragma unroll
           for (int u = 0; u < kN; ++u) {
-            const int k = min(k0 + u, c - 1);
-            slot[u] = k0 + u < c ? (int)sl[k] : i;  // (the node itself: a zero difference)
-            f[u] = __ldg(f4 + k);
+            const int at = lane_place(run, k0 + u, c, lane);
+            const int to = (int)__ldcg(&a.lane_slots[at]);
+            f[u] = __ldcg(&a.lane_vals[at]);
+            slot[u] = k0 + u < c ? to : i;  // (the node itself: a zero difference)
           }
 #pragma unroll
           for (int u = 0; u < kN; ++u) {
@@ -689,6 +706,7 @@ __device__ __forceinline__ void solve_cases(const BatchArgs& a, const cg::cluste
       }
 #pragma unroll
       for (int q = 0; q < G; ++q) {
+        if (!on) break;
         Ap.at(i, q) = y[q];
         pap[q] = dot2(pn[q], y[q], pap[q]);
       }
@@ -970,6 +988,21 @@ __global__ void __launch_bounds__(T, 1) k_batch_halo(const BatchArgs a) {
           a.slots[o++] = s16;
         }
       }
+      // the rows of each warp's 32 nodes regrouped, by the lanes that will read them (and wrote the slots)
+      if (a.A32.val32)
+        for (int i0 = tid - lane; i0 < cnt; i0 += T) {
+          const bool on = i0 + lane < cnt;
+          const int n = n0 + (on ? i0 + lane : cnt - 1), b0 = a.A64.node_ptr[n], from = b0 - n;
+          const int c = on ? a.A64.node_ptr[n + 1] - b0 - 1 : 0;
+          const int longest = __reduce_max_sync(0xffffffffu, c);
+          int run = __shfl_sync(0xffffffffu, from, 0);
+          for (int k = 0; k < longest; ++k) {
+            const int at = lane_place(run, k, c, lane);
+            if (k >= c) continue;
+            a.lane_slots[at] = a.slots[from + k];
+            a.lane_vals[at] = a.A32.val32[from + k];
+          }
+        }
     }
     cl.sync();  // the wanted marks of all blocks
     unsigned* want = reinterpret_cast<unsigned*>(hid + nh);

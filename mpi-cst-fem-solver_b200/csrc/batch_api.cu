@@ -60,7 +60,8 @@ int prepare(cstg_ctx* ctx, int n_sys, const int32_t* offs, int n_rhs, const cstg
   ENSURE(ctx->bat_order, sizeof(int) * (size_t)n_sys);
   ENSURE(ctx->bat_queue, sizeof(int) * ((size_t)n_sys + 64));
   ENSURE(ctx->bat_wanted, (size_t)ctx->n_nodes);
-  ENSURE(ctx->bat_slots, sizeof(unsigned short) * (size_t)(ctx->nnz / 4));
+  ENSURE(ctx->bat_slots, 2 * sizeof(unsigned short) * (size_t)(ctx->nnz / 4));
+  if (o.precision == CSTG_PRECISION_MIXED) ENSURE(ctx->bat_lane, sizeof(float4) * (size_t)(ctx->nnz / 4));
   ENSURE(ctx->bat_b, vec);
   ENSURE(ctx->bat_x, vec);
   ENSURE(ctx->bat_r, vec);
@@ -120,6 +121,8 @@ int enqueue(cstg_ctx* ctx, int n_sys, int n_rhs, const double* d_b, double* d_x,
     a.rest = a.queue + 64;
     a.wanted = buf_ptr<unsigned char>(ctx->bat_wanted);
     a.slots = buf_ptr<unsigned short>(ctx->bat_slots);
+    a.lane_slots = a.slots + ctx->nnz / 4;
+    a.lane_vals = buf_ptr<float4>(ctx->bat_lane);
     if (o.precision == CSTG_PRECISION_MIXED) a.A32 = mixed_view(ctx);
     a.A64 = block_view(ctx);
     a.start_fp64 = o.precision == CSTG_PRECISION_FP64;

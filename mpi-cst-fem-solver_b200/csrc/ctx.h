@@ -91,7 +91,7 @@ struct cstg_ctx {
   DevBuf mat, mat_tab;
 
   // batched solves: plate table, LPT order, interleaved load-case vectors, per-system results
-  DevBuf bat_sys, bat_order, bat_queue, bat_wanted, bat_slots, bat_b, bat_x, bat_r, bat_p, bat_Ap, bat_stats, bat_in, bat_out;
+  DevBuf bat_sys, bat_order, bat_queue, bat_wanted, bat_slots, bat_lane, bat_b, bat_x, bat_r, bat_p, bat_Ap, bat_stats, bat_in, bat_out;
   std::vector<int32_t> bat_offsets;  // host copy of the last validated plate table
   unsigned long long bat_checked_gen = ~0ull;
   cstg_batch_config bat_cfg{};       // tuned launch shape (cluster_ctas == 0: not tuned)

@@ -146,6 +146,9 @@ struct BatchArgs {
   int* rest = nullptr;            // [n_sys] those plates
   unsigned char* wanted = nullptr;  // [N] nodes that other blocks need, zero at launch
   unsigned short* slots = nullptr;  // neighbours in a block's own numbering, one per off-diagonal block
+  // the same and the FP32 blocks, regrouped over 32 nodes by their place in the row (k_batch_halo)
+  unsigned short* lane_slots = nullptr;
+  float4* lane_vals = nullptr;
   unsigned smem = 0;              // dynamic shared memory of a block
   MixedMatrix A32;                // FP32 difference-form operator (unused when start_fp64)
   BlockMatrix A64;                // FP64 operator (true residuals, FP64 mode)
