@@ -29,8 +29,7 @@ MpnnParams params_view(cstg_ctx* ctx) {
 }
 
 // The layers' gather plan for the current node pattern (built once per pattern): per tile of 128
-// nodes the runs of consecutive rows its nodes read, and per node the slots of its own and its
-// neighbours' rows in that union.
+// nodes the runs of the other rows its nodes read, and per node the places of its neighbours' rows.
 int plan_ready(cstg_ctx* ctx) {
   if (!ctx->lp_plan_on || ctx->lp_plan_for == ctx->pattern_count) return CSTG_OK;
   const int N = ctx->n_nodes;
@@ -48,7 +47,7 @@ int plan_ready(cstg_ctx* ctx) {
     CK(cudaStreamSynchronize(ctx->stream));
     for (const int4& h : hdr) planned += h.z == 0 ? 1 : 0;
   }
-  // the plan kernel (2 CTAs per SM, bulk-copied unions) pays off when a good share of the tiles
+  // the plan kernel (one CTA per SM, bulk-copied rows) pays off when a good share of the tiles
   // is planned; patterns numbered without locality (most tiles rejected) keep the row kernel
   ctx->lp_plan_use = 4 * planned >= tiles;
   ctx->lp_plan_for = ctx->pattern_count;
