@@ -582,39 +582,31 @@ __global__ void __launch_bounds__(kEncT, kEncCtasPerSm) k_mp_encode(int N, const
 }
 
 
-// Two FP32 values in one 64-bit register, and the packed adds and products on them: one instruction
-// for two IEEE round-to-nearest operations (the bits of the scalar ones).
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack_f2(uint32_t lo, uint32_t hi) {
-  f32x2 d;
-  asm("mov.b64 %0, {%1, %2};\n" : "=l"(d) : "r"(lo), "r"(hi));
+// Neighbour sums in FP32: acc[j] += feature j of the chunk v (8 BF16) with the mixed-precision
+// add.rn.f32.bf16 (the BF16 operand widened exactly, one IEEE round-to-nearest add: the same result
+// as widening and a scalar add, in one instruction per feature; packed adds of two widened features take
+// three for two).
+__device__ __forceinline__ void add_chunk_bf(float (&acc)[8], const uint4 v) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    asm("{\n\t.reg .b16 lo, hi;\n\t"
+        "mov.b32 {lo, hi}, %2;\n\t"
+        "add.rn.f32.bf16 %0, lo, %0;\n\t"
+        "add.rn.f32.bf16 %1, hi, %1;\n\t}\n"
+        : "+f"(acc[2 * q]), "+f"(acc[2 * q + 1])
+        : "r"(w[q]));
+}
+// g + the low / high BF16 of w, widened exactly: one IEEE round-to-nearest add.
+__device__ __forceinline__ float add_bf_lo(uint32_t w, float g) {
+  float d;
+  asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %1;\n\tadd.rn.f32.bf16 %0, lo, %2;\n\t}\n" : "=f"(d) : "r"(w), "f"(g));
   return d;
 }
-__device__ __forceinline__ float2 unpack_f2(f32x2 v) {
-  float2 d;
-  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(d.x), "=f"(d.y) : "l"(v));
+__device__ __forceinline__ float add_bf_hi(uint32_t w, float g) {
+  float d;
+  asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %1;\n\tadd.rn.f32.bf16 %0, hi, %2;\n\t}\n" : "=f"(d) : "r"(w), "f"(g));
   return d;
-}
-__device__ __forceinline__ f32x2 add_f2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 mul_f2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-// The two BF16 of w, widened exactly (low one first).
-__device__ __forceinline__ f32x2 widen_bf2(uint32_t w) { return pack_f2(w << 16, w & 0xFFFF0000u); }
-
-// Neighbour sums in FP32: acc[q] += features 2q, 2q + 1 of the chunk v (8 BF16), the BF16 operands
-// widened exactly.
-__device__ __forceinline__ void add_chunk_bf(f32x2 (&acc)[4], const uint4 v) {
-  acc[0] = add_f2(acc[0], widen_bf2(v.x));
-  acc[1] = add_f2(acc[1], widen_bf2(v.y));
-  acc[2] = add_f2(acc[2], widen_bf2(v.z));
-  acc[3] = add_f2(acc[3], widen_bf2(v.w));
 }
 // Eight BF16 -0.0: the chunk a missing neighbour contributes. x + (-0) = x exactly for every x
 // (both zeros included), so a sum padded with it has the bits of the sum without it, and the
@@ -635,16 +627,9 @@ __device__ __forceinline__ float inv_deg(int deg) {
   return r;
 }
 // The chunk's mean as 8 BF16: each sum times inv, rounded to nearest.
-__device__ __forceinline__ uint4 mean_chunk(const f32x2 (&acc)[4], float inv) {
-  const f32x2 ii = pack_f2(__float_as_uint(inv), __float_as_uint(inv));
-  const float2 a = unpack_f2(mul_f2(acc[0], ii)), b = unpack_f2(mul_f2(acc[1], ii)),
-               c = unpack_f2(mul_f2(acc[2], ii)), d = unpack_f2(mul_f2(acc[3], ii));
-  return make_uint4(pack_bf2(a.x, a.y), pack_bf2(b.x, b.y), pack_bf2(c.x, c.y), pack_bf2(d.x, d.y));
-}
-// The residual add of two features: the BF16 pair w of the node's own row, widened exactly, plus g.
-__device__ __forceinline__ uint32_t residual_bf2(uint32_t w, float g0, float g1) {
-  const float2 h = unpack_f2(add_f2(widen_bf2(w), pack_f2(__float_as_uint(g0), __float_as_uint(g1))));
-  return pack_bf2(h.x, h.y);
+__device__ __forceinline__ uint4 mean_chunk(const float (&acc)[8], float inv) {
+  return make_uint4(pack_bf2(acc[0] * inv, acc[1] * inv), pack_bf2(acc[2] * inv, acc[3] * inv),
+                    pack_bf2(acc[4] * inv, acc[5] * inv), pack_bf2(acc[6] * inv, acc[7] * inv));
 }
 
 // A tile the plan takes: its union fits one stage in at most kPlanMaxRuns runs.
@@ -760,7 +745,7 @@ __global__ void __launch_bounds__(kLT, kLayerCtasPerSm) k_mp_layer_tc(const MpLa
         const int k0 = __shfl_sync(0xffffffffu, np, li) - np0;
         const int k1 = __shfl_sync(0xffffffffu, np, li + 1) - np0;
         uint4 own = make_uint4(0u, 0u, 0u, 0u);
-        f32x2 acc[4] = {0ull, 0ull, 0ull, 0ull};
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         int deg = 0;
         if (n < N) {
           own = __ldg(reinterpret_cast<const uint4*>(a.Hin + (size_t)n * F) + c);
@@ -960,7 +945,7 @@ __global__ void __launch_bounds__(kLT, kLayerCtasPerSm) k_mp_layer_tc(const MpLa
 //            come from global memory.
 //  gather (warps 0..15): 8 nodes per warp, four at once with 8 lanes per node (lane c: features
 //            8c..8c+7); the rows at a node's six places (the seventh only in tiles that have such a node)
-//            are read and summed in pattern order with packed FP32 adds, times 1/deg, rounded to BF16 into
+//            are read and summed in pattern order with add.rn.f32.bf16, times 1/deg, rounded to BF16 into
 //            the mean half (K-major, 128-byte swizzle); one arrival per warp on the union (free) and on
 //            the mean half (ready). The next tile's places are loaded a tile ahead.
 //  MMA (warp 25, one thread): 8 x tcgen05.mma (M=128, N=64, K=16: four K-slices of the own rows,
@@ -976,12 +961,13 @@ __global__ void __launch_bounds__(kLT, kLayerCtasPerSm) k_mp_layer_tc(const MpLa
 // issue slots; each is bounded (spin_limit polls). A role that gives up records the timeout and
 // raises the CTA's abort flag, which every other wait polls. Before the CTA leaves, the copies and
 // MMAs already issued have completed (bounded waits) and the tensor stores have read their staging.
-// Bound by the gathers' instructions (73 % of the issue slots; shared memory 61 %), not by HBM. Measured on
-// the 2M-DOF plate, 86 us a layer and 100 us the last (41 at the measured HBM bandwidth). Before: 89 and
-// 107 us with the own rows copied twice, two stages, a barrier per kind of copy, seven places summed with
-// scalar adds, and four epilogue warps, which were the last layer's limit. A third stage, other rows alone in the
-// union, or fewer adds gave nothing by themselves; dropping waits from the gather warps' path did (each costs
-// ~270 cycles behind their loads). 16 gather warps and plain rows without branches were worth 186 -> 106 us.
+// Bound by the gathers' instructions (73 % of the issue slots; shared memory 55 %), not by HBM. Measured on
+// the 2M-DOF plate, 82 us a layer and 96 us the last (41 at the measured HBM bandwidth). Before: 89 and
+// 107 us with the own rows copied twice, two stages, a barrier per kind of copy, seven places, and four
+// epilogue warps, which were the last layer's limit. A third stage, other rows alone in the union, or six
+// places gave nothing by themselves; dropping waits from the gather warps' path did (each costs ~270 cycles
+// behind their loads). Packed FP32 adds of widened pairs, three instructions for two, took 84 and 97. 16
+// gather warps and plain rows without branches were worth 186 -> 106 us.
 constexpr int kWsGatherWarps = 16, kWsEpiWarps = 4;
 constexpr int kWsEpi0 = kWsGatherWarps;                    // warps 16..19 (TMEM lane quarters 0..3)
 constexpr int kWsOwnProd = kWsEpi0 + 2 * kWsEpiWarps;      // warp 24
@@ -1196,7 +1182,7 @@ __global__ void __launch_bounds__(kWsT, 1)
       for (int u = 0; u < 2; ++u) {
         const int m = warp * 8 + u * 4 + g;
         const int n = tile * kTile + m;
-        f32x2 acc[4] = {0ull, 0ull, 0ull, 0ull};
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         int deg = 0;
         if (planned && n < N) {
           // chunk c of the row at place e is at unit e ^ c: own rows carry their swizzle key in e's
@@ -1290,7 +1276,7 @@ __global__ void __launch_bounds__(kWsT, 1)
           for (int j = 0; j < 4; ++j) {  // (the accumulator holds the bias already)
             const float g0 = fmaxf(__uint_as_float(v[cc * 8 + 2 * j]), 0.f);
             const float g1 = fmaxf(__uint_as_float(v[cc * 8 + 2 * j + 1]), 0.f);
-            hw[j] = residual_bf2(ow[j], g0, g1);
+            hw[j] = pack_bf2(add_bf_lo(ow[j], g0), add_bf_hi(ow[j], g1));
             gw[j] = pack_bf2(g0, g1);
           }
           if (TRAIN && n < N)
