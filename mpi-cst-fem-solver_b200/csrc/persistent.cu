@@ -43,6 +43,7 @@
 
 #include <algorithm>
 
+#include "block_max.cuh"
 #include "common.cuh"
 #include "kernels.h"
 
@@ -525,10 +526,7 @@ __global__ void __launch_bounds__(T, 1) k_pcg_persistent(const SolveArgs a) {
   const int cnt = n1 - n0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned tag = 0;
-  if (threadIdx.x == 0) {
-    sh.ok = 1;
-    sh.widest = 0;
-  }
+  if (threadIdx.x == 0) sh.ok = 1;
   if constexpr (CLUSTER) cg::this_cluster().sync();  // every block runs before its inbox is written
 
   // -- the halo and the rows' local numbering
@@ -542,11 +540,11 @@ __global__ void __launch_bounds__(T, 1) k_pcg_persistent(const SolveArgs a) {
   const int groups = (cnt + kGroup - 1) / kGroup;
   unsigned stage_S = 0, stage_col = 0, stage_bytes = 0;  // a stage: offsets of the sums and slots, size
   if constexpr (!RES) {
-    for (int g = threadIdx.x; g < groups; g += T) atomicMax(&sh.widest, Group<OP>(gptr, n0, cnt, g, kGroup).ne);
-    __syncthreads();
-    stage_S = ((unsigned)sh.widest * kEntryBytes<OP> + 15u) & ~15u;
+    const unsigned widest =
+        (unsigned)block_max<T>(&sh.widest, groups, [&](int g) { return Group<OP>(gptr, n0, cnt, g, kGroup).ne; });
+    stage_S = (widest * kEntryBytes<OP> + 15u) & ~15u;
     stage_col = stage_S + (OP == kMixed ? 32u * kGroup : 0u);
-    stage_bytes = stage_col + (((unsigned)sh.widest * 2u + 14u + 15u) & ~15u);
+    stage_bytes = stage_col + ((widest * 2u + 14u + 15u) & ~15u);
   }
   {
     // p at own nodes and halo, the halo's list, the row starts and the wanted bits must fit, and
