@@ -366,11 +366,21 @@ __device__ __forceinline__ void cst_element(const double* xy, const double* D, d
 // Half of B is zero (B(1, even) and B(0, odd)), and the reference multiplies and adds those zeros. The
 // terms are left out here: a sum that starts from +0.0 is never -0.0, and adding +-0.0 to any other
 // value changes nothing, so every nonzero entry keeps its bits; a zero's sign is lost when it is added
-// to the matrix entry, which starts from +0.0 too. (D, B and DB finite, as they have to be.)
+// to the matrix entry, which starts from +0.0 too. That needs D, B and DB finite (a zero times an infinity is
+// not a number, and the diagonal's check then refuses the system): nodes with others take assemble_node_full.
 __device__ __forceinline__ double ke_entry(const CstB& o, int i, int j) {
   const int p = i < j ? i : j, q = i < j ? j : i;
   const double x = (p & 1) ? __dmul_rn(o.B[6 + p], o.DB[6 + q]) : __dmul_rn(o.B[p], o.DB[q]);
   return __dmul_rn(o.scale, __dadd_rn(x, __dmul_rn(o.B[12 + p], o.DB[12 + q])));
+}
+
+// D and B are finite and D B has not overflowed: every entry of D meets a nonzero place of B and every
+// entry of B one of D's in the terms that DB keeps, so DB shows it.
+__device__ __forceinline__ bool finite_element(const CstB& o) {
+  int most = 0;
+#pragma unroll
+  for (int k = 0; k < 18; ++k) most = max(most, __double2hiint(o.DB[k]) & 0x7fffffff);
+  return most < 0x7ff00000;
 }
 
 // Rows 2A, 2A+1 of an element's Ke added into a node's two CSR rows (entry k of row r at
@@ -398,6 +408,38 @@ __device__ __forceinline__ void add_element(const CstB& o, int corner, unsigned 
     add_corner_rows<1>(o, slots, at);
   else
     add_corner_rows<2>(o, slots, at);
+}
+
+// A node's two rows with B's zeros multiplied and added, as the reference does; entry k at to[k stride]. A call,
+// so that the nodes that need it cost the others no registers.
+__device__ __noinline__ void assemble_node_full(const double* xy, const int* tri, const int* ne, const unsigned* slot,
+                                                int q0, int q1, Mat3 Dm, double thickness, const int* mat,
+                                                const double* Dtab, const double* ttab, int deg, double* to,
+                                                int stride) {
+  for (int k = 0; k < 4 * deg; ++k) to[k * stride] = 0.0;
+  for (int q = q0; q < q1; ++q) {
+    const int e = ne[q] / 3, corner = ne[q] - 3 * e;
+    double exy[6], B[18], DB[18];
+    for (int c = 0; c < 6; ++c) exy[c] = xy[2 * tri[3 * e + (c >> 1)] + (c & 1)];
+    const double* D = mat ? Dtab + 9 * mat[e] : Dm.v;
+    cst_B(exy, B);
+    for (int i = 0; i < 3; ++i)
+      for (int j = 0; j < 6; ++j) {
+        double s = 0.0;
+        for (int k = 0; k < 3; ++k) s = __dadd_rn(s, __dmul_rn(D[i * 3 + k], B[k * 6 + j]));
+        DB[i * 6 + j] = s;
+      }
+    const double scale = __dmul_rn(mat ? ttab[mat[e]] : thickness,
+                                   fabs(signed_area(exy[0], exy[1], exy[2], exy[3], exy[4], exy[5])));
+    for (int r = 0; r < 2; ++r)
+      for (int j = 0; j < 6; ++j) {
+        const int i = 2 * corner + r, u = min(i, j), v = max(i, j);
+        double s = 0.0;
+        for (int k = 0; k < 3; ++k) s = __dadd_rn(s, __dmul_rn(B[k * 6 + u], DB[k * 6 + v]));
+        double& entry = to[(r * 2 * deg + 2 * (int)((slot[q] >> (8 * (j >> 1))) & 0xff) + (j & 1)) * stride];
+        entry = __dadd_rn(entry, __dmul_rn(scale, s));
+      }
+  }
 }
 
 // One thread per node: the node's two rows are zeroed, then every incident element (in
@@ -431,6 +473,7 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(
     else
       for (int k = 0; k < 4 * deg; ++k) ra[k] = 0.0;
     const int q1 = ne_ptr[n + 1];
+    bool finite = true;
     for (int q = ne_ptr[n]; q < q1; ++q) {
       const int code = ne[q], e = code / 3, a = code - 3 * e;
       const unsigned slots = slot[q];
@@ -448,11 +491,15 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(
       } else {
         cst_element(exy, Dm.v, thickness, o);
       }
+      finite &= finite_element(o);
       if (small)
         add_element(o, a, slots, [&](int r, int k) -> double& { return acc[r * 2 * deg + k][threadIdx.x]; });
       else
         add_element(o, a, slots, [&](int r, int k) -> double& { return ra[r * 2 * deg + k]; });
     }
+    if (!finite)
+      assemble_node_full(xy, tri, ne, slot, ne_ptr[n], q1, Dm, thickness, mat, Dtab, ttab, deg,
+                         small ? &acc[0][threadIdx.x] : ra, small ? kAsmThreads + 1 : 1);
     const int k = 2 * self[n];
     diag[n] = small ? make_double2(acc[k][threadIdx.x], acc[2 * deg + k + 1][threadIdx.x])
                     : make_double2(ra[k], ra[2 * deg + k + 1]);
