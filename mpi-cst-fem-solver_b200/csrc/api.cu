@@ -674,6 +674,10 @@ static int run_solve(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg_s
                      ? next_team(PcgTeam::kFirst)
                      : PcgTeam::kNone;
   if (team < PcgTeam::kGrid) ENSURE(ctx->pcg_work, pcg_persistent_work(n));
+  const auto slots_room = [&]() -> int {  // (rounded up to what a bulk copy reads)
+    ENSURE(ctx->pcg_slots, sizeof(unsigned short) * ((size_t)entries + 32));
+    return CSTG_OK;
+  };
   const int chunk = snap ? snap->every : instrumented ? kBdChunk : (o.check_interval > 0 ? o.check_interval : 50);
   // (Re)captures the chunk graph when a buffer, the shape or the method changed. The mixed
   // graph reads b (reliable updates), so it is also tied to the right-hand-side pointer.
@@ -733,13 +737,20 @@ static int run_solve(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg_s
         return fail(ctx, CSTG_ERR_TIMEOUT, "pcg_solve: the device state did not finish after %lld chunks",
                     chunks);
       const int it0 = ctx->h_state->iter;
+      rc = CSTG_OK;
+      CK(launch_first_team(
+          team,
+          [&](PcgTeam t) {
+            if ((mixed || t >= PcgTeam::kStream) && t != PcgTeam::kGrid) rc = slots_room();
+            return rc ? cudaSuccess
+                      : launch_pcg_persistent(t, w, pbm, mixed ? &mm : nullptr, pcm, ctx->pcg_work.p,
+                                              buf_ptr<unsigned short>(ctx->pcg_slots), o.max_refinements,
+                                              ctx->barrier_spin, ctx->stream);
+          },
+          next_team));
+      if (rc) return rc;
       if (team != PcgTeam::kNone) {
-        // (rounded up to what a bulk copy reads)
-        if ((mixed || team >= PcgTeam::kStream) && team != PcgTeam::kGrid)
-          ENSURE(ctx->pcg_slots, sizeof(unsigned short) * ((size_t)entries + 32));
-        CK(launch_pcg_persistent(team, w, pbm, mixed ? &mm : nullptr, pcm, ctx->pcg_work.p,
-                                 buf_ptr<unsigned short>(ctx->pcg_slots), o.max_refinements, ctx->barrier_spin,
-                                 ctx->stream));
+        // (launched)
       } else if (instrumented) {
         // SpMV (with its fused p'Ap partials), then the vector phase (x, r, p updates with their
         // fused dots), an event after each; the elapsed times are summed after the batch

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "teams.h"
+
 namespace cstg {
 
 // Slots of the device error word (each holds the smallest offending index, INT_MAX if none).
@@ -506,11 +508,7 @@ cudaError_t launch_true_residual(const PcgBuffers& w, bool restart, int max_repl
                                  cudaStream_t s);
 
 // persistent.cu: every iteration of a solve in one kernel, run by a team of blocks; the state must be
-// initialised (launch_pcg_init / launch_mixed_init). Teams from the smallest systems up: one cluster;
-// one block per SM with the matrix in shared memory; one block per SM that streams it (by wide or
-// narrow groups of rows); and, for the meshes that none of these holds, all vectors in global memory
-// (persistent_grid.cu).
-enum class PcgTeam { kFirst = -1, kCluster = 0, kResident, kStream, kStreamNarrow, kGrid, kNone };
+// initialised (launch_pcg_init / launch_mixed_init).
 // spin_limit: polls of a wait between blocks before the solve gives up (kBarrierSpinDefault).
 constexpr long long kBarrierSpinDefault = 50000000LL;  // polls of ~40 ns: ~2 s
 // The first team after `after` that should hold the system (n nodes or CSR rows, entries in blocks or
@@ -527,7 +525,8 @@ inline bool pcg_persistent_rows(int n, long long nnz, int longest) {
 cudaError_t launch_longest_row(int n, const int* row_ptr, int* longest, cudaStream_t s);
 // slots: room for one 16-bit number per matrix block, rounded up to 16 bytes (mixed solves and the
 // streaming teams). On return PcgState::no_halo is set when a block's share did not fit (nothing was
-// done then).
+// done then). An error for which unplaced() holds: the device has no room for the team (nothing was launched, but
+// `work` was overwritten).
 cudaError_t launch_pcg_persistent(PcgTeam team, const PcgBuffers& w, const BlockMatrix* A64, const MixedMatrix* A32,
                                   const CsrMatrixDev* csr, void* work, unsigned short* slots, int max_final_checks,
                                   long long spin_limit, cudaStream_t s);

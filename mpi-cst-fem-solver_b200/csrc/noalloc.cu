@@ -162,13 +162,16 @@ extern "C" int cstg_pcg_solve_static(int n_rows, const int32_t* d_row_ptr, const
   // The context's rule for the persistent kernel, where what passes between its blocks fits in place of
   // p and Ap, which it does not use.
   int longest = 0;
+  const auto next_team = [&](PcgTeam after) {
+    return pcg_persistent_team(n_rows, nnz, false, true, o.launch_mode == CSTG_LAUNCH_AUTO, after);
+  };
   PcgTeam team = PcgTeam::kNone;
   if (n_rows && pcg_persistent_work(n_rows) <= 2 * kVecBytes && h.done == 0) {
     SCK(launch_longest_row(n_rows, d_row_ptr, err + kErrSlots, s));
     SCK(cudaMemcpyAsync(&longest, err + kErrSlots, sizeof longest, cudaMemcpyDeviceToHost, s));
     SCK(cudaStreamSynchronize(s));
     if (pcg_persistent_rows(n_rows, nnz, longest))
-      team = pcg_persistent_team(n_rows, nnz, false, true, o.launch_mode == CSTG_LAUNCH_AUTO, PcgTeam::kFirst);
+      team = next_team(PcgTeam::kFirst);
     if (o.launch_mode == CSTG_LAUNCH_GRAPH || o.launch_mode == CSTG_LAUNCH_INSTRUMENTED) team = PcgTeam::kNone;
   }
   long long chunks = 0, spmv_calls = 0;
@@ -178,15 +181,21 @@ extern "C" int cstg_pcg_solve_static(int n_rows, const int32_t* d_row_ptr, const
       if (++chunks > max_chunks)
         return fail_msg(stats, CSTG_ERR_TIMEOUT, "pcg_solve_static: no end after %lld chunks", chunks);
       const int it0 = h.iter;
-      if (team != PcgTeam::kNone)
-        SCK(launch_pcg_persistent(team, w, nullptr, nullptr, &A, p, nullptr, o.max_refinements, kBarrierSpinDefault, s));
-      else
+      const bool asked = team != PcgTeam::kNone;
+      SCK(launch_first_team(
+          team,
+          [&](PcgTeam t) {
+            return launch_pcg_persistent(t, w, nullptr, nullptr, &A, p, nullptr, o.max_refinements, kBarrierSpinDefault, s);
+          },
+          next_team));
+      if (asked && team == PcgTeam::kNone) SCK(launch_pcg_init(w, o.rtol, o.max_iter, false, s));  // (p was overwritten)
+      if (team == PcgTeam::kNone)
         for (int k = 0; k < chunk; ++k) SCK(launch_pcg_iteration(w, nullptr, &A, s));
       SCK(snap());
       if (h.done == CSTG_SOLVE_TIMEOUT + 1)
         return fail_msg(stats, CSTG_ERR_TIMEOUT, "pcg_solve_static: a barrier of the persistent solve timed out");
       if (team != PcgTeam::kNone && h.no_halo) {  // (nothing was done, but p was overwritten)
-        team = pcg_persistent_team(n_rows, nnz, false, true, o.launch_mode == CSTG_LAUNCH_AUTO, team);
+        team = next_team(team);
         if (team == PcgTeam::kNone) SCK(launch_pcg_init(w, o.rtol, o.max_iter, false, s));
       }
       spmv_calls += h.iter - it0 + (h.done == CSTG_SOLVE_BREAKDOWN + 1);

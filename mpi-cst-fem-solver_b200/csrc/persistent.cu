@@ -990,7 +990,15 @@ cudaError_t launch_team(SolveArgs& a, int blocks, cudaStream_t s) {
   cfg.stream = s;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, a);
+  if (CLUSTER) {  // (a cooperative launch that does not fit is refused by itself)
+    int room = 0;
+    e = cudaOccupancyMaxActiveClusters(&room, kern, &cfg);
+    if (e != cudaSuccess) return e;
+    if (room < 1) return cudaErrorInvalidClusterSize;
+  }
+  e = cudaLaunchKernelEx(&cfg, kern, a);
+  if (e == cudaSuccess) count_launches(1);
+  return e;
 }
 
 // Blocks of a grid team: one per SM, but at least 64 nodes (rows) each, so that small systems wait for
@@ -1097,7 +1105,6 @@ cudaError_t launch_pcg_persistent(PcgTeam team, const PcgBuffers& w, const Block
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(&w.st->no_halo, 0, 2 * sizeof(int), s);  // (and bar_err)
   if (e != cudaSuccess) return e;
-  count_launches(1);
   return csr ? launch_op<kCsr>(a, team, s) : A32 ? launch_op<kMixed>(a, team, s) : launch_op<kBlock64>(a, team, s);
 }
 

@@ -440,7 +440,7 @@ cudaError_t launch_pcg_grid(const PcgBuffers& w, const BlockMatrix& A64, const M
   if (grid <= 0) return cudaErrorCooperativeLaunchTooLarge;
   e = A32 ? cudaLaunchCooperativeKernel((void*)k_pcg_grid<true>, grid, kPT, args, 0, s)
           : cudaLaunchCooperativeKernel((void*)k_pcg_grid<false>, grid, kPT, args, 0, s);
-  count_launches(1);
+  if (e == cudaSuccess) count_launches(1);
   return e;
 }
 
