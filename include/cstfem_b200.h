@@ -173,13 +173,16 @@ int cstg_version(void);
 /* The compute architecture of the library's kernels as the CUDA runtime reports it for `device`
  * (cudaFuncGetAttributes binaryVersion: 100 for sm_100a). */
 int cstg_binary_version(int device, int* version);
-/* Bounded device waits (no reference counterpart). Every device-side wait of the library gives
+/* Bounded device waits (no reference counterpart). Every device-side wait that polls gives
  * up after a number of polls and reports CSTG_ERR_TIMEOUT (stats->status CSTG_SOLVE_TIMEOUT where
  * a solve was running) with the context still usable: the persistent solve's waits
  * between blocks (default 50,000,000 polls, about 2 s) and the learned network's tensor-core waits (default
  * 4,194,304 polls). 0 makes a wait give up at once (failure-detection tests); -1 restores the
  * default. A tensor-core wait that gives up still lets its matrix multiply finish (bounded)
- * before the kernel releases its memory. */
+ * before the kernel releases its memory.
+ * The barrier of a thread-block cluster (batched solves, the multigrid's coarse levels, small solves with
+ * CSTG_LAUNCH_AUTO) is the hardware's own, among blocks that run together, and has no limit. With barrier_polls
+ * set, solves keep to the teams that poll, and solves of a caller's CSR to the captured kernels. */
 int cstg_set_wait_limits(cstg_ctx* ctx, long long barrier_polls, long long mma_polls);
 /* Kernel launches issued by this library in this process so far (every kernel node of a
  * replayed CUDA graph counts). Benchmarks read it around a timed region. */

@@ -664,11 +664,15 @@ static int run_solve(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg_s
   if (instrumented && mixed)
     return fail(ctx, CSTG_ERR_UNSUPPORTED, "pcg_solve: the instrumented launch mode runs FP64 Jacobi-PCG only");
   const bool csr = ctx->kind != 1;
-  const bool even_rows = !csr || pcg_persistent_rows(n, ctx->nnz, ctx->csr_longest);
+  // With a limit on its waits set by the caller, a solve takes only the waits it always had: the teams that poll for
+  // the mesh pattern (a cluster's barrier is the hardware's own and knows no limit), none for CSR.
+  const bool own_limit = ctx->barrier_spin != kBarrierSpinDefault;
+  const bool even_rows = !csr || (!own_limit && pcg_persistent_rows(n, ctx->nnz, ctx->csr_longest));
   const int units = csr ? n : ctx->n_nodes;
   const long long entries = csr ? ctx->nnz : ctx->nnz / 4;
+  const bool small_ok = o.launch_mode == CSTG_LAUNCH_AUTO && !own_limit;
   const auto next_team = [&](PcgTeam after) {
-    return pcg_persistent_team(units, entries, mixed, csr, o.launch_mode == CSTG_LAUNCH_AUTO, after);
+    return pcg_persistent_team(units, entries, mixed, csr, small_ok, after);
   };
   PcgTeam team = n > 0 && even_rows && o.launch_mode != CSTG_LAUNCH_GRAPH && !instrumented && !snap
                      ? next_team(PcgTeam::kFirst)
