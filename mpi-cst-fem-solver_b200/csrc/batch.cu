@@ -37,6 +37,7 @@
 #include <cooperative_groups.h>
 
 #include "../../include/cstfem_b200.h"
+#include "batch_rule.h"
 #include "common.cuh"
 #include "kernels.h"
 
@@ -1080,6 +1081,7 @@ cudaError_t launch_shape(const BatchArgs* a, int cluster, const int* n_clusters,
   }
   auto halo = k_batch_halo<R, T>;
   unsigned smem = 0;
+  bool halo_ok = true;
   {
     int dev = 0, most = 0;
     cudaGetDevice(&dev);
@@ -1089,7 +1091,8 @@ cudaError_t launch_shape(const BatchArgs* a, int cluster, const int* n_clusters,
     if (max_clusters) {
       e = cudaFuncSetAttribute(halo, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(halo, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e != cudaSuccess) return e;
+      halo_ok = e == cudaSuccess;
+      if (!halo_ok) cudaGetLastError();
     }
   }
   cudaLaunchConfig_t cfg = {};
@@ -1106,20 +1109,21 @@ cudaError_t launch_shape(const BatchArgs* a, int cluster, const int* n_clusters,
   if (max_clusters) {
     cfg.gridDim = dim3((unsigned)cluster);
     int n = 0;
-    *max_clusters = 0;
+    max_clusters[0] = max_clusters[1] = 0;
     cudaError_t e = cudaOccupancyMaxActiveClusters(&n, (void*)kern, &cfg);
     if (e != cudaSuccess) return e;
-    *max_clusters = n;
+    max_clusters[0] = n;
+    if (!halo_ok) return cudaSuccess;
     cfg.dynamicSmemBytes = smem;
-    e = cudaOccupancyMaxActiveClusters(&n, (void*)halo, &cfg);
-    max_clusters[1] = e == cudaSuccess ? n : 0;
-    return e;
+    if (cudaOccupancyMaxActiveClusters(&n, (void*)halo, &cfg) == cudaSuccess)
+      max_clusters[1] = n;
+    else
+      cudaGetLastError();
+    return cudaSuccess;
   }
   BatchArgs b = *a;
   b.smem = smem;
-  // by the largest plate and a halo of a few rows of nodes (a plate that then does not fit is listed)
-  const double own = std::ceil((double)a->largest / cluster), nodes = own + 3.0 * std::sqrt((double)a->largest) + 64.0;
-  if (nodes * (16.0 * R + 4.0) + 4096.0 <= (double)smem) {
+  if (batch_halo_runs({n_clusters[0], n_clusters[1]}, a->largest, cluster, R, smem)) {
     cfg.dynamicSmemBytes = smem;
     cfg.gridDim = dim3((unsigned)(std::min(n_clusters[1], a->n_sys) * cluster));
     const cudaError_t e = cudaLaunchKernelEx(&cfg, halo, b);

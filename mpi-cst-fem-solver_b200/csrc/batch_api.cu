@@ -5,6 +5,7 @@
 
 #include <numeric>
 
+#include "batch_rule.h"
 #include "ctx.h"
 
 static_assert(sizeof(cstg_batch_result) == sizeof(BatchResultDev), "result layouts differ");
@@ -166,7 +167,7 @@ int run(cstg_ctx* ctx, int n_sys, int n_rhs, const double* d_b, double* d_x, con
         Shape sh, bool graph, double* seconds) {
   int maxc[2] = {0, 0};
   fit_shape(ctx, n_rhs, sh, maxc);
-  if (maxc[0] < 1 || maxc[1] < 1)
+  if (!batch_shape_runs(maxc))
     return fail(ctx, CSTG_ERR_UNSUPPORTED, "batch_solve: launch shape %d CTAs x %d threads does not fit",
                 sh.cluster, sh.threads);
   long long launched = 0;
@@ -302,7 +303,7 @@ int cstg_batch_autotune(cstg_ctx* ctx, int n_systems, const int32_t* node_offset
   for (const Shape& sh : kShapes) {
     int maxc[2] = {0, 0};
     fit_shape(ctx, n_rhs, sh, maxc);
-    if (maxc[0] < 1 || maxc[1] < 1) continue;
+    if (!batch_shape_runs(maxc)) continue;
     double t0 = 0.0, t1 = 0.0;
     rc = run(ctx, n_systems, n_rhs, d_b, d_x, o, sh, false, &t0);  // warm-up (first-launch costs)
     if (rc) return rc;
