@@ -342,7 +342,8 @@ int cstg_batch_solve_device(cstg_ctx* ctx, int n_systems, const int32_t* node_of
                             double* seconds);
 /* Times every feasible launch shape (cluster 1/2/4/8/16 CTAs x 256/512 threads) on this batch
  * (device vectors; the solve runs with `opt`, e.g. a reduced max_iter to bound the tuning
- * time), keeps the fastest for later cstg_batch_solve calls on this context and returns it. */
+ * time: the largest system gets max_iter iterations, the others their share by the square root of
+ * their size, as in a whole solve), keeps the fastest for later cstg_batch_solve calls on this context and returns it. */
 int cstg_batch_autotune(cstg_ctx* ctx, int n_systems, const int32_t* node_offsets, int n_rhs,
                         const double* d_b, double* d_x, const cstg_solver_options* opt,
                         cstg_batch_config* best, double* best_seconds);

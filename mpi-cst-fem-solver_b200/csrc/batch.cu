@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(T, (T >= 512 ? 1 : 512 / T)) k_batch_pcg(const
   __shared__ double wsum[(T / 32 > 16 ? T / 32 : 16) * V];  // warp partials, then <= 16 ranks' partials
   __shared__ double red[2 * V];
   __shared__ double tot[V];
-  __shared__ int s_plate;
+  __shared__ int s_plate, s_limit;
   int buf = 0;
   const double2* __restrict__ invd2 = reinterpret_cast<const double2*>(a.inv_diag);
   const double2* __restrict__ b2 = reinterpret_cast<const double2*>(a.b);
@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(T, (T >= 512 ? 1 : 512 / T)) k_batch_pcg(const
     const int plate = *cl.map_shared_rank(&s_plate, 0);
     if (plate < 0) break;
     const int n0 = a.sys_node[plate], n1 = a.sys_node[plate + 1];
+    if (threadIdx.x == 0) s_limit = a.limit[plate];  // (read after the first sums)
     const int first = n0 + crank * T + (int)threadIdx.x, stride = C * T;
 
     // x = 0, r = b, p = D^-1 b; r'z and b'b per load case (solver.cpp:42-58)
@@ -296,7 +297,7 @@ __global__ void __launch_bounds__(T, (T >= 512 ? 1 : 512 / T)) k_batch_pcg(const
         const double rr = tot[R + q];
         rel[q] = sqrt(rr / bn2[q]);
         rmax[q] = fmax(rmax[q], rr);
-        if (rr <= rtol2 * bn2[q] || it[q] >= a.max_iter) {
+        if (rr <= rtol2 * bn2[q] || it[q] >= s_limit) {
           check |= 1u << q;
         } else if (rr <= kBatchDelta2 * rmax[q] || it[q] - last_rep[q] >= kBatchCycle) {
           repl |= 1u << q;
@@ -354,7 +355,7 @@ __global__ void __launch_bounds__(T, (T >= 512 ? 1 : 512 / T)) k_batch_pcg(const
             active &= ~(1u << q);
             continue;
           }
-          if (it[q] >= a.max_iter) {
+          if (it[q] >= s_limit) {
             status[q] = CSTG_SOLVE_MAX_ITER;
             active &= ~(1u << q);
             continue;
@@ -526,6 +527,7 @@ __device__ __forceinline__ void solve_cases(const BatchArgs& a, const cg::cluste
   const double2* __restrict__ invd2 = reinterpret_cast<const double2*>(a.inv_diag) + n0;
   const double2* __restrict__ v64 = reinterpret_cast<const double2*>(a.A64.vals);
   const double rtol2 = a.rtol * a.rtol;
+  const int limit = __ldg(&a.limit[plate]);
   const size_t base = (size_t)n0 * R;
   double2* zg = reinterpret_cast<double2*>(a.p);  // z of wanted nodes, in p's array
   const double2* bg = reinterpret_cast<const double2*>(a.b) + base;
@@ -774,7 +776,7 @@ __device__ __forceinline__ void solve_cases(const BatchArgs& a, const cg::cluste
           sh.rel[lane] = sqrt(rr / sh.bn2[lane]);
           const double rm = fmax(sh.rmax[lane], rr);
           sh.rmax[lane] = rm;
-          if (rr <= rtol2 * sh.bn2[lane] || it >= a.max_iter) {
+          if (rr <= rtol2 * sh.bn2[lane] || it >= limit) {
             chk = true;
           } else if (rr <= kBatchDelta2 * rm || it - sh.last_rep[lane] >= kBatchCycle) {
             rep = true;
@@ -847,7 +849,7 @@ __device__ __forceinline__ void solve_cases(const BatchArgs& a, const cg::cluste
           if (is_check && rr <= rtol2 * sh.bn2[lane]) {
             sh.status[lane] = CSTG_SOLVE_CONVERGED;
             off = true;
-          } else if (sh.it[lane] >= a.max_iter) {
+          } else if (sh.it[lane] >= limit) {
             sh.status[lane] = CSTG_SOLVE_MAX_ITER;
             off = true;
           } else {

@@ -3,6 +3,7 @@
 // CUDA graph that holds one batched solve, and the launch-shape autotuner.
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <numeric>
 
 #include "batch_rule.h"
@@ -59,7 +60,7 @@ int prepare(cstg_ctx* ctx, int n_sys, const int32_t* offs, int n_rhs, const cstg
   const size_t vec = sizeof(double) * (size_t)ctx->n_rows * group;
   ENSURE(ctx->bat_sys, sizeof(int) * table.size());
   ENSURE(ctx->bat_order, sizeof(int) * (size_t)n_sys);
-  ENSURE(ctx->bat_queue, sizeof(int) * ((size_t)n_sys + 64));
+  ENSURE(ctx->bat_queue, sizeof(int) * (2 * (size_t)n_sys + 64));
   ENSURE(ctx->bat_wanted, (size_t)ctx->n_nodes);
   ENSURE(ctx->bat_slots, 2 * sizeof(unsigned short) * (size_t)(ctx->nnz / 4));
   if (o.precision == CSTG_PRECISION_MIXED) ENSURE(ctx->bat_lane, sizeof(float4) * (size_t)(ctx->nnz / 4));
@@ -120,6 +121,7 @@ int enqueue(cstg_ctx* ctx, int n_sys, int n_rhs, const double* d_b, double* d_x,
     a.n_rest = a.queue + 2;
     for (int p = 0; p < n_sys; ++p) a.largest = std::max(a.largest, ctx->bat_offsets[p + 1] - ctx->bat_offsets[p]);
     a.rest = a.queue + 64;
+    a.limit = a.rest + n_sys;
     a.wanted = buf_ptr<unsigned char>(ctx->bat_wanted);
     a.slots = buf_ptr<unsigned short>(ctx->bat_slots);
     a.lane_slots = a.slots + ctx->nnz / 4;
@@ -134,7 +136,7 @@ int enqueue(cstg_ctx* ctx, int n_sys, int n_rhs, const double* d_b, double* d_x,
     a.p = buf_ptr<double>(ctx->bat_p);
     a.Ap = buf_ptr<double>(ctx->bat_Ap);
     a.rtol = o.rtol;
-    a.max_iter = o.max_iter;
+
     a.max_refine = o.max_refinements;
     a.res = buf_ptr<BatchResultDev>(ctx->bat_stats);
     a.res_stride = n_rhs;
@@ -162,7 +164,30 @@ int fit_shape(cstg_ctx* ctx, int n_rhs, Shape sh, int (&max_clusters)[2]) {
   return CSTG_OK;
 }
 
-// One batched solve with shape `sh` (graph-captured when `graph`), timed with CUDA events.
+// The plates' iteration limits. A solve gives every plate max_iter; a trial of launch shapes that max_iter cuts
+// short gives the plates their shares of a whole solve, whose iterations go with the square root of the
+// nodes. With max_iter for all, the small plates' work counted for too much against the largest plate's time,
+// which bounds a whole solve: plates of n_r 20 .. 200 took 153 ms at 8 x 256 threads and 149 at 8 x 512 in 300
+// iterations, and 2.91 and 1.86 s to the end.
+int limits_ready(cstg_ctx* ctx, int n_sys, int max_iter, bool trial) {
+  std::vector<int32_t> limits(n_sys, max_iter);
+  if (trial) {
+    const std::vector<int32_t>& at = ctx->bat_offsets;
+    int largest = 1;
+    for (int p = 0; p < n_sys; ++p) largest = std::max(largest, at[p + 1] - at[p]);
+    for (int p = 0; p < n_sys; ++p)
+      limits[p] = std::max(1, (int)(max_iter * std::sqrt((double)(at[p + 1] - at[p]) / largest)));
+  }
+  if (ctx->bat_limits == limits && ctx->bat_limits_gen == ctx->generation) return CSTG_OK;
+  CK(cudaMemcpyAsync(buf_ptr<int>(ctx->bat_queue) + 64 + n_sys, limits.data(), sizeof(int) * limits.size(),
+                     cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));  // (the host table goes out of scope)
+  ctx->bat_limits = std::move(limits);
+  ctx->bat_limits_gen = ctx->generation;
+  return CSTG_OK;
+}
+
+// One batched solve with shape `sh` (graph-captured when `graph`, else a trial), timed with CUDA events.
 int run(cstg_ctx* ctx, int n_sys, int n_rhs, const double* d_b, double* d_x, const cstg_solver_options& o,
         Shape sh, bool graph, double* seconds) {
   int maxc[2] = {0, 0};
@@ -170,6 +195,8 @@ int run(cstg_ctx* ctx, int n_sys, int n_rhs, const double* d_b, double* d_x, con
   if (!batch_shape_runs(maxc))
     return fail(ctx, CSTG_ERR_UNSUPPORTED, "batch_solve: launch shape %d CTAs x %d threads does not fit",
                 sh.cluster, sh.threads);
+  const int rl = limits_ready(ctx, n_sys, o.max_iter, !graph);
+  if (rl) return rl;
   long long launched = 0;
   if (graph) {
     unsigned long long key = 0x5eedull;

@@ -94,6 +94,8 @@ struct cstg_ctx {
   DevBuf bat_sys, bat_order, bat_queue, bat_wanted, bat_slots, bat_lane, bat_b, bat_x, bat_r, bat_p, bat_Ap, bat_stats, bat_in, bat_out;
   std::vector<int32_t> bat_offsets;  // host copy of the last validated plate table
   unsigned long long bat_checked_gen = ~0ull;
+  std::vector<int32_t> bat_limits;   // host copy of the plates' iteration limits on the device
+  unsigned long long bat_limits_gen = ~0ull;
   cstg_batch_config bat_cfg{};       // tuned launch shape (cluster_ctas == 0: not tuned)
   cudaGraphExec_t bat_graph = nullptr;
   unsigned long long bat_graph_key = 0;

@@ -159,7 +159,8 @@ struct BatchArgs {
   const double* b = nullptr;      // [N][R][2]
   double *x = nullptr, *r = nullptr, *p = nullptr, *Ap = nullptr;
   double rtol = 1e-10;
-  int max_iter = 0, max_refine = 0;
+  const int* limit = nullptr;     // [n_sys] iterations that each plate may take
+  int max_refine = 0;
   BatchResultDev* res = nullptr;
   int res_stride = 0, res_offset = 0;  // result index = plate * res_stride + res_offset + q
 };
