@@ -223,7 +223,8 @@ struct MpnnWork {  // activations (training keeps every layer; inference ping-po
   float* Y = nullptr;          // [N][2]
   float* dY = nullptr;         // [2N]
   float *dH = nullptr, *dH2 = nullptr, *dAs = nullptr, *dAs2 = nullptr;  // [N][64]
-  float* dU = nullptr;         // [kMpL + 1][N][64]: the layers', the encoder's
+  float* dU = nullptr;         // [N][64], one for each layer and the encoder, dU_step floats apart (0: one for all)
+  size_t dU_step = 0;
   float* part = nullptr;       // [kMpL + 1][kMpPartBlocks][kMpPartStride]: the layers'; decoder and encoder
 };
 

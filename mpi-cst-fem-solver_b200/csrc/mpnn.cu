@@ -1732,8 +1732,8 @@ constexpr int kWgNodes = 128;
 constexpr int kWgSmem = kWgNodes * 2 * F * 2 /*Xc rows*/ + kWgNodes * F * 2 /*dU rows*/ + kASmem + kBSmem + 1024;
 
 struct WgradLayers {
-  const float* dU[kMpL];
-  const __nv_bfloat16 *H[kMpL], *A[kMpL];
+  const float* dU[kMpL] = {};
+  const __nv_bfloat16 *H[kMpL] = {}, *A[kMpL] = {};
 };
 
 __global__ void __launch_bounds__(256, 2) k_mp_wgrad_tc(int N, const WgradLayers L, long long spin_limit,
@@ -2223,7 +2223,7 @@ cudaError_t launch_mp_backward(const MpnnGraph& g, const MpnnParams& P, MpnnWork
   for (int l = kMpL - 1; l >= 0; --l) {
     float* dout = din == w.dH ? w.dH2 : w.dH;
     float* aout = as == w.dAs ? w.dAs2 : w.dAs;
-    float* du = w.dU + (size_t)l * N * F;
+    float* du = w.dU + (size_t)l * w.dU_step;
     k_mp_layer_bwd<<<grid, 256, kBwSmem, s>>>(N, g.node_ptr, g.nbr, P, l, din, as, w.G[l], du, dout, aout);
     wl.dU[l] = du;
     wl.H[l] = w.H[l];
@@ -2231,19 +2231,30 @@ cudaError_t launch_mp_backward(const MpnnGraph& g, const MpnnParams& P, MpnnWork
     seg.part[1 + l] = w.part + l * layer_part;
     seg.stride[1 + l] = kMpPartStride;
     seg.dst[1 + l] = kMpOffL0 + l * kMpLStride;
+    if (!w.dU_step) {  // (the next layer overwrites it)
+      WgradLayers one;
+      one.dU[0] = du;
+      one.H[0] = w.H[l];
+      one.A[0] = w.A[l];
+      k_mp_wgrad_tc<<<dim3(kMpPartBlocks, 1), 256, kWgSmem, s>>>(N, one, spin_limit, w.part + l * layer_part, err);
+      count_launches(1);
+    }
     din = dout;
     as = aout;
   }
-  k_mp_wgrad_tc<<<dim3(kMpPartBlocks, kMpL), 256, kWgSmem, s>>>(N, wl, spin_limit, w.part, err);
+  if (w.dU_step) {
+    k_mp_wgrad_tc<<<dim3(kMpPartBlocks, kMpL), 256, kWgSmem, s>>>(N, wl, spin_limit, w.part, err);
+    count_launches(1);
+  }
   // encoder
-  float* du0 = w.dU + (size_t)kMpL * N * F;
+  float* du0 = w.dU + (size_t)kMpL * w.dU_step;
   k_mp_enc_bwd<<<grid_nodes((long long)N * (F / 4), 256), 256, 0, s>>>(N, g.node_ptr, g.nbr, din, as, w.H[0], du0);
   k_mp_wgrad<kMpIn><<<G, 256, 0, s>>>(N, du0, w.X, nullptr, enc_part);
   seg.part[1 + kMpL] = enc_part;
   seg.stride[1 + kMpL] = F * kMpIn + F;
   seg.dst[1 + kMpL] = kMpOffWin;
   k_mp_reduce_parts<<<dim3((kMpPartStride + 63) / 64, kMpL + 2), 64, 0, s>>>(seg, grad);
-  count_launches(5 + kMpL);
+  count_launches(4 + kMpL);
   return cudaGetLastError();
 }
 
