@@ -67,6 +67,14 @@ __device__ __forceinline__ int ld_cg(const int* p) { return __ldcg(p); }
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
+// A load of what the kernel before wrote: this kernel was alive then, so the data is not read-only for its
+// lifetime, which __ldg (ld.global.nc) asks for. After wait_previous().
+__device__ __forceinline__ uint4 ld_chained(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
 template <class... P, class... A>
 cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
   cudaLaunchConfig_t cfg = {};

@@ -748,7 +748,7 @@ __global__ void __launch_bounds__(kLT, kLayerCtasPerSm) k_mp_layer_tc(const MpLa
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         int deg = 0;
         if (n < N) {
-          own = __ldg(reinterpret_cast<const uint4*>(a.Hin + (size_t)n * F) + c);
+          own = ld_chained(reinterpret_cast<const uint4*>(a.Hin + (size_t)n * F) + c);
           for (int k = k0; k < k1; k += 8) {
             int mm[8];
             uint4 v[8];
@@ -759,7 +759,7 @@ __global__ void __launch_bounds__(kLT, kLayerCtasPerSm) k_mp_layer_tc(const MpLa
             }
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              v[j] = mm[j] != n ? __ldg(reinterpret_cast<const uint4*>(a.Hin + (size_t)mm[j] * F) + c)
+              v[j] = mm[j] != n ? ld_chained(reinterpret_cast<const uint4*>(a.Hin + (size_t)mm[j] * F) + c)
                                 : make_uint4(kNegZero2, kNegZero2, kNegZero2, kNegZero2);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {  // (a missing neighbour adds -0: no branch)
@@ -1206,7 +1206,7 @@ __global__ void __launch_bounds__(kWsT, 1)
             for (int j = 0; j < 8; ++j) mm[j] = k + j < k1 ? __ldg(&a.nbr[k + j]) : n;
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              v[j] = mm[j] != n ? __ldg(reinterpret_cast<const uint4*>(a.Hin + (size_t)mm[j] * F) + c)
+              v[j] = mm[j] != n ? ld_chained(reinterpret_cast<const uint4*>(a.Hin + (size_t)mm[j] * F) + c)
                                 : make_uint4(kNegZero2, kNegZero2, kNegZero2, kNegZero2);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
