@@ -391,6 +391,7 @@ struct cstg_trainer {
   std::string err;
   DevBuf p32, m, v, grad, pb, pf, sc[2], losses;
   DevBuf work;  // z, A z and the network's arrays (trainer_work)
+  int lean_from = INT_MAX;  // nodes for which the larger work arrays did not fit the GPU's memory
   int step = 0;
   int cap_nodes = 0;
 };
@@ -433,15 +434,15 @@ int tensure(cstg_trainer* tr, DevBuf& b, size_t bytes) {
     if (rc_) return rc_;                           \
   } while (0)
 
-// Systems of up to this many nodes have two samples in flight and their layers' weight gradients in one launch;
-// above it one kernel fills the GPU, and the arrays for that, 2 KB a node, would buy nothing.
+// Two samples are in flight on systems of up to this many nodes (above it one sample's kernels fill the
+// GPU, and a second set of activations, 1.3 KB a node, would buy nothing).
 constexpr int kPipelineNodes = 200000;
 
-// The work arrays of `sets` samples in flight, all in one allocation (34 of their own took 9.3 ms of a trainer's
-// first step on 33,153 nodes, whose work takes 2.2). Bytes a node: 2,368 with one set, 4,440 with two.
-int trainer_work(cstg_trainer* tr, int N, int sets, double*& z, double*& az, MpnnWork (&w)[2]) {
+// The work arrays' places behind `base` for `sets` samples in flight; split: an array of the backward pass for each
+// layer, so that the layers' weight gradients go in one launch (501,651 nodes: 2.8 ms a sample, 3.1 with one
+// for all). Returns their bytes: 2,368 a node with one set, 1,304 more for the second, 768 more when split.
+size_t trainer_places(char* base, int N, int sets, bool split, double*& z, double*& az, MpnnWork (&w)[2]) {
   const size_t nf = (size_t)N * kMpF;
-  char* base = nullptr;
   size_t used = 0;
   const auto take = [&](auto*& p, size_t count, bool packed = false) {
     using T = std::remove_reference_t<decltype(*p)>;
@@ -449,37 +450,56 @@ int trainer_work(cstg_trainer* tr, int N, int sets, double*& z, double*& az, Mpn
     used += sizeof(T) * count;
     if (!packed) used = (used + 255) & ~(size_t)255;
   };
-  const bool many = N <= kPipelineNodes;
-  for (int pass = 0; pass < 2; ++pass) {  // the size, then the places
-    if (pass) {
-      TENSURE(tr->work, used);
-      base = static_cast<char*>(tr->work.p);
-      used = 0;
-    }
-    MpnnWork& a = w[0];
-    take(z, 2 * (size_t)N);
-    take(az, 2 * (size_t)N);
-    take(a.Y, 2 * (size_t)N);
-    take(a.dH, nf);
-    take(a.dH2, nf);
-    take(a.dAs, nf);
-    take(a.dU, nf * (many ? kMpL + 1 : 1));
-    a.dU_step = many ? nf : 0;
-    take(a.part, (size_t)kMpPartBlocks * kMpPartStride * (kMpL + 1));
-    w[1] = a;
-    for (int k = 0; k < sets; ++k) {
-      // the backward pass has done with the last layer's H and G when it first writes dAs2: it lies on them
-      take(w[k].H[kMpL], nf, true);
-      w[k].dAs2 = reinterpret_cast<float*>(w[k].H[kMpL]);
-      take(w[k].G[kMpL - 1], nf);
-      for (int l = 0; l < kMpL; ++l) take(w[k].H[l], nf);
-      for (int l = 0; l + 1 < kMpL; ++l) take(w[k].G[l], nf);
-      for (int l = 0; l < kMpL; ++l) take(w[k].A[l], nf);
-      take(w[k].X, (size_t)N * kMpIn);
-      take(w[k].dY, 2 * (size_t)N);
-    }
-    if (sets == 1) w[1] = w[0];
+  MpnnWork& a = w[0];
+  take(z, 2 * (size_t)N);
+  take(az, 2 * (size_t)N);
+  take(a.Y, 2 * (size_t)N);
+  take(a.dH, nf);
+  take(a.dH2, nf);
+  take(a.dAs, nf);
+  take(a.dU, nf * (split ? kMpL + 1 : 1));
+  a.dU_step = split ? nf : 0;
+  take(a.part, (size_t)kMpPartBlocks * kMpPartStride * (kMpL + 1));
+  w[1] = a;
+  for (int k = 0; k < sets; ++k) {
+    // the backward pass has done with the last layer's H and G when it first writes dAs2: it lies on them
+    take(w[k].H[kMpL], nf, true);
+    w[k].dAs2 = reinterpret_cast<float*>(w[k].H[kMpL]);
+    take(w[k].G[kMpL - 1], nf);
+    for (int l = 0; l < kMpL; ++l) take(w[k].H[l], nf);
+    for (int l = 0; l + 1 < kMpL; ++l) take(w[k].G[l], nf);
+    for (int l = 0; l < kMpL; ++l) take(w[k].A[l], nf);
+    take(w[k].X, (size_t)N * kMpIn);
+    take(w[k].dY, 2 * (size_t)N);
   }
+  if (sets == 1) w[1] = w[0];
+  return used;
+}
+
+// The work arrays, all in one allocation (34 of their own took 9.3 ms of a trainer's first step on 33,153 nodes,
+// whose work takes 2.2). Where the GPU's memory does not hold them, those of one sample at a time with one array
+// for all layers (sets becomes 1): the same sums in the same order.
+int trainer_work(cstg_trainer* tr, int N, int& sets, double*& z, double*& az, MpnnWork (&w)[2]) {
+  if (N < tr->lean_from) {
+    const size_t bytes = trainer_places(nullptr, N, sets, true, z, az, w);
+    if (tr->work.bytes < bytes) {
+      free_buf(tr->work);  // (both streams have finished: accumulate_samples)
+      const cudaError_t e = cudaMalloc(&tr->work.p, bytes);
+      if (e == cudaSuccess) {
+        tr->work.bytes = bytes;
+      } else {
+        cudaGetLastError();
+        tr->work.p = nullptr;
+        tr->lean_from = N;
+      }
+    }
+  }
+  const bool lean = N >= tr->lean_from;
+  if (lean) {
+    sets = 1;
+    TENSURE(tr->work, trainer_places(nullptr, N, sets, false, z, az, w));
+  }
+  trainer_places(static_cast<char*>(tr->work.p), N, sets, !lean, z, az, w);
   return CSTG_OK;
 }
 
@@ -491,7 +511,7 @@ int accumulate_samples(cstg_trainer* tr, cstg_ctx* ctx, int n_samples, const dou
                        double* losses, const double* winvd, cudaStream_t s, const MpnnGraph& g, const MpnnParams& P,
                        Forward forward) {
   const int N = ctx->n_nodes, n = ctx->n_rows;
-  const int sets = N <= kPipelineNodes && n_samples > 1 ? 2 : 1;
+  int sets = N <= kPipelineNodes && n_samples > 1 ? 2 : 1;
   MpnnWork w[2];
   double *z = nullptr, *az = nullptr;
   const int rc = trainer_work(tr, N, sets, z, az, w);

@@ -1,5 +1,5 @@
-"""The trainer's work arrays: their bytes a node on either side of the size up to which two samples are in flight,
-and the gradients above it, where all layers share one array of the backward pass."""
+"""The trainer's work arrays: their bytes a node on either side of the size up to which two samples are in flight;
+the gradients above it; and the same bits from the smaller arrays that a full GPU leaves room for."""
 import numpy as np
 import pytest
 
@@ -9,6 +9,8 @@ from test_oracle_mpnn import node_graph
 
 pytestmark = pytest.mark.gpu
 
+PARTIAL_SUMS = 4 * 148 * (64 * 128 + 64) * 4
+
 
 def _samples(K, mesh, count):
     import torch
@@ -16,7 +18,7 @@ def _samples(K, mesh, count):
     return torch.stack([K.multiply(e.contiguous()) for e in E]), E
 
 
-@pytest.mark.parametrize("n_r,n_t,samples,per_node", [(128, 256, 2, 4440), (400, 500, 2, 2368)])
+@pytest.mark.parametrize("n_r,n_t,samples,per_node", [(128, 256, 2, 4440), (400, 500, 2, 3136)])
 def test_bytes(pkg, oracle, gpu_lib, n_r, n_t, samples, per_node):
     import torch
     mesh = pkg.plate.quarter_plate(n_r, n_t)
@@ -32,8 +34,40 @@ def test_bytes(pkg, oracle, gpu_lib, n_r, n_t, samples, per_node):
         tr.accumulate(K, R, E)
         taken.append(free - torch.cuda.mem_get_info()[0])
         tr.close()
-    partial_sums = 4 * 148 * (64 * 128 + 64) * 4
-    assert taken[1] <= per_node * mesh.num_nodes + partial_sums + (8 << 20), taken  # (2 MB pages and small arrays)
+    assert taken[1] <= per_node * mesh.num_nodes + PARTIAL_SUMS + (8 << 20), taken  # (2 MB pages and small arrays)
+    K.ctx.close()
+
+
+@pytest.mark.parametrize("n_r,n_t", [(128, 256), (400, 500)])
+def test_same_bits_on_a_full_gpu(pkg, oracle, gpu_lib, n_r, n_t):
+    import torch
+    mesh = pkg.plate.quarter_plate(n_r, n_t)
+    K, mat = _system(pkg, mesh, pkg.plate.symmetry_dirichlet(mesh)[0])
+    p, _ = _bf16_params(oracle, pkg, seed=3)
+    pkg.learned.setup(K, p, mat)
+    R, E = _samples(K, mesh, 3)
+    torch.cuda.empty_cache()
+
+    def train():
+        tr = pkg.learned.Trainer(p)
+        free = torch.cuda.mem_get_info()[0]
+        losses = tr.accumulate(K, R, E)
+        taken = free - torch.cuda.mem_get_info()[0]
+        again = tr.accumulate(K, R, E)
+        assert np.array_equal(losses, again)
+        grads = tr.params(grads=True)[1]
+        tr.close()
+        return losses, grads, taken
+
+    losses, grads, taken = train()
+    lean = 2368 * mesh.num_nodes + PARTIAL_SUMS + (8 << 20)
+    assert lean < taken
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - (lean + taken) // 2, dtype=torch.uint8, device="cuda")
+    losses_f, grads_f, taken_f = train()
+    del filler
+    torch.cuda.empty_cache()
+    assert taken_f <= lean
+    assert np.array_equal(losses, losses_f) and np.array_equal(grads, grads_f)
     K.ctx.close()
 
 
