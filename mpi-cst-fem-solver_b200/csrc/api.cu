@@ -82,7 +82,7 @@ void cstg_destroy(cstg_ctx* ctx) {
   amg_free(ctx);
   DevBuf* all[] = {&ctx->xy,      &ctx->tri,    &ctx->cnt,      &ctx->cursor,   &ctx->ne_ptr,
                    &ctx->ne,      &ctx->scan_tmp, &ctx->deg,    &ctx->node_ptr, &ctx->bnbr,
-                   &ctx->slot,    &ctx->self_pos, &ctx->diag,    &ctx->row_ptr, &ctx->cols,    &ctx->vals,     &ctx->fixed,
+                   &ctx->slot,    &ctx->row_ptr, &ctx->cols,    &ctx->vals,     &ctx->fixed,
                    &ctx->ubar,    &ctx->dofs,   &ctx->dvals,    &ctx->b_in,     &ctx->x,
                    &ctx->pcg_work, &ctx->pcg_slots, &ctx->r,       &ctx->p,      &ctx->Ap,       &ctx->inv_diag, &ctx->partials,
                    &ctx->state,   &ctx->err_word, &ctx->hist,   &ctx->vec_in,   &ctx->vec_out,
@@ -239,16 +239,14 @@ int cstg_build_pattern(cstg_ctx* ctx, int64_t* nnz_out) {
     return fail(ctx, CSTG_ERR_INVALID_ARGUMENT, "build_pattern: nnz = %lld exceeds the int32 range",
                 4 * nb);
   ENSURE(ctx->bnbr, sizeof(int) * (size_t)nb);
-  ENSURE(ctx->slot, sizeof(unsigned) * 3 * (size_t)E);
-  ENSURE(ctx->self_pos, (size_t)N);
+  ENSURE(ctx->slot, sizeof(unsigned) * 3 * (size_t)E + (size_t)N);
   ENSURE(ctx->row_ptr, sizeof(int) * (2 * (size_t)N + 1));
   ENSURE(ctx->cols, sizeof(int) * 4 * (size_t)nb);
-  ENSURE(ctx->vals, sizeof(double) * 4 * (size_t)nb);
-  ENSURE(ctx->diag, sizeof(double) * 2 * (size_t)N);
+  ENSURE(ctx->vals, sizeof(double) * (4 * (size_t)nb + 2 * (size_t)N));
   if (N)
     CK(launch_pattern_fill(m, buf_ptr<int>(ctx->ne_ptr), buf_ptr<int>(ctx->ne),
                            buf_ptr<int>(ctx->node_ptr), buf_ptr<int>(ctx->bnbr), buf_ptr<unsigned>(ctx->slot),
-                           buf_ptr<unsigned char>(ctx->self_pos), buf_ptr<int>(ctx->row_ptr),
+                           self_positions(ctx), buf_ptr<int>(ctx->row_ptr),
                            buf_ptr<int>(ctx->cols), ctx->stream));
   else
     CK(cudaMemsetAsync(ctx->row_ptr.p, 0, sizeof(int), ctx->stream));
@@ -278,8 +276,8 @@ int cstg_assemble(cstg_ctx* ctx, const double D[9], double thickness) {
   if (ctx->n_nodes)
     CK(launch_assemble(m, buf_ptr<int>(ctx->ne_ptr), buf_ptr<int>(ctx->ne), buf_ptr<unsigned>(ctx->slot),
                        buf_ptr<int>(ctx->node_ptr), d, thickness, nullptr, nullptr, nullptr,
-                       buf_ptr<unsigned char>(ctx->self_pos), buf_ptr<double>(ctx->vals),
-                       buf_ptr<double>(ctx->diag), ctx->stream));
+                       self_positions(ctx), buf_ptr<double>(ctx->vals),
+                       matrix_diagonal(ctx), ctx->stream));
   ctx->has_values = true;
   ctx->setup_done = false;
   return CSTG_OK;
@@ -315,8 +313,8 @@ int cstg_assemble_materials(cstg_ctx* ctx, int n_materials, const double* D, con
   if (ctx->n_nodes)
     CK(launch_assemble(m, buf_ptr<int>(ctx->ne_ptr), buf_ptr<int>(ctx->ne), buf_ptr<unsigned>(ctx->slot),
                        buf_ptr<int>(ctx->node_ptr), d, 0.0, buf_ptr<int>(ctx->mat), tab,
-                       tab + 9 * (size_t)n_materials, buf_ptr<unsigned char>(ctx->self_pos),
-                       buf_ptr<double>(ctx->vals), buf_ptr<double>(ctx->diag), ctx->stream));
+                       tab + 9 * (size_t)n_materials, self_positions(ctx),
+                       buf_ptr<double>(ctx->vals), matrix_diagonal(ctx), ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));  // the host tables may go out of scope
   ctx->has_values = true;
   ctx->setup_done = false;
@@ -525,7 +523,7 @@ int cstg_pcg_setup(cstg_ctx* ctx) {
   RESET_ERR();
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   if (n && ctx->kind == 1)
-    CK(launch_inv_diag_nodes(ctx->n_nodes, buf_ptr<double>(ctx->diag), buf_ptr<double>(ctx->inv_diag),
+    CK(launch_inv_diag_nodes(ctx->n_nodes, matrix_diagonal(ctx), buf_ptr<double>(ctx->inv_diag),
                              buf_ptr<int>(ctx->err_word), ctx->stream));
   else if (n)
     CK(launch_inv_diag(n, buf_ptr<int>(ctx->row_ptr), buf_ptr<int>(ctx->cols), buf_ptr<double>(ctx->vals),

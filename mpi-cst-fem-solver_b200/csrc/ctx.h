@@ -60,8 +60,9 @@ struct cstg_ctx {
   DevBuf xy, tri;
 
   // incidence + pattern
-  DevBuf cnt, cursor, ne_ptr, ne, scan_tmp, deg, node_ptr, bnbr, slot, self_pos, diag;
-  DevBuf row_ptr, cols, vals;
+  DevBuf cnt, cursor, ne_ptr, ne, scan_tmp, deg, node_ptr, bnbr;
+  DevBuf slot;  // the element slot map, then every node's own position in its row (self_positions)
+  DevBuf row_ptr, cols, vals;  // (mesh pattern: the diagonal follows the values, matrix_diagonal)
   int kind = 0;  // 0 none, 1 mesh block pattern, 2 caller CSR
   int n_rows = 0;
   long long nnz = 0;
@@ -279,6 +280,12 @@ inline void g_fmt(char* out, size_t n, const char* fmt, ...) {
   std::vsnprintf(out, n, fmt, ap);
   va_end(ap);
 }
+
+// Of a mesh pattern: each node's position in its block row, and the diagonal that the assembly leaves.
+inline unsigned char* self_positions(cstg_ctx* ctx) {
+  return buf_ptr<unsigned char>(ctx->slot) + sizeof(unsigned) * 3 * (size_t)ctx->n_tri;
+}
+inline double* matrix_diagonal(cstg_ctx* ctx) { return buf_ptr<double>(ctx->vals) + ctx->nnz; }
 
 // Defined in amg_api.cu: the multigrid hierarchy (built when missing or stale) and z = M r.
 int amg_ready(cstg_ctx* ctx);
