@@ -107,7 +107,7 @@ int enqueue(cstg_ctx* ctx, int n_sys, int n_rhs, const double* d_b, double* d_x,
             Shape sh, const int* n_clusters, long long* launched) {
   const int N = ctx->n_nodes;
   const long long ld = ctx->n_rows;
-  const long long before = launches_total();
+  const long long before = launches_here();
   for (int q0 = 0; q0 < n_rhs; q0 += kMaxGroup) {
     const int R = std::min(kMaxGroup, n_rhs - q0);
     CK(cudaMemsetAsync(ctx->bat_queue.p, 0, sizeof(int) * 64, ctx->stream));
@@ -144,7 +144,7 @@ int enqueue(cstg_ctx* ctx, int n_sys, int n_rhs, const double* d_b, double* d_x,
     CK(launch_batch_pcg(a, R, sh.cluster, sh.threads, n_clusters, ctx->stream));
     CK(launch_batch_unpack(N, R, q0, ld, buf_ptr<double>(ctx->bat_x), d_x, ctx->stream));
   }
-  *launched = launches_total() - before;
+  *launched = launches_here() - before;
   return CSTG_OK;
 }
 

@@ -441,9 +441,10 @@ cudaError_t amg_tail(const int* skip, const AmgTail& t, int cluster, int* max_cl
 cudaError_t amg_rigid_modes(int N, const double* xy, double* Bf, cudaStream_t s);
 
 // Process-wide count of kernel launches issued by this library (graph launches count every
-// kernel node they run).
+// kernel node they run); launches_here: those of the calling thread (what a capture has recorded).
 void count_launches(long long k);
 long long launches_total();
+long long launches_here();
 
 // mesh_kernels.cu
 cudaError_t scan_exclusive(const int* in, int n, int* out, int* tmp, cudaStream_t s);

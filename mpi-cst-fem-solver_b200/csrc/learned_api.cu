@@ -242,13 +242,13 @@ int cstg_host::run_fcg(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg
       cudaGraphExecDestroy(ctx->fcg_graph);
       ctx->fcg_graph = nullptr;
     }
-    const long long l0 = launches_total();
+    const long long l0 = launches_here();
     cudaGraph_t gr = nullptr;
     CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     int rc = CSTG_OK;
     for (int k = 0; k < chunk && rc == CSTG_OK; ++k) rc = iteration();
     const cudaError_t ee = cudaStreamEndCapture(ctx->stream, &gr);
-    const long long captured = launches_total() - l0;
+    const long long captured = launches_here() - l0;
     count_launches(-captured);
     if (rc) {
       if (gr) cudaGraphDestroy(gr);

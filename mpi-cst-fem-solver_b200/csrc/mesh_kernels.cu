@@ -25,8 +25,13 @@
 namespace cstg {
 
 static std::atomic<long long> g_launches{0};
-void count_launches(long long k) { g_launches.fetch_add(k, std::memory_order_relaxed); }
+static thread_local long long t_launches = 0;
+void count_launches(long long k) {
+  g_launches.fetch_add(k, std::memory_order_relaxed);
+  t_launches += k;
+}
 long long launches_total() { return g_launches.load(std::memory_order_relaxed); }
+long long launches_here() { return t_launches; }
 
 // ---------------------------------------------------------------------------------------
 // exclusive scan of int32 counts: out[0..n] (out[n] = total). Three passes, 2048 items per
