@@ -34,6 +34,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "stage_drain.cuh"
 
 namespace cstg {
 
@@ -1052,6 +1053,18 @@ __device__ __forceinline__ bool ws_wait(uint32_t bar, uint32_t parity, long long
   if (!ok) ok = ws_poll(bar, parity, limit, abort_v, err, tile);
   return __all_sync(0xffffffffu, ok);
 }
+// The copies issued land before the CTA leaves (bounded). After a timeout one producer may have stopped before a
+// tile whose copies the other has issued: without its arrival that phase would not end. So the own producer
+// waits for the other's end (whose waits are bounded too) and then for the copies of both.
+__device__ __noinline__ void ws_drain(uint32_t full0, int own, const volatile int* stopped) {
+  int other = 0;
+  for (long long i = 0; i < kMbarSpinLimit && (other = *stopped) == 0; ++i) __nanosleep(100);
+  for (int j = 0; j < kWsStages; ++j) {
+    const StageDrain d = stage_drain(j, kWsStages, own, other ? other - 1 : own);
+    if (d.arrive) mbar_arrive(full0 + 8u * j);
+    if (d.wait) mbar_wait(full0 + 8u * j, d.parity, kMbarSpinLimit);
+  }
+}
 // Stage k % 3 and phase (k / 3) & 1 of a role's tile k, stepped without divisions.
 struct WsStage {
   uint32_t s = 0, phase = 0;
@@ -1081,6 +1094,7 @@ __global__ void __launch_bounds__(kWsT, 1)
   __shared__ uint64_t mma_done[2], acc_empty[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
+  __shared__ int stopped;  // tiles whose copies the union producer has issued, plus one (0: not yet at its end)
   __shared__ __align__(16) float wout[2 * F];
   __shared__ float bout[2];
   __shared__ float s_inv[kPlanMaxLocal + 1];  // 1/deg (IEEE quotients), 0 for no neighbour
@@ -1139,7 +1153,7 @@ __global__ void __launch_bounds__(kWsT, 1)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&acc_empty[j])), "r"(kWsEpiWarps));
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    abort_flag = 0;
+    abort_flag = stopped = 0;
   }
   wait_previous();  // (so far: parameters and flags that the kernel before does not write)
   if (!LAST) start_next();
@@ -1343,9 +1357,7 @@ __global__ void __launch_bounds__(kWsT, 1)
                      : "memory");
         tma_load_rows(smem_u32(sOwn + (size_t)os * kWsStage), &tin, tile * kTile, fb);  // (past N: zeros)
       }
-      // the copies issued land before the CTA leaves (bounded)
-      for (int j = max(0, kt - kWsStages); j < kt; ++j)
-        mbar_wait(full0 + 8u * (j % kWsStages), (uint32_t)(j / kWsStages) & 1u, kMbarSpinLimit);
+      ws_drain(full0, kt, &stopped);
     }
   } else if (warp == kWsUnionProd) {
     // ---- union producer: each tile's union and its node slots
@@ -1392,10 +1404,7 @@ __global__ void __launch_bounds__(kWsT, 1)
                      "l"(a.Hin + (size_t)rn.x * F), "r"((uint32_t)rn.y * 128u), "r"(fb)
                      : "memory");
     }
-    // the copies issued land before the CTA leaves (bounded)
-    if (lane == 0)
-      for (int j = max(0, kt - kWsStages); j < kt; ++j)
-        mbar_wait(full0 + 8u * (j % kWsStages), (uint32_t)(j / kWsStages) & 1u, kMbarSpinLimit);
+    if (lane == 0) *reinterpret_cast<volatile int*>(&stopped) = kt + 1;
   } else if (lane == 0) {
     // ---- MMA: one thread
     const uint32_t b_addr = smem_u32(sB);
