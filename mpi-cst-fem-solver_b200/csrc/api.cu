@@ -261,6 +261,15 @@ int cstg_build_pattern(cstg_ctx* ctx, int64_t* nnz_out) {
 
 // ---- assemble_stiffness ---------------------------------------------------------------------
 
+static double largest(const double* v, size_t n) {  // of the magnitudes; NaN if one is
+  double m = 0.0;
+  for (size_t k = 0; k < n; ++k) {
+    if (v[k] != v[k]) return v[k];
+    m = std::max(m, std::fabs(v[k]));
+  }
+  return m;
+}
+
 int cstg_assemble(cstg_ctx* ctx, const double D[9], double thickness) {
   BEGIN(ctx);
   if (!D) return fail(ctx, CSTG_ERR_INVALID_ARGUMENT, "assemble: null D");
@@ -275,7 +284,7 @@ int cstg_assemble(cstg_ctx* ctx, const double D[9], double thickness) {
   std::memcpy(d.v, D, sizeof d.v);
   if (ctx->n_nodes)
     CK(launch_assemble(m, buf_ptr<int>(ctx->ne_ptr), buf_ptr<int>(ctx->ne), buf_ptr<unsigned>(ctx->slot),
-                       buf_ptr<int>(ctx->node_ptr), d, thickness, nullptr, nullptr, nullptr,
+                       buf_ptr<int>(ctx->node_ptr), d, thickness, nullptr, nullptr, nullptr, largest(D, 9),
                        self_positions(ctx), buf_ptr<double>(ctx->vals),
                        matrix_diagonal(ctx), ctx->stream));
   ctx->has_values = true;
@@ -313,7 +322,7 @@ int cstg_assemble_materials(cstg_ctx* ctx, int n_materials, const double* D, con
   if (ctx->n_nodes)
     CK(launch_assemble(m, buf_ptr<int>(ctx->ne_ptr), buf_ptr<int>(ctx->ne), buf_ptr<unsigned>(ctx->slot),
                        buf_ptr<int>(ctx->node_ptr), d, 0.0, buf_ptr<int>(ctx->mat), tab,
-                       tab + 9 * (size_t)n_materials, self_positions(ctx),
+                       tab + 9 * (size_t)n_materials, largest(D, 9 * (size_t)n_materials), self_positions(ctx),
                        buf_ptr<double>(ctx->vals), matrix_diagonal(ctx), ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));  // the host tables may go out of scope
   ctx->has_values = true;

@@ -458,8 +458,8 @@ cudaError_t launch_pattern_fill(const MeshDev& m, const int* ne_ptr, const int* 
                                 int* row_ptr, int* cols, cudaStream_t s);
 cudaError_t launch_assemble(const MeshDev& m, const int* ne_ptr, const int* ne, const unsigned* slot,
                             const int* node_ptr, const Mat3& D, double t, const int* mat,
-                            const double* Dtab, const double* ttab, const unsigned char* self, double* vals,
-                            double* diag, cudaStream_t s);
+                            const double* Dtab, const double* ttab, double d_max /* largest |entry| of D: NaN if one is */,
+                            const unsigned char* self, double* vals, double* diag, cudaStream_t s);
 // node_ptr, bnbr: the mesh pattern's block rows (null: a caller's CSR)
 cudaError_t launch_dirichlet(int n_rows, const int* row_ptr, const int* cols, double* vals,
                              int n_fixed, const int* dofs, const double* values,

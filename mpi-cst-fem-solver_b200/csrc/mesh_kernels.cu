@@ -17,7 +17,10 @@
 // plate: pattern 477 -> 205 us, assembly 1,202 -> 246, elimination 96 -> 31, diagonal 105 -> 12).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
+#include <cmath>
+#include <cstring>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -379,13 +382,14 @@ __device__ __forceinline__ double ke_entry(const CstB& o, int i, int j) {
   return __dmul_rn(o.scale, __dadd_rn(x, __dmul_rn(o.B[12 + p], o.DB[12 + q])));
 }
 
-// D and B are finite and D B has not overflowed: every entry of D meets a nonzero place of B and every
-// entry of B one of D's in the terms that DB keeps, so DB shows it.
-__device__ __forceinline__ bool finite_element(const CstB& o) {
+// Whether the short sums hold for an element: B's six different entries are below the limit (a double's upper
+// word) up to which D B is finite, see b_limit.
+__device__ __forceinline__ bool finite_element(const CstB& o, int limit) {
   int most = 0;
 #pragma unroll
-  for (int k = 0; k < 18; ++k) most = max(most, __double2hiint(o.DB[k]) & 0x7fffffff);
-  return most < 0x7ff00000;
+  for (int k = 0; k < 6; k += 2)
+    most = max(most, max(__double2hiint(o.B[k]) & 0x7fffffff, __double2hiint(o.B[7 + k]) & 0x7fffffff));
+  return most < limit;
 }
 
 // Rows 2A, 2A+1 of an element's Ke added into a node's two CSR rows (entry k of row r at
@@ -463,7 +467,7 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(
     const int* __restrict__ ne_ptr, const int* __restrict__ ne, const unsigned* __restrict__ slot,
     const int* __restrict__ node_ptr, const Mat3 Dm, double thickness,
     const int* __restrict__ mat, const double* __restrict__ Dtab, const double* __restrict__ ttab,
-    const unsigned char* __restrict__ self, double* __restrict__ vals, double2* __restrict__ diag) {
+    const unsigned char* __restrict__ self, int limit, double* __restrict__ vals, double2* __restrict__ diag) {
   __shared__ double acc[4 * kRowNodes][kAsmThreads + 1];
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31, t0 = threadIdx.x & ~31;
@@ -496,7 +500,7 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(
       } else {
         cst_element(exy, Dm.v, thickness, o);
       }
-      finite &= finite_element(o);
+      finite &= finite_element(o, limit);
       if (small)
         add_element(o, a, slots, [&](int r, int k) -> double& { return acc[r * 2 * deg + k][threadIdx.x]; });
       else
@@ -733,12 +737,22 @@ cudaError_t launch_pattern_fill(const MeshDev& m, const int* ne_ptr, const int* 
   return cudaGetLastError();
 }
 
+// The upper word of the double below which B's entries leave every D B (a sum of two products) finite, for entries
+// of D up to d_max: 0 (never) where D is not finite itself.
+static int b_limit(double d_max) {
+  if (!(d_max <= 1.7976931348623157e308)) return 0;
+  const double most = std::min(8.9e307, std::ldexp(1.0, 1021) / d_max);  // (d_max 0: infinity)
+  long long bits;
+  std::memcpy(&bits, &most, sizeof bits);
+  return (int)(bits >> 32);
+}
+
 cudaError_t launch_assemble(const MeshDev& m, const int* ne_ptr, const int* ne, const unsigned* slot,
                             const int* node_ptr, const Mat3& D, double t, const int* mat,
-                            const double* Dtab, const double* ttab, const unsigned char* self, double* vals,
-                            double* diag, cudaStream_t s) {
+                            const double* Dtab, const double* ttab, double d_max, const unsigned char* self,
+                            double* vals, double* diag, cudaStream_t s) {
   k_assemble<<<nblk(m.n_nodes, kAsmThreads), kAsmThreads, 0, s>>>(m.n_nodes, m.xy, m.tri, ne_ptr, ne, slot, node_ptr,
-                                                  D, t, mat, Dtab, ttab, self, vals,
+                                                  D, t, mat, Dtab, ttab, self, b_limit(d_max), vals,
                                                   reinterpret_cast<double2*>(diag));
   count_launches(1);
   return cudaGetLastError();
