@@ -95,6 +95,13 @@ typedef struct {
                                    cstg_learned_setup (with the smoother's weights) after
                                    cstg_pcg_setup                                                */
 
+/* What a persistent solve is launched on (cstg_solve_teams) */
+#define CSTG_TEAM_CLUSTER 0   /* one cluster of 16 blocks                                       */
+#define CSTG_TEAM_RESIDENT 1  /* a block per SM, matrix and vectors in shared memory            */
+#define CSTG_TEAM_STREAM 2    /* a block per SM that streams the matrix                         */
+#define CSTG_TEAM_NARROW 3    /* the same by narrower groups of rows                            */
+#define CSTG_TEAM_GRID 4      /* all vectors in global memory                                   */
+
 /* launch_mode of cstg_pcg_solve */
 #define CSTG_LAUNCH_AUTO 0        /* one persistent kernel runs all iterations (mesh pattern, or CSR
                                      with short rows of like length) where the blocks' shares of the
@@ -168,6 +175,9 @@ int cstg_set_stream(cstg_ctx* ctx, void* cuda_stream); /* NULL: the context's ow
 int cstg_get_stream(cstg_ctx* ctx, void** cuda_stream);
 /* The phase times of the last instrumented solve (CSTG_LAUNCH_INSTRUMENTED) since cstg_pcg_setup. */
 int cstg_solve_breakdown(cstg_ctx* ctx, cstg_breakdown* out);
+/* The teams that the last cstg_pcg_solve of this context was launched on, in order: the first *count of at most `max`
+ * (a team whose blocks' shares did not fit leaves the solve to the next one; none: captured kernels). */
+int cstg_solve_teams(cstg_ctx* ctx, int* teams, int max, int* count);
 void cstg_default_options(cstg_solver_options* opt);
 int cstg_version(void);
 /* The compute architecture of the library's kernels as the CUDA runtime reports it for `device`

@@ -132,6 +132,15 @@ int cstg_solve_breakdown(cstg_ctx* ctx, cstg_breakdown* out) {
   return CSTG_OK;
 }
 
+int cstg_solve_teams(cstg_ctx* ctx, int* teams, int max, int* count) {
+  BEGIN(ctx);
+  if (!count || max < 0 || (max > 0 && !teams))
+    return fail(ctx, CSTG_ERR_INVALID_ARGUMENT, "solve_teams: bad output");
+  *count = (int)ctx->teams.size();
+  std::copy_n(ctx->teams.begin(), std::min(max, *count), teams);
+  return CSTG_OK;
+}
+
 int cstg_get_stream(cstg_ctx* ctx, void** stream) {
   BEGIN(ctx);
   if (!stream) return fail(ctx, CSTG_ERR_INVALID_ARGUMENT, "get_stream: null output");
@@ -674,6 +683,7 @@ static int run_solve(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg_s
   // With a limit on its waits set by the caller, a solve takes only the waits it always had: the teams that poll for
   // the mesh pattern (a cluster's barrier is the hardware's own and knows no limit), none for CSR.
   const bool own_limit = ctx->barrier_spin != kBarrierSpinDefault;
+  ctx->teams.clear();
   const bool even_rows = !csr || (!own_limit && pcg_persistent_rows(n, ctx->nnz, ctx->csr_longest));
   const int units = csr ? n : ctx->n_nodes;
   const long long entries = csr ? ctx->nnz : ctx->nnz / 4;
@@ -761,7 +771,7 @@ static int run_solve(cstg_ctx* ctx, const double* d_b, double* d_x, const cstg_s
           next_team));
       if (rc) return rc;
       if (team != PcgTeam::kNone) {
-        // (launched)
+        ctx->teams.push_back((int)team);
       } else if (instrumented) {
         // SpMV (with its fused p'Ap partials), then the vector phase (x, r, p updates with their
         // fused dots), an event after each; the elapsed times are summed after the batch

@@ -74,6 +74,7 @@ struct cstg_ctx {
   DevBuf fixed, ubar, dofs, dvals;
 
   // solver
+  std::vector<int> teams;      // that the last Jacobi-PCG solve was launched on
   DevBuf pcg_work, pcg_slots;  // persistent solve: what passes between blocks, rows in their numbering
   DevBuf b_in, x, r, p, Ap, inv_diag, partials, state, err_word, hist, vec_in, vec_out, stress;
   // mixed precision: FP32 difference-form operator and FP32 work vectors

@@ -1,10 +1,10 @@
-"""Which team of blocks solves a system, read from the kernels that ran: a team whose blocks' shares do not fit
+"""Which team of blocks solves a system, as the library reports it: a team whose blocks' shares do not fit
 declines, and the next one takes the solve. The sizes on either side of each limit follow from what a block
 keeps in its shared memory (231,424 bytes): FP64 in shared memory 320 bytes a node of an O-grid and 20 a
 halo node (224 x 448 fits with room for 126 more halo nodes, 226 x 452 lacks 71), mixed 223 and 20 (268 x 536
 fits with 80, 270 x 540 lacks 81). Numbered at random, 300 x 600 has 63 (FP64) and 415 (mixed) to spare in narrow
 groups of rows, and 330 x 660 lacks more than 1,300. Their values are compared at convergence."""
-import re
+import ctypes as C
 
 import numpy as np
 import pytest
@@ -13,38 +13,21 @@ from test_gpu_teams import _both, _plate
 
 pytestmark = pytest.mark.gpu
 
-TEAMS = {("true", "true", 256): "cluster", ("false", "true", 256): "resident", ("0", 384): "stream", ("0", 256): "narrow",
-         ("1", 1): "stream", ("1", 2): "narrow"}
+TEAMS = ["cluster", "resident", "stream", "narrow", "grid"]
 
 
-def _teams(f):
-    """The teams launched by f, in order."""
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
-        f()
-        torch.cuda.synchronize()
-    kernels = sorted((e.time_range.start, e.name) for e in p.events() if "k_" in e.name and "cstg" in e.name)
-    if not kernels:
-        pytest.skip("the profiler records no kernels here")
-    out = []
-    for _, name in kernels:
-        if "k_pcg_grid" in name:
-            out.append("grid")
-        m = re.search(r"k_pcg_persistent<([^>]*)>", name)
-        if m:
-            op, cluster, resident, lanes, threads = (re.sub(r"\(\w+\)", "", a).strip() for a in m[1].split(","))
-            op, cluster, resident = op[-1], {"1": "true", "0": "false"}.get(cluster, cluster), \
-                {"1": "true", "0": "false"}.get(resident, resident)
-            key = (cluster, resident, int(threads)) if resident == "true" else (op, int(threads) if op == "0" else int(lanes))
-            out.append(TEAMS[key])
-    return out
+def _teams(K):
+    """The teams that the last solve was launched on, in order."""
+    got, count = (C.c_int * 8)(), C.c_int(0)
+    K.ctx.check(K.ctx.L.cstg_solve_teams(K.ctx.h, got, 8, C.byref(count)))
+    return [TEAMS[t] for t in got[:count.value]]
 
 
 def _check(pkg, K, b, want, **kw):
     s = pkg.CgJacobiSolver(pkg.SolverOptions(**kw))
     s.setup(K)
-    assert _teams(lambda: s.solve(b)) == want
+    s.solve(b)
+    assert _teams(K) == want
     K.ctx.close()
 
 
