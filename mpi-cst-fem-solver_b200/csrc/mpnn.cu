@@ -962,8 +962,9 @@ __global__ void __launch_bounds__(kLT, kLayerCtasPerSm) k_mp_layer_tc(const MpLa
 // issue slots; each is bounded (spin_limit polls). A role that gives up records the timeout and
 // raises the CTA's abort flag, which every other wait polls. Before the CTA leaves, the copies and
 // MMAs already issued have completed (bounded waits) and the tensor stores have read their staging.
-// Bound by the gathers' instructions (73 % of the issue slots; shared memory 55 %), not by HBM. Measured on
-// the 2M-DOF plate, 82 us a layer and 96 us the last (41 at the measured HBM bandwidth). Before: 89 and
+// Not bound by HBM (41 us at the measured bandwidth); what bounds it is not known: the issue slots are 67 % busy,
+// shared memory 56 %, but without the gathers' work the kernel still takes 77 of its 82 us, and without the
+// other rows and the stores too 68. Measured on the 2M-DOF plate, 82 us a layer and 94 to 96 the last. Before: 89 and
 // 107 us with the own rows copied twice, two stages, a barrier per kind of copy, seven places, and four
 // epilogue warps, which were the last layer's limit. A third stage, other rows alone in the union, or six
 // places gave nothing by themselves; dropping waits from the gather warps' path did (each costs ~270 cycles

@@ -14,10 +14,11 @@
 // per matrix block. The halo, the rows' 16-bit numbering of their neighbours in [own | halo] and
 // the list of nodes that others need are built at the start of the launch. r, Ap, x and D^-1 at own
 // nodes live in shared memory as far as they fit, and so does the matrix when all of it fits (33 MB
-// over 148 SMs: FP64 to about 230k DOFs, mixed to about 330k). A larger matrix is streamed: every
+// over 148 SMs: O-grids of up to about 200k DOFs in FP64, 290k mixed). A larger matrix is streamed: every
 // warp has a ring of stages that bulk copies fill with its next groups of rows, also while the block
-// waits in a reduction, so the copies never stop for one. A numbering without locality, whose halos
-// do not fit, is left to the per-phase kernels.
+// waits in a reduction, so the copies never stop for one. What no block can hold, O-grids above about 2.1M DOFs
+// and, from about 400k, numberings without locality, whose halos do not fit, is left to the grid kernel
+// (persistent_grid.cu), or for a caller's CSR to the captured kernels.
 //
 // Nothing between blocks needs a memory fence: a word of z or of a partial sum carries the number of
 // its reduction in its upper half (32 bits of payload per 64-bit word), so a reader polls the data
@@ -29,7 +30,7 @@
 // of the last-block kind after each (us an iteration, before and now): 3,321 nodes FP64 20 -> 3.9;
 // 65,341 nodes FP64 21 -> 7.9; 15,006 CSR rows 25 -> 5.9 (three kernels an iteration in a graph before);
 // 501,651 nodes mixed 47 -> 22 (120 MB that cannot be avoided: 18 at the measured 6.5 TB/s), FP64 54 ->
-// 28; 1,000,122 nodes FP64 96 -> 60, mixed 77 -> 52.
+// 28; 1,000,122 nodes FP64 96 -> 61, mixed 77 -> 49.
 //
 // Reductions. A block adds its threads' values in a fixed order and hands the sums to every block;
 // every block adds all blocks' sums in index order and takes the same decisions, so no last block
@@ -920,7 +921,7 @@ __global__ void __launch_bounds__(T, 1) k_pcg_persistent(const SolveArgs a) {
   }
 
   // ---- end: copies in flight land (bounded), the last step of x, the state. A streamed mixed solve
-  // that switched precision (done = 0) leaves its iteration to the per-phase kernels: r and the
+  // that switched precision (done = 0) leaves its iteration to the grid kernel: r and the
   // next direction go back to global memory.
   if (!RES && lane == 0)
     for (; taken != issued; ++taken)

@@ -1,9 +1,8 @@
-// Persistent Jacobi-PCG for meshes that no team of persistent.cu holds (above about 2.6M DOFs, or numbered
-// without locality): one cooperative launch runs every iteration of a solve on the mesh
+// Persistent Jacobi-PCG for meshes that no team of persistent.cu holds (O-grids above about 2.1M DOFs; numbered
+// without locality, from about 400k): one cooperative launch runs every iteration of a solve on the mesh
 // (2x2-block) pattern, FP64 or mixed precision, instead of three or four kernels per iteration, with
-// all vectors in global memory. 4,007,502 DOFs, us an iteration against the captured kernels: FP64 195
-// against 198, mixed 137 against 143; 1,003,302 DOFs numbered at random, mixed 58 against 60 (FP64 61
-// against 59).
+// all vectors in global memory. 4,006,602 DOFs, us an iteration against the captured kernels: mixed 137 against
+// 145, FP64 197 against 195; 1,003,302 DOFs numbered at random, mixed 58 against 60, FP64 62 against 60.
 //
 // Per iteration (FP64; the mixed method swaps the SpMV operator and may add the replacement
 // phase R, see mixed_kernels.cu for the method):
